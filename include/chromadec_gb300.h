@@ -122,7 +122,7 @@ int chdg_chroma_device(chdg_engine *e, const uint16_t *d_fields, int64_t field_s
  * their own allocator or budget, and latency-critical loops where cudaMalloc's
  * implicit device synchronisation would stall other work. The chroma scratch
  * and the guard-band decision records are fixed arrays compiled into the
- * library (81.6 MB: 8 frames of the 948x576 active picture), which every GPU
+ * library (81.1 MB: 8 frames of the 948x576 active picture), which every GPU
  * that loads the library holds until the process exits; calls asking for
  * more than 8 frames, a negative or reversed frame range, or a larger active
  * picture fail with CHDG_E_INVALID_ARG. No cudaMalloc/cudaFree or other

@@ -268,10 +268,9 @@ int Engine::ensure_deferred(int frames, int nchunks)
     unc_rec_ = nullptr;
     rerun_ = nullptr;
     unc_cap_ = 0;
-    // every kx group of every step can hold a record, and each record lists
-    // at most one work item
+    // every kx group of every step can hold a record, listed at most once
     if ((e = cudaMalloc(&unc_rec_, need * sizeof(tpal::UncRecord))) != cudaSuccess ||
-        (e = cudaMalloc(&rerun_, 2 * need * sizeof(unsigned))) != cudaSuccess) {
+        (e = cudaMalloc(&rerun_, need * sizeof(unsigned))) != cudaSuccess) {
         if (unc_rec_) cudaFree(unc_rec_);
         unc_rec_ = nullptr;
         rerun_ = nullptr;
@@ -331,7 +330,7 @@ int Engine::run_transform(const uint16_t *fields, long long stride, int field_ba
         if (tc_variant_ >= 0) return tpal::tc3_transform(P, g_.field_height, tc_variant_, s);
         if (net_ != nullptr) return run_learned(P, s);
         // guard-band decisions: recorded by the walk, decided by the resolve
-        // pass, work items with a wrong FP32 decision walked again exactly
+        // pass, outputs of a wrong FP32 decision walked again exactly
         if (static_) {
             const int ntiles = P.ntx * P.nty;
             if (unc_rec_ == nullptr || tpal::tp3_unc_capacity(ntiles, fe - fb, P.nchunks) > unc_cap_)

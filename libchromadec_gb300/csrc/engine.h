@@ -62,8 +62,8 @@ public:
                        float *scratch, size_t scratch_floats, cudaStream_t s);
     static size_t scratch_floats_for(const chdg_geometry &g, int nframes);
     // Caller-provided buffers of the guard-band decision passes for the
-    // allocation-free decode: records, a list of as many (work item, step)
-    // pairs, two counters.
+    // allocation-free decode: records, a list of as many entries, two
+    // counters.
     void set_static_decisions(void *records, unsigned *items, unsigned long long cap, unsigned *counters)
     {
         unc_rec_ = records;

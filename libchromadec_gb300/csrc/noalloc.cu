@@ -13,9 +13,9 @@
 // exits (sizes at the default 948x576 active picture, 4,440 tile positions):
 //   chroma scratch   4 overlap planes x 16 fields x 288 x 948 FP32   69.9 MB
 //   decision records 133,200 x 80 B (every kx group of an 8-frame call) 10.7 MB
-//   work-item list   2 x 133,200 x 4 B                                  1.1 MB
+//   corrected list   133,200 x 4 B                                      0.5 MB
 //   per-bin table    768 x 3 FP32, two counters
-// in all 81.6 MB. Calls with more than 8 frames, or with a picture whose
+// in all 81.1 MB. Calls with more than 8 frames, or with a picture whose
 // planes or tile grid do not fit these arrays, are rejected.
 #include <mutex>
 #include <string>
@@ -43,7 +43,7 @@ static_assert(sizeof(tpal::UncRecord) == 80, "decision record layout");
 static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats];
 static __device__ __align__(256) float g_static_thresholds[3 * 768];
 static __device__ __align__(256) tpal::UncRecord g_static_records[kStaticRecords];
-static __device__ __align__(256) unsigned g_static_items[2 * kStaticRecords];
+static __device__ __align__(256) unsigned g_static_items[kStaticRecords];
 static __device__ __align__(256) unsigned g_static_counters[2];
 
 struct DeviceSymbols {

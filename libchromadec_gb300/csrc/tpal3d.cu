@@ -28,11 +28,11 @@
 //    writes its own partial plane and the demodulator sums the four planes.
 //    No atomics; results are deterministic.
 //  * Threshold decisions: the spectrum is computed in FP32 with a per-bin
-//    error bound E = K * 2^-24 * (sum_z w_z (A_z[kx] + R_z/2) + sum_z w_z |S_z|_1)
+//    error estimate E = K * 2^-24 * (sum_z w_z (A_z[kx] + R_z/2) + sum_z w_z |S_z|_1)
 //    where A is the L1 norm of the field's column-DFT outputs for that kx and R
 //    the L1 norm of its DC-removed windowed rows. A decision whose margin is
-//    inside the bound is recomputed by the whole warp in double-float from the
-//    raw samples, so every decision equals the FP64 reference's.
+//    inside that band is taken again in double-float from the raw samples by
+//    the resolve pass, so every decision equals the FP64 reference's.
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -76,29 +76,18 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
     return make_float2(__fmaf_rn(a.x, b.x, -a.y * b.y), __fmaf_rn(a.x, b.y, a.y * b.x));
 }
 
+template <int N>
+struct Int {
+    static constexpr int value = N;
+};
+
 __device__ __forceinline__ float l1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 
 // multiply by -i: (y, -x); by the tables' exp(-i pi/2) = (6e-17, -1), whose
 // tiny real part is below the rounding of any non-degenerate product
 __device__ __forceinline__ float2 mul_negi(float2 a) { return make_float2(a.y, -a.x); }
 
-__device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
-{
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
-}
-
-__device__ __forceinline__ float2 shfl2(float2 v, int src)
-{
-    return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-
 __device__ __forceinline__ df dfc_abs2(dfc v) { return df_add(df_mul(v.re, v.re), df_mul(v.im, v.im)); }
-
-__device__ __forceinline__ dfc dfc_tw32(int r)
-{
-    r &= 31;
-    return {{c3_dftw32[r][0], c3_dftw32[r][1]}, {c3_dftw32[r][2], c3_dftw32[r][3]}};
-}
 
 // Squared threshold of visited bin (z, y, x-2) for x in 2..4.
 struct Thr {
@@ -117,132 +106,6 @@ __device__ __forceinline__ Thr thr_of(const T3Params &P, int m, int kz, int ky, 
     }
     const float *t = P.thr_table + 3 * ((kz * 32 + ky) * 3 + (kx - 2));
     return {t[0], {t[1], t[2]}};
-}
-
-// ---------------------------------------------------------------------------
-// Per-lane constants of the forward/inverse stages (fixed for the whole walk:
-// lane (j, i) always handles row i of the field with offset j).
-// ---------------------------------------------------------------------------
-struct LaneConst {
-    int j, i, y0, kk;
-    float wy;          // w_y(y0 + 2i)
-    float2 ftw[4];     // radix-2 stage twiddles, h = 8, 4, 2, 1: exp(-2 pi i r / 2h)
-    float2 ptw;        // exp(-2 pi i kk y0 / 32)
-};
-
-__device__ __forceinline__ LaneConst lane_const(int lane, int tileY, int swap)
-{
-    LaneConst c;
-    c.j = lane >> 4;
-    c.i = lane & 15;
-    c.y0 = ((c.j ^ swap) - tileY) & 1;   // field offset (j ^ swap): its rows have that parity
-    c.kk = rev4(c.i);
-    c.wy = c3_wy[c.y0][c.i];
-    int s = 0;
-#pragma unroll
-    for (int h = 8; h >= 1; h >>= 1, s++) c.ftw[s] = c3_tw16[(c.i & (h - 1)) * (8 / h)];
-    c.ptw = c.y0 ? c3_tw32[c.kk] : make_float2(1.f, 0.f);
-    return c;
-}
-
-// ---------------------------------------------------------------------------
-// Forward X and Y stages of fields 2q (half-warp 0) and 2q+1 (half-warp 1).
-// Writes S_f[kappa(l)][kx] into the shared window slot f & 7 and the bound
-// terms of both fields into bnd[f & 7].
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void forward_pair(const T3Params &P, int q, int tileX, int tileY, const LaneConst &LC,
-                                             int lane, float2 *win /* [8][5][32] */, float *bnd /* [8][8] */)
-{
-    const int f = 2 * q + LC.j;
-    const int L = tileY + LC.y0 + 2 * LC.i;   // frame line of this lane's row
-    const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
-    const bool valid = (fp != nullptr) && (L >= P.fafl) && (L <= P.lafl);
-
-    // Row samples with black and the row mean removed, folded about the
-    // window's centre: s_x = a_x + a_15-x - 2*mean, d_x = a_x - a_15-x
-    // (exact in FP32); the window weight wy is applied to both.
-    float2 sd[8];   // (s_x, d_x)
-    float rowl1 = 0.0f;
-    if (valid) {
-        const uint16_t *row = fp + (long long)(L >> 1) * P.fw;
-        int a[16];
-        int sum = 0;
-        if (tileX >= 0 && (L >> 1) >= 1 && ((L >> 1) + 1 < P.fh || tileX + 18 <= P.fw)) {
-            // Rows start on any 2-byte boundary (odd line and field
-            // lengths): nine aligned 32-bit words cover the 16 samples, and a
-            // funnel shift by 0 or 16 bits lines each pair up -- 9 loads
-            // instead of 16, each warp load touching 32 rows either way. The
-            // words span at most the sample before and two after the 16,
-            // inside the field: the row is not its first, and it is not the
-            // last unless the words end inside it.
-            const uintptr_t pa = reinterpret_cast<uintptr_t>(row + tileX);
-            const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
-            const unsigned sh = (unsigned)(pa & 2) * 8u;
-            uint32_t wd[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) wd[k] = __ldg(w + k);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t v = __funnelshift_r(wd[k], wd[k + 1], sh);
-                a[2 * k] = (int)(v & 0xFFFFu) - P.black;
-                a[2 * k + 1] = (int)(v >> 16) - P.black;
-            }
-#pragma unroll
-            for (int x = 0; x < 16; x++) sum += a[x];
-        } else {
-#pragma unroll
-            for (int x = 0; x < 16; x++) {
-                const int xx = max(tileX + x, -(L >> 1) * P.fw);   // never before the field start
-                a[x] = (int)__ldg(row + xx) - P.black;
-                sum += a[x];
-            }
-        }
-        const float m16 = (float)sum * 0.0625f;
-#pragma unroll
-        for (int x = 0; x < 8; x++) {
-            sd[x] = make_float2((float)(8 * (a[x] + a[15 - x]) - sum) * 0.125f, (float)(a[x] - a[15 - x]));
-            rowl1 = __fmaf_rn(c3_wx[x], fabsf((float)a[x] - m16) + fabsf((float)a[15 - x] - m16), rowl1);
-        }
-    } else {
-#pragma unroll
-        for (int x = 0; x < 8; x++) sd[x] = make_float2(0.f, 0.f);
-    }
-    rowl1 *= LC.wy;
-#pragma unroll
-    for (int h = 1; h < 16; h <<= 1) rowl1 += __shfl_xor_sync(0xffffffffu, rowl1, h);
-    const int fslot = f & 7;
-    if (LC.i == 0) bnd[8 * fslot + 5] = rowl1;
-    const int f0slot = (2 * q) & 7;
-
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        // column DFT bin kx = k+2 of this row (window and centre phase folded)
-        float2 X = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int x = 0; x < 8; x++) X = __ffma2_rn(c3_xf[k][x], sd[x], X);
-        X = __fmul2_rn(X, make_float2(LC.wy, LC.wy));
-        // bound term: sum over the field's rows of |X|_1
-        float A = l1(X);
-#pragma unroll
-        for (int h = 1; h < 16; h <<= 1) A += __shfl_xor_sync(0xffffffffu, A, h);
-        if (LC.i == 0) bnd[8 * fslot + k] = A;
-        // 16-point DFT over the half-warp's rows (radix-2 DIF; lane i ends
-        // with bin rev4(i))
-        int st = 0;
-#pragma unroll
-        for (int h = 8; h >= 1; h >>= 1, st++) {
-            const bool upper = (LC.i & h) != 0;
-            const float2 o = shfl_xor2(X, h);
-            X = upper ? cmul(sub2(o, X), LC.ftw[st]) : add2(X, o);
-        }
-        // parity twiddle: S[kk] = exp(-2 pi i kk y0/32) A[kk], S[kk+16] = (-1)^y0 S[kk];
-        // swap halves so lane l holds both fields at ky = kappa(l)
-        const float2 lo = cmul(X, LC.ptw);
-        const float2 hi = LC.y0 ? make_float2(-lo.x, -lo.y) : lo;
-        const float2 recv = shfl_xor2(LC.j ? lo : hi, 16);
-        win[(f0slot * 5 + k) * 32 + lane] = LC.j ? recv : lo;            // field 2q
-        win[((f0slot + 1) * 5 + k) * 32 + lane] = LC.j ? hi : recv;      // field 2q+1
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -313,63 +176,6 @@ __device__ __forceinline__ void x_row_pair(const uint16_t *field, long long base
     xb = {df_from_fixed60(e[0] - o[0], e[1] - o[1]), df_from_fixed60(o[2] - e[2], o[3] - e[3])};
 }
 
-// ---------------------------------------------------------------------------
-// Exact (double-float) magnitudes of bin b = (kzb, kyb, kxb) and its mirror
-// r of Z tile T(2m). All 32 lanes cooperate; every lane returns the result.
-// ---------------------------------------------------------------------------
-__device__ __noinline__ void exact_pair(const T3Params &P, int m, int tileX, int tileY, int kzb, int kyb, int kxb,
-                                        df &mb, df &mr)
-{
-    const int lane = threadIdx.x & 31;
-    const int kzr = (10 - kzb) & 7, kyr = (40 - kyb) & 31;
-    const int z = lane >> 2;
-    const int part = lane & 3;
-    const int f = 2 * m + z;
-    const int p = (f & 1) ^ P.swap;   // SourceField::getOffset of window field f
-    const int y0 = (p - tileY) & 1;
-    dfc accb = {{0.f, 0.f}, {0.f, 0.f}}, accr = accb;
-    const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
-    if (fp != nullptr) {
-        for (int r4 = 0; r4 < 4; r4++) {
-            const int i = part * 4 + r4;
-            const int y = y0 + 2 * i;
-            const int L = tileY + y;
-            if (L < P.fafl || L > P.lafl) continue;
-            const long long base = (long long)(L >> 1) * P.fw + tileX;   // within the field
-            dfc xb, xr;
-            x_row_pair(fp, base, (long long)P.fh * P.fw, P.black, kxb, xb, xr);
-            const df wy = {c3_dfwy[y][0], c3_dfwy[y][1]};
-            dfc cb = dfc_tw32(kyb * y), cr = dfc_tw32(kyr * y);
-            cb.re = df_mul(cb.re, wy); cb.im = df_mul(cb.im, wy);
-            cr.re = df_mul(cr.re, wy); cr.im = df_mul(cr.im, wy);
-            accb = dfc_add(accb, dfc_mul(xb, cb));
-            accr = dfc_add(accr, dfc_mul(xr, cr));
-        }
-    }
-    accb = dfc_add(accb, dfc_shfl_xor(accb, 1));
-    accb = dfc_add(accb, dfc_shfl_xor(accb, 2));
-    accr = dfc_add(accr, dfc_shfl_xor(accr, 1));
-    accr = dfc_add(accr, dfc_shfl_xor(accr, 2));
-    {
-        const df wz = {c3_dfwz[z][0], c3_dfwz[z][1]};
-        dfc tb = dfc_tw32(4 * ((kzb * z) & 7)), tr = dfc_tw32(4 * ((kzr * z) & 7));
-        tb.re = df_mul(tb.re, wz); tb.im = df_mul(tb.im, wz);
-        tr.re = df_mul(tr.re, wz); tr.im = df_mul(tr.im, wz);
-        accb = dfc_mul(accb, tb);
-        accr = dfc_mul(accr, tr);
-    }
-    // sum the 8 fields (lanes differing in bits 2..4; the 4 lanes of a field
-    // hold identical values, so only lane bits 2..4 are combined)
-    accb = dfc_add(accb, dfc_shfl_xor(accb, 4));
-    accb = dfc_add(accb, dfc_shfl_xor(accb, 8));
-    accb = dfc_add(accb, dfc_shfl_xor(accb, 16));
-    accr = dfc_add(accr, dfc_shfl_xor(accr, 4));
-    accr = dfc_add(accr, dfc_shfl_xor(accr, 8));
-    accr = dfc_add(accr, dfc_shfl_xor(accr, 16));
-    mb = dfc_abs2(accb);
-    mr = dfc_abs2(accr);
-}
-
 // sim(a, b, t) = !(a < b t || b < a t) evaluated in double-float
 __device__ __forceinline__ bool df_sim(df a, df b, df t)
 {
@@ -378,102 +184,438 @@ __device__ __forceinline__ bool df_sim(df a, df b, df t)
     return !(df_sign(d1) < 0 || df_sign(d2) < 0);
 }
 
-// 8-point forward DFT of windowed column values (natural order in/out),
-// radix-2 with paired FP32 butterflies; the twiddles 1 and -i are applied
-// exactly, exp(-i pi/4) and exp(-3i pi/4) by complex multiplication.
-__device__ __forceinline__ void dft8_fwd(const float2 (&in)[8], float2 (&out)[8])
-{
-    float2 a[8];
-#pragma unroll
-    for (int z = 0; z < 8; z++) a[z] = __fmul2_rn(in[z], make_float2(c3_wz[z], c3_wz[z]));
-    // stage 1: pairs (z, z+4), twiddles exp(-2 pi i z / 8)
-    float2 b[8];
-#pragma unroll
-    for (int z = 0; z < 4; z++) b[z] = add2(a[z], a[z + 4]);
-    b[4] = sub2(a[0], a[4]);
-    b[5] = cmul(sub2(a[1], a[5]), c3_tw32[4]);
-    b[6] = mul_negi(sub2(a[2], a[6]));
-    b[7] = cmul(sub2(a[3], a[7]), c3_tw32[12]);
-    // stage 2: pairs (z, z+2) within each half, twiddles 1 and -i
-    float2 c[8];
-#pragma unroll
-    for (int hb = 0; hb < 8; hb += 4) {
-        c[hb] = add2(b[hb], b[hb + 2]);
-        c[hb + 1] = add2(b[hb + 1], b[hb + 3]);
-        c[hb + 2] = sub2(b[hb], b[hb + 2]);
-        c[hb + 3] = mul_negi(sub2(b[hb + 1], b[hb + 3]));
-    }
-    // stage 3: pairs (z, z+1); outputs in bit-reversed order
-    float2 d[8];
-#pragma unroll
-    for (int z = 0; z < 8; z += 2) {
-        d[z] = add2(c[z], c[z + 1]);
-        d[z + 1] = sub2(c[z], c[z + 1]);
-    }
-    out[0] = d[0]; out[4] = d[1]; out[2] = d[2]; out[6] = d[3];
-    out[1] = d[4]; out[5] = d[5]; out[3] = d[6]; out[7] = d[7];
-}
-
 // ---------------------------------------------------------------------------
-// The kernel
+// The walk: layout and per-lane constants
 // ---------------------------------------------------------------------------
+// One warp walks one tile position through a chunk of frames, two fields (one
+// frame) a step. What bounds it is the number of instructions it issues, so
+// each stage's data is laid out where that stage needs no exchange:
+//
+//  * X stage: lane (j, i) owns row i of field j of the pair. Component j of
+//    every packed pair is that field.
+//  * Y stage: lanes 0..19 own one (kx, quarter) each: 4 of the column's 16
+//    points, both fields packed in f32x2 registers, two radix-4 passes with
+//    one exchange through shared memory. The shuffle version ran the 4
+//    radix-2 stages across 16 lanes: 8 shuffles, 8 selects and the twiddles
+//    of both halves per column and field.
+//  * Z stage: a field's spectrum at ky + 16 is +- its value at ky, the sign
+//    by the parity of its rows, which alternates with z. So a tile's bin at
+//    (kz, ky + 16) is +- the bin at (kz + 4, ky), bit for bit in the radix-2
+//    order used here: 16 values of ky are transformed, compared and masked,
+//    and the other 16 reuse them. Half-warp h takes the columns kx = 2 + h
+//    and, at the mirror ky, 6 - h: both bins of every pair the filter
+//    compares are in one lane, no shuffles of magnitudes or decisions. kx = 4
+//    mirrors onto itself; its pass runs all 32 ky.
+//  * Signs: everything at ky >= 16 is kept with the sign of odd z, which
+//    is the true value or its negative for the whole launch; the inverse Y
+//    stage folds the two halves with the factors (1, -1).
+//
+// Shared memory per warp (float4 units): the window [4 pairs][5 kx][16]
+// as (re0, re1, im0, im1) of the pair's two fields, the Z carries
+// [m & 1][5 kx][32] as (slice 4, slice 5), an exchange buffer of 5 x 20 (rows
+// padded by 4: the columns of a quarter-warp fall on different banks), the
+// output spectra [5][32], and the bound terms.
+//
+// The inverse Y stage of one step runs together with the forward Y stage of
+// the next: two independent chains through the same two exchanges.
+//
+// Measured against the walk before it (one ky per lane in the Z stage, shuffle
+// DFTs in the Y stages, every bin's guard band in the loop): 2,671 -> 1,551
+// warp instructions a step, 526 -> 363 us for 60 fields. The kx pairs unrolled
+// into straight-line code, four blocks a SM at 128 registers (spills) and two
+// warps a block all measured slower.
 constexpr int kWarps3 = 4;
 constexpr float kBoundFactor = 2.0f;   // guard band, in units of the per-bin error estimate
 constexpr float kEps32 = 5.9604645e-8f;
 // a + b + E^2 + rE^2 below this (with a margin for the FP32 magnitudes)
 // keeps the effect of a decision under 1/4 sample unit: (4/4096) * 256 = 1/4
 constexpr float kTinyPair = 65000.0f;
-constexpr int kWarpSmemF2 = 8 * 5 * 32 + 2 * 2 * 5 * 32 + 32;   // float2 units per warp
-
-struct Col {
-    float2 Y[8];
-    float mag[8], ab[8], E;
-};
-
-// 8-point Z DFT of one (ky, kx) column from the shared window, with its
-// magnitudes, L1 magnitudes and error bound.
-__device__ __forceinline__ void z_column(const float2 *win, int m, int k, int lane, float ek, Col &c)
+constexpr int kWinF4 = 4 * 5 * 16;
+constexpr int kCarryF4 = 2 * 5 * 32;
+constexpr int kExchF4 = 5 * 20;
+constexpr int kOutF4 = 5 * 32;         // output spectra; then an exchange at 0, then the output rows at kRowsAt
+constexpr int kRowsAt = kOutF4 - 5 * 20;
+constexpr int kBndF4 = 4 * 4;          // [4 pairs][8] float2: kx 0..4 and the row term at 5
+constexpr int kWarpF4 = kWinF4 + kCarryF4 + kExchF4 + kOutF4 + kBndF4;
+constexpr int kTwF4 = 4 * 11;          // Y twiddles per quarter r, per block
+constexpr int kThrF4 = 3 * 8 * 32 / 4; // squared per-bin thresholds, per block (per-bin walks only)
+constexpr size_t walk_smem(bool per_bin)
 {
-    float2 col[8];
-    float B = 0.f;
-#pragma unroll
-    for (int z = 0; z < 8; z++) {
-        col[z] = win[((((2 * m + z) & 7) * 5) + k) * 32 + lane];
-        B = __fmaf_rn(c3_wz[z], l1(col[z]), B);
-    }
-    dft8_fwd(col, c.Y);
-#pragma unroll
-    for (int kz = 0; kz < 8; kz++) {
-        c.mag[kz] = __fmaf_rn(c.Y[kz].x, c.Y[kz].x, c.Y[kz].y * c.Y[kz].y);
-        c.ab[kz] = l1(c.Y[kz]);
-    }
-    c.E = kBoundFactor * kEps32 * (ek + B);
+    return sizeof(float4) * (size_t)(kWarps3 * kWarpF4 + kTwF4 + (per_bin ? kThrF4 : 0));
 }
 
-// Mask a column, inverse-DFT it to Z slices 0, 1, 4, 5 and overlap-add:
-// R(field 2m) = slice 0 + carried slice 4 of tile 2m-4, R(2m+1) = slice 1 +
-// carried slice 5; then carry this tile's slices 4, 5 for frame m+2.
-__device__ __forceinline__ void z_inverse(const float2 (&Y)[8], unsigned keep, float2 *carry /* [2][5][32] */,
-                                          float2 *RA, float2 *RB /* [5][32] each */, int k, int lane)
+// A position p of 16 or 32 is stored at p ^ ((p >> 2) & 3): lanes that read
+// or write 4r + e for fixed e and lanes that access consecutive positions
+// both fall on distinct banks.
+__device__ __forceinline__ int swz(int p) { return p ^ ((p >> 2) & 3); }
+
+struct LaneConst {
+    int j, i;             // field of the pair, row
+    float wy;             // w_y(y0 + 2i), y0 the parity of the field's rows
+    int rowL;             // frame line of this lane's row
+    bool row_ok, row_fast;
+    long long row_off;    // its first sample within the field
+    int ky;               // of position lane & 15 (below 16)
+    int posA, posB;       // window positions of ky and its mirror
+    int laneB;            // position (of 32) of the mirror ky
+    float2 wzB[4];        // w_z of fields 2q, 2q+1, odd fields negated for a mirror ky >= 16
+};
+
+__device__ __forceinline__ LaneConst lane_const(const T3Params &P, int lane, int tileX, int tileY)
 {
-    float2 y[8];
+    LaneConst c;
+    c.j = lane >> 4;
+    c.i = lane & 15;
+    const int odd = 1 ^ ((P.swap ^ tileY) & 1);   // the field whose rows have parity 1 within the tile
+    const int y0 = c.j == odd;
+    c.wy = c3_wy[y0][c.i];
+    c.rowL = tileY + y0 + 2 * c.i;
+    c.row_ok = c.rowL >= P.fafl && c.rowL <= P.lafl;
+    const int fl = c.rowL >> 1;
+    // Nine aligned words around the row stay inside the field: the row is not
+    // its first, and it is not the last unless the words end inside it.
+    c.row_fast = tileX >= 0 && fl >= 1 && (fl + 1 < P.fh || tileX + 18 <= P.fw);
+    c.row_off = (long long)fl * P.fw + tileX;
+    c.ky = rev4(c.i);
+    c.laneB = kappa((40 - c.ky) & 31);
+    c.posA = swz(c.i);
+    c.posB = swz(c.laneB & 15);
 #pragma unroll
-    for (int kz = 0; kz < 8; kz++) y[kz] = ((keep >> kz) & 1u) ? Y[kz] : make_float2(0.f, 0.f);
-    const float2 E0 = add2(add2(add2(y[0], y[2]), y[4]), y[6]);
-    const float2 O0 = add2(add2(add2(y[1], y[3]), y[5]), y[7]);
-    // slice 1: even part y0 + i y2 - y4 - i y6; odd part with powers of exp(+i pi/4)
-    const float2 E1 = make_float2(y[0].x - y[2].y - y[4].x + y[6].y, y[0].y + y[2].x - y[4].y - y[6].x);
-    const float2 o1 = cmul(y[1], make_float2(c3_tw32[4].x, -c3_tw32[4].y));
-    const float2 o3 = cmul(y[3], make_float2(c3_tw32[12].x, -c3_tw32[12].y));
-    const float2 o5 = cmul(y[5], make_float2(c3_tw32[20].x, -c3_tw32[20].y));
-    const float2 o7 = cmul(y[7], make_float2(c3_tw32[28].x, -c3_tw32[28].y));
-    const float2 O1 = add2(add2(add2(o1, o3), o5), o7);
-    const int i4 = k * 32 + lane, i5 = (5 + k) * 32 + lane;
-    const float2 c4 = carry[i4], c5 = carry[i5];
-    RA[k * 32 + lane] = add2(add2(E0, O0), c4);
-    RB[k * 32 + lane] = add2(add2(E1, O1), c5);
-    carry[i4] = sub2(E0, O0);
-    carry[i5] = sub2(E1, O1);
+    for (int q = 0; q < 4; q++)
+        c.wzB[q] = make_float2(c3_wz[2 * q], c.laneB >= 16 ? -c3_wz[2 * q + 1] : c3_wz[2 * q + 1]);
+    return c;
+}
+
+// w_z of fields 2q, 2q+1 of a Z tile for a ky below 16 (high = false) or not
+__device__ __forceinline__ void z_window(float2 (&wz)[4], bool high)
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++) wz[q] = make_float2(c3_wz[2 * q], high ? -c3_wz[2 * q + 1] : c3_wz[2 * q + 1]);
+}
+
+// Both fields' complex values, packed: (re of component 0, of component 1).
+struct cp2 {
+    float2 re, im;
+};
+__device__ __forceinline__ cp2 cadd(cp2 a, cp2 b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
+__device__ __forceinline__ cp2 csub(cp2 a, cp2 b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
+__device__ __forceinline__ cp2 cp_of(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+__device__ __forceinline__ float4 f4_of(cp2 v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
+// A twiddle of each component: x = (x0, x1), y = (y0, y1), n = -y (rounds as
+// cmul does per component); conj: by the conjugate
+struct tw2 {
+    float2 x, y, n;
+};
+__device__ __forceinline__ cp2 ctw(cp2 a, tw2 t, bool conj)
+{
+    const float2 y = conj ? t.n : t.y, n = conj ? t.y : t.n;
+    return {__ffma2_rn(a.re, t.x, __fmul2_rn(a.im, n)), __ffma2_rn(a.re, y, __fmul2_rn(a.im, t.x))};
+}
+__device__ __forceinline__ float2 cmulc(float2 a, float2 b)   // a * conj(b), rounded as cmul(a, conj b)
+{
+    return make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)), __fmaf_rn(a.x, -b.y, __fmul_rn(a.y, b.x)));
+}
+
+// The block's Y twiddles, per quarter r: exp(-2 pi i n / 16) for n = r, r + 4
+// and 2r in both components, then for the positions 4r + e (bin k =
+// rev4(4r + e)) exp(-2 pi i k / 32) in the component of the field with odd
+// rows and 1 in the other. Entry v of quarter r: (x0, x1, y0, y1) at
+// tw[11 r + v], (-y0, -y1) in half v & 1 of tw[11 r + 7 + v / 2].
+__device__ __forceinline__ void fill_twiddles(const T3Params &P, float4 *tw)
+{
+    const int odd = 1 ^ ((P.swap ^ P.tileY0) & 1);   // tile rows start 16 lines apart
+    for (int t = threadIdx.x; t < 4 * 7; t += blockDim.x) {
+        const int r = t / 7, v = t % 7;
+        float2 w = v < 3 ? c3_tw16[v == 0 ? r : v == 1 ? r + 4 : 2 * r] : c3_tw32[rev4(4 * r + v - 3)];
+        float2 w0 = w, w1 = w;
+        if (v >= 3) (odd ? w0 : w1) = make_float2(1.f, 0.f);
+        tw[11 * r + v] = make_float4(w0.x, w1.x, w0.y, w1.y);
+        reinterpret_cast<float2 *>(tw + 11 * r + 7)[v] = make_float2(-w0.y, -w1.y);
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ tw2 twiddle(const float4 *tw, int r, int v)
+{
+    const float4 a = tw[11 * r + v];
+    return {make_float2(a.x, a.y), make_float2(a.z, a.w), reinterpret_cast<const float2 *>(tw + 11 * r + 7)[v]};
+}
+
+constexpr unsigned kYLanes = 0xFFFFFu;   // lanes 0..19 run the Y stages
+
+// The 16 samples of this lane's row of field 2q + j, as words that a funnel
+// shift lines up.
+struct RowWords {
+    uint32_t w[9];
+    unsigned sh;
+    bool valid;   // else the row is black: outside the capture or the active lines
+};
+
+__device__ __forceinline__ void load_row(const T3Params &P, int q, const LaneConst &LC, RowWords &r)
+{
+    const int f = 2 * q + LC.j;
+    const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
+    r.valid = fp != nullptr && LC.row_ok;
+    r.sh = 0;
+    if (!r.valid) return;
+    if (LC.row_fast) {
+        // Rows start on any 2-byte boundary (odd line and field lengths):
+        // nine aligned 32-bit words cover the 16 samples and a funnel
+        // shift by 0 or 16 bits lines each pair up.
+        const uintptr_t pa = reinterpret_cast<uintptr_t>(fp + LC.row_off);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
+        r.sh = (unsigned)(pa & 2) * 8u;
+#pragma unroll
+        for (int k = 0; k < 9; k++) r.w[k] = __ldg(w + k);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {   // never before the field start
+            const long long e = LC.row_off + 2 * k;
+            r.w[k] = (uint32_t)__ldg(fp + (e < 0 ? 0 : e)) | ((uint32_t)__ldg(fp + (e + 1 < 0 ? 0 : e + 1)) << 16);
+        }
+        r.w[8] = 0;
+    }
+}
+
+// Forward X stage of fields 2q and 2q+1: this lane's row into the exchange
+// buffer, and R, the L1 norm of the field's DC-removed windowed rows, into bnd.
+__device__ __forceinline__ void x_forward(const RowWords &row, int q, const LaneConst &LC, float4 *exch, float2 *bnd)
+{
+    // Row samples with the row mean removed, folded about the window's
+    // centre: s_x = a_x + a_15-x - 2*mean, d_x = a_x - a_15-x. Both are exact
+    // in FP32 and free of the black level. |a_x - mean| + |a_15-x - mean| is
+    // max(|s_x|, |d_x|).
+    float2 sd[8];   // (s_x, d_x)
+    float rowl1 = 0.0f;
+    if (row.valid) {
+        uint32_t v[8];   // samples 2k, 2k+1
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = __funnelshift_r(row.w[k], row.w[k + 1], row.sh);
+        // 2^23 + a from the sample's bits; subtracting 2^24 from one side of
+        // each sum leaves a_x + a_15-x exactly
+        float2 t[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 p = make_float2(__uint_as_float(__byte_perm(v[k], 0x4B000000u, 0x7610)),
+                                         __uint_as_float(__byte_perm(v[k], 0x4B000000u, 0x7632)));
+            const float2 o = make_float2(__uint_as_float(__byte_perm(v[7 - k], 0x4B000000u, 0x7632)),
+                                         __uint_as_float(__byte_perm(v[7 - k], 0x4B000000u, 0x7610)));
+            sd[2 * k].y = __fsub_rn(p.x, o.x);
+            sd[2 * k + 1].y = __fsub_rn(p.y, o.y);
+            t[k] = add2(add2(p, make_float2(-16777216.f, -16777216.f)), o);
+        }
+        const float2 u = add2(add2(t[0], t[1]), add2(t[2], t[3]));
+        const float mean2 = __fmul_rn(__fadd_rn(u.x, u.y), 0.125f);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            sd[2 * k].x = __fsub_rn(t[k].x, mean2);
+            sd[2 * k + 1].x = __fsub_rn(t[k].y, mean2);
+        }
+#pragma unroll
+        for (int x = 0; x < 8; x++) rowl1 = __fmaf_rn(c3_wx[x], fmaxf(fabsf(sd[x].x), fabsf(sd[x].y)), rowl1);
+    } else {
+#pragma unroll
+        for (int x = 0; x < 8; x++) sd[x] = make_float2(0.f, 0.f);
+    }
+    rowl1 *= LC.wy;
+#pragma unroll
+    for (int h = 1; h < 16; h <<= 1) rowl1 += __shfl_xor_sync(0xffffffffu, rowl1, h);
+    float *bq = reinterpret_cast<float *>(bnd + 8 * (q & 3));
+    if (LC.i == 0) bq[2 * 5 + LC.j] = rowl1;
+
+    // column DFT bin kx = k+2 of this row (window and centre phase folded)
+    float *xr = reinterpret_cast<float *>(exch) + 4 * LC.i + LC.j;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        float2 X = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int x = 0; x < 8; x++) X = __ffma2_rn(c3_xf[k][x], sd[x], X);
+        X = __fmul2_rn(X, make_float2(LC.wy, LC.wy));
+        xr[80 * k] = X.x;
+        xr[80 * k + 2] = X.y;
+    }
+}
+
+// Y stages, lanes 0..19: the forward one of fields 2q and 2q+1 from their
+// rows in `exch` to window slot q & 3 (and A per kx, the L1 norm of the
+// column-DFT outputs over the rows, into bnd); with INV the inverse one of the
+// output spectra R (re0, re1, im0, im1), their rows into R + kRowsAt.
+template <bool INV>
+__device__ __forceinline__ void y_stages(int q, const LaneConst &LC, int lane, float4 *win, float4 *exch, float4 *R,
+                                         float2 *bnd, const float4 *tw)
+{
+    const int k = lane >> 2, r = lane & 3;
+    float4 *x = exch + 20 * k, *y = R + 20 * k;
+    cp2 a[4], G[4];
+#pragma unroll
+    for (int n = 0; n < 4; n++) a[n] = cp_of(x[r + 4 * n]);
+    const tw2 t0 = twiddle(tw, r, 0), t1 = twiddle(tw, r, 1), t2 = twiddle(tw, r, 2);
+    if (INV) {
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+            // fold ky = kk and kk + 16, then exp(+i pi kk / 16) for the odd field
+            const float4 *s = R + 32 * k + 4 * r + (n ^ r);
+            const cp2 lo = cp_of(s[0]), hi = cp_of(s[16]);
+            G[n] = ctw({__ffma2_rn(hi.re, make_float2(1.f, -1.f), lo.re), __ffma2_rn(hi.im, make_float2(1.f, -1.f), lo.im)},
+                       twiddle(tw, r, 3 + n), true);
+        }
+    }
+    float A0 = 0.f, A1 = 0.f;
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+        A0 += fabsf(a[n].re.x) + fabsf(a[n].im.x);
+        A1 += fabsf(a[n].re.y) + fabsf(a[n].im.y);
+    }
+#pragma unroll
+    for (int h = 1; h < 4; h <<= 1) {
+        A0 += __shfl_xor_sync(kYLanes, A0, h);
+        A1 += __shfl_xor_sync(kYLanes, A1, h);
+    }
+    if (r == 0) bnd[8 * (q & 3) + k] = make_float2(A0, A1);
+    // Forward: 16-point DFT over the rows, radix-2 DIF: spans 8 and 4 over
+    // the rows r + 4n, spans 2 and 1 over the positions 4r + e; position p
+    // ends with bin rev4(p). Inverse: bit-reversed input to natural order
+    // (DIT), spans 1 and 2 over 4r + e, spans 4 and 8 over r + 4n.
+    const cp2 u0 = cadd(a[0], a[2]), u1 = cadd(a[1], a[3]);
+    const cp2 v0 = ctw(csub(a[0], a[2]), t0, false), v1 = ctw(csub(a[1], a[3]), t1, false);
+    __syncwarp(kYLanes);   // rows and spectra have been read: both buffers may be written
+    x[0 + r] = f4_of(cadd(u0, u1));
+    x[4 + (r ^ 1)] = f4_of(ctw(csub(u0, u1), t2, false));
+    x[8 + (r ^ 2)] = f4_of(cadd(v0, v1));
+    x[12 + (r ^ 3)] = f4_of(ctw(csub(v0, v1), t2, false));
+    if (INV) {
+        const cp2 w0 = cadd(G[0], G[1]), w1 = csub(G[0], G[1]), w2 = cadd(G[2], G[3]), d3 = csub(G[2], G[3]);
+        y[4 * r + (0 ^ r)] = f4_of(cadd(w0, w2));
+        y[4 * r + (2 ^ r)] = f4_of(csub(w0, w2));
+        // the odd branch of span 2 times exp(+i pi/2): (-d3.im, d3.re)
+        y[4 * r + (1 ^ r)] = f4_of({sub2(w1.re, d3.im), add2(w1.im, d3.re)});
+        y[4 * r + (3 ^ r)] = f4_of({add2(w1.re, d3.im), sub2(w1.im, d3.re)});
+    }
+    __syncwarp(kYLanes);
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+        a[n] = cp_of(x[4 * r + (n ^ r)]);
+        if (INV) G[n] = cp_of(y[4 * n + (r ^ n)]);
+    }
+    if (INV) __syncwarp(kYLanes);   // the output rows overlap the exchange
+    const cp2 w0 = cadd(a[0], a[2]), w1 = cadd(a[1], a[3]), w2 = csub(a[0], a[2]), d3 = csub(a[1], a[3]);
+    // the odd branch of span 2 times exp(-i pi/2): (d3.im, -d3.re)
+    const cp2 o[4] = {cadd(w0, w1), csub(w0, w1), {add2(w2.re, d3.im), sub2(w2.im, d3.re)},
+                      {sub2(w2.re, d3.im), add2(w2.im, d3.re)}};
+    // parity twiddle of the odd field: S[kk] = exp(-2 pi i kk/32) A[kk]
+    float4 *dst = win + (5 * (q & 3) + k) * 16 + 4 * r;
+#pragma unroll
+    for (int n = 0; n < 4; n++) dst[n ^ r] = f4_of(ctw(o[n], twiddle(tw, r, 3 + n), false));
+    if (INV) {
+        const cp2 f1 = ctw(G[1], t2, true), f3 = ctw(G[3], t2, true);
+        const cp2 g0 = cadd(G[0], f1), g1 = csub(G[0], f1);
+        const cp2 g2 = ctw(cadd(G[2], f3), t0, true), g3 = ctw(csub(G[2], f3), t1, true);
+        float4 *z = y + kRowsAt;
+        z[r] = f4_of(cadd(g0, g2));
+        z[r + 4] = f4_of(cadd(g1, g3));
+        z[r + 8] = f4_of(csub(g0, g2));
+        z[r + 12] = f4_of(csub(g1, g3));
+    }
+}
+
+// 8-point forward DFT of one windowed column (natural order out): radix-2
+// DIF, the first two stages on the packed fields (z, z+1), the twiddles 1 and
+// -i applied exactly, exp(-i pi/4) and exp(-3i pi/4) by complex multiplication.
+__device__ __forceinline__ void z_dft(const float4 *win, int m, int k, int pos, const float2 (&wz)[4], float2 (&Y)[8])
+{
+    cp2 a[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const cp2 v = cp_of(win[(5 * ((m + q) & 3) + k) * 16 + pos]);
+        a[q] = {__fmul2_rn(v.re, wz[q]), __fmul2_rn(v.im, wz[q])};
+    }
+    const cp2 b01 = cadd(a[0], a[2]), b23 = cadd(a[1], a[3]);   // b0, b1 / b2, b3
+    const cp2 d01 = csub(a[0], a[2]), d23 = csub(a[1], a[3]);   // a0 - a4, a1 - a5 / a2 - a6, a3 - a7
+    const float2 b5 = cmul(make_float2(d01.re.y, d01.im.y), c3_tw32[4]);
+    const float2 b7 = cmul(make_float2(d23.re.y, d23.im.y), c3_tw32[12]);
+    const cp2 c01 = cadd(b01, b23), c23 = csub(b01, b23);       // c0, c1 / c2, b1 - b3
+    Y[0] = make_float2(__fadd_rn(c01.re.x, c01.re.y), __fadd_rn(c01.im.x, c01.im.y));
+    Y[4] = make_float2(__fsub_rn(c01.re.x, c01.re.y), __fsub_rn(c01.im.x, c01.im.y));
+    Y[2] = make_float2(__fadd_rn(c23.re.x, c23.im.y), __fsub_rn(c23.im.x, c23.re.y));   // c3 = -i (b1 - b3)
+    Y[6] = make_float2(__fsub_rn(c23.re.x, c23.im.y), __fadd_rn(c23.im.x, c23.re.y));
+    // b4 = a0 - a4, b6 = -i (a2 - a6)
+    const float2 c4 = make_float2(__fadd_rn(d01.re.x, d23.im.x), __fsub_rn(d01.im.x, d23.re.x));
+    const float2 c6 = make_float2(__fsub_rn(d01.re.x, d23.im.x), __fadd_rn(d01.im.x, d23.re.x));
+    const float2 c5 = add2(b5, b7), v = sub2(b5, b7);           // c7 = -i v
+    Y[1] = add2(c4, c5);
+    Y[5] = sub2(c4, c5);
+    Y[3] = make_float2(__fadd_rn(c6.x, v.y), __fsub_rn(c6.y, v.x));
+    Y[7] = make_float2(__fsub_rn(c6.x, v.y), __fadd_rn(c6.y, v.x));
+}
+
+__device__ __forceinline__ float mag2(float2 y) { return __fmaf_rn(y.x, y.x, __fmul_rn(y.y, y.y)); }
+
+// Inverse Z of one masked column to slices 0, 1, 4, 5: the even and odd parts
+// of slices 0 and 1, each a sum in the order of kz.
+struct ZInverse {
+    float2 E0, E1, O0, O1;
+    // y: the masked bins; o[i]: bin 2i + 1 times exp(+2 pi i (2i + 1) / 8)
+    __device__ __forceinline__ void sum(const float2 (&y)[8], const float2 (&o)[4])
+    {
+        E0 = add2(add2(add2(y[0], y[2]), y[4]), y[6]);
+        O0 = add2(add2(add2(y[1], y[3]), y[5]), y[7]);
+        // slice 1: even part y0 + i y2 - y4 - i y6
+        E1.x = __fadd_rn(__fsub_rn(__fsub_rn(y[0].x, y[2].y), y[4].x), y[6].y);
+        E1.y = __fsub_rn(__fsub_rn(__fadd_rn(y[0].y, y[2].x), y[4].y), y[6].x);
+        O1 = add2(add2(add2(o[0], o[1]), o[2]), o[3]);
+    }
+    // the sums of ky + 16 where its masked bins are those of ky moved by 4
+    // (O1 negated: exp(2 pi i (kz + 4) / 8) = -exp(2 pi i kz / 8))
+    __device__ __forceinline__ void sum_moved(const float2 (&y)[8], const float2 (&o)[4])
+    {
+        const float2 ym[8] = {y[4], y[5], y[6], y[7], y[0], y[1], y[2], y[3]};
+        const float2 om[4] = {o[2], o[3], o[0], o[1]};
+        sum(ym, om);
+        O1 = make_float2(-O1.x, -O1.y);
+    }
+    // R(field 2m) = slice 0 + carried slice 4 of tile 2m-4, R(2m+1) = slice 1
+    // + carried slice 5; then carry this tile's slices 4, 5 for frame m+2.
+    __device__ __forceinline__ void finish(float4 *carry, float4 *R, int k, int at) const
+    {
+        const float4 c = carry[32 * k + at];
+        const float2 s0 = add2(E0, O0), d0 = sub2(E0, O0);
+        const float2 s1 = make_float2(__fadd_rn(E1.x, O1.x), __fadd_rn(E1.y, O1.y));
+        const float2 d1 = make_float2(__fsub_rn(E1.x, O1.x), __fsub_rn(E1.y, O1.y));
+        R[32 * k + swz(at)] = make_float4(__fadd_rn(s0.x, c.x), __fadd_rn(s1.x, c.z), __fadd_rn(s0.y, c.y),
+                                          __fadd_rn(s1.y, c.w));
+        carry[32 * k + at] = make_float4(d0.x, d0.y, d1.x, d1.y);
+    }
+};
+
+__device__ __forceinline__ void z_rotate(const float2 (&y)[8], float2 (&o)[4])
+{
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[i] = cmulc(y[2 * i + 1], c3_tw32[4 * (2 * i + 1)]);
+}
+
+// Masks column Y at ky (position `at`) by k and at ky + 16 by kh, inverse Z
+// and overlap-add of both. MOVED: kh is k moved by 4, the sums share the
+// masked bins.
+template <bool MOVED>
+__device__ __forceinline__ void z_inverse(const float2 (&Y)[8], const float (&k)[8], const float (&kh)[8],
+                                          float4 *carry, float4 *R, int col, int at)
+{
+    float2 y[8], o[4];
+#pragma unroll
+    for (int z = 0; z < 8; z++) y[z] = __fmul2_rn(Y[z], make_float2(k[z], k[z]));
+    z_rotate(y, o);
+    ZInverse Z;
+    Z.sum(y, o);
+    Z.finish(carry, R, col, at);
+    if (MOVED) {
+        Z.sum_moved(y, o);
+    } else {
+        float2 yh[8];
+#pragma unroll
+        for (int z = 0; z < 8; z++) yh[z] = __fmul2_rn(Y[z ^ 4], make_float2(kh[z], kh[z]));
+        z_rotate(yh, o);
+        Z.sum(yh, o);
+    }
+    Z.finish(carry, R, col, at ^ 16);
 }
 
 __device__ __forceinline__ bool fsim(float a, float b, float t) { return (__fmaf_rn(-b, t, a) >= 0.f) && (__fmaf_rn(-a, t, b) >= 0.f); }
@@ -483,73 +625,143 @@ __device__ __forceinline__ bool funcertain(float a, float b, float t, float pa, 
     return (fabsf(__fmaf_rn(-b, t, a)) <= pa + t * pb) || (fabsf(__fmaf_rn(-a, t, b)) <= pb + t * pa);
 }
 
-// Exact resolution of the guard-band decisions of one kx group inside the
-// exact walk, one pair at a time, all lanes cooperating.
-__device__ __forceinline__ unsigned resolve_uncertain(const T3Params &P, int m, int tileX, int tileY, int g,
-                                                      int kxa, int lane, unsigned keep, unsigned unc)
+__device__ __forceinline__ float sqrt_approx(float x)
 {
-    unsigned any = __ballot_sync(0xffffffffu, unc != 0);
-    while (any) {
-        const int src = __ffs(any) - 1;
-        const unsigned su = __shfl_sync(0xffffffffu, unc, src);
-        const int kz = __ffs(su) - 1;
-        const int kyb = kappa(src);
-        df mb, mr;
-        exact_pair(P, m, tileX, tileY, kz, kyb, kxa, mb, mr);
-        const int kzr = (10 - kz) & 7, kybr = (40 - kyb) & 31;
-        bool sim = df_sim(mb, mr, thr_of(P, m, kz, kyb, kxa).d);
-        if (kxa == 4) sim |= df_sim(mb, mr, thr_of(P, m, kzr, kybr, 4).d);
-        if (lane == src) {
-            keep = sim ? (keep | (1u << kz)) : (keep & ~(1u << kz));
-            unc &= ~(1u << kz);
-        }
-        if (g == 2 && lane == kappa(kybr)) {   // kx = 4: the pair's other bin is a visitor too
-            keep = sim ? (keep | (1u << kzr)) : (keep & ~(1u << kzr));
-            unc &= ~(1u << kzr);
-        }
-        any = __ballot_sync(0xffffffffu, unc != 0);
-    }
-    return keep;
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// Output stage of step m: inverse Y then X of output fields 2m (RA) and
-// 2m + 1 (RB), and the store of each lane's row into its overlap class.
-__device__ __forceinline__ void walk_store(const T3Params &P, const LaneConst &LC, const float2 *RA, const float2 *RB,
-                                           int m, int tileX, int tileY, int cls)
+// The error bounds of one step. Lane k of 0..4 holds, for kx = k+2,
+//   ek = sum_z w_z (A_z[kx] + R_z / 2), the part of the per-bin estimate
+//        E = K 2^-24 (ek + sum_z w_z |S_z|_1) every ky shares, and
+//   em = an upper bound of E over every ky of columns kx and 8 - kx:
+//        |S_z|_1 <= sqrt(2) |S_z| <= sqrt(2) A_z.
+struct StepBounds {
+    float ek, em;
+};
+
+__device__ __forceinline__ StepBounds step_bounds(const float2 *bnd, int m, int lane)
 {
-    // Inverse Y then X, one kx at a time: lane (j, i) folds ky = kk and
-    // kk+16 of output field 2m+j for its row parity, runs a 16-point
-    // inverse DFT over the half-warp, and accumulates row i's cosine and
-    // sine sums of the inverse X transform.
+    const int kk = lane & 7, q = lane >> 3;
+    const float2 b = bnd[8 * ((m + q) & 3) + kk];
+    float v = __fmaf_rn(c3_wz[2 * q], b.x, c3_wz[2 * q + 1] * b.y);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    const float r = __shfl_sync(0xffffffffu, v, 5);
+    StepBounds o;
+    o.ek = __fmaf_rn(0.5f, r, v);
+    const float es = kBoundFactor * kEps32 * 1.001f * __fmaf_rn(2.41422f, v, 0.5f * r);
+    o.em = fmaxf(es, __shfl_sync(0xffffffffu, es, (4 - kk) & 7));
+    return o;
+}
+
+// A column with everything its guard band needs, recomputed from the window
+// (the same magnitudes the walk decided on).
+struct Col {
+    float2 Y[8];
+    float mag[8], E;
+};
+
+__device__ __forceinline__ void z_column(const float4 *win, int m, int k, int pos, const float2 (&wz)[4], float ek,
+                                         Col &c)
+{
+    float B = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const cp2 v = cp_of(win[(5 * ((m + q) & 3) + k) * 16 + pos]);
+        B = __fmaf_rn(fabsf(wz[q].x), fabsf(v.re.x) + fabsf(v.im.x), B);
+        B = __fmaf_rn(fabsf(wz[q].y), fabsf(v.re.y) + fabsf(v.im.y), B);
+    }
+    z_dft(win, m, k, pos, wz, c.Y);
+#pragma unroll
+    for (int kz = 0; kz < 8; kz++) c.mag[kz] = mag2(c.Y[kz]);
+    c.E = kBoundFactor * kEps32 * (ek + B);
+}
+
+// The guard band of one kx group of a step, bin by bin, and its record for
+// tp3_resolve_kernel. `last` is the warp's latest record of this item (the
+// records of one item form a list in the order of (m, g)).
+template <bool PER_BIN>
+__device__ __forceinline__ void record_group(const T3Params &P, const LaneConst &LC, const float4 *win,
+                                             const float *thr, int item, int m, int g, int lane, float tf_m, float ekA,
+                                             float ekB, int &last)
+{
+    // all 32 ky, one per lane, each with its mirror
+    const int ky = kappa(lane), kyr = (40 - ky) & 31, laneB = kappa(kyr);
+    float2 wz[4];
+    Col A, B;
+    z_window(wz, lane >= 16);
+    z_column(win, m, g, LC.posA, wz, ekA, A);
+    z_window(wz, laneB >= 16);
+    z_column(win, m, 4 - g, LC.posB, wz, ekB, B);
+    unsigned keep = 0, unc = 0;
+    // A pair too small to matter is left to FP32: toggling bins of
+    // magnitudes |Y_b|, |Y_r| moves any output sample by at most
+    // (2/4096)(|Y_b| + |Y_r|) <= (4/4096) sqrt(a + b + E^2 + rE^2)
+    // (true magnitudes within E of the computed ones), so under
+    // kTinyPair the change is below 1/4 of a composite sample unit
+    // (0.38 LSB of yuv444p16, 7e-6 of yuv444ps).
+    const float tiny_lim = kTinyPair - __fmaf_rn(A.E, A.E, B.E * B.E);
+#pragma unroll
+    for (int kz = 0; kz < 8; kz++) {
+        const int kzr = (10 - kz) & 7;
+        const float a = A.mag[kz], b = B.mag[kzr];
+        const float pa = 2.f * A.E * l1(A.Y[kz]) + A.E * A.E;
+        const float pb = 2.f * B.E * l1(B.Y[kzr]) + B.E * B.E;
+        float t = tf_m;
+        if (PER_BIN) t = thr[(8 * g + kz) * 32 + lane];
+        bool sim = fsim(a, b, t);
+        bool u = funcertain(a, b, t, pa, pb);
+        if (PER_BIN && g == 2) {   // kx = 4: the mirror bin visits too, with its own threshold
+            const float t2 = thr[(16 + kzr) * 32 + laneB];
+            sim |= fsim(a, b, t2);
+            u |= funcertain(a, b, t2, pa, pb);
+        }
+        // a carrier (its own mirror) is always kept
+        const bool self = (g == 2) && (kz == kzr) && (ky == kyr);
+        if (sim || self) keep |= 1u << kz;
+        if (u && !self && !(a + b < tiny_lim)) unc |= 1u << kz;
+    }
+    // (a flat or black tile, whose bound is zero, never has any)
+    if (!__any_sync(0xffffffffu, unc != 0)) return;
+    unsigned slot = 0;
+    if (lane == 0) slot = atomicAdd(P.counters, 1u);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (slot >= P.unc_cap) return;   // sized for every kx group of the launch
+    UncRecord &rec = P.unc_rec[slot];
+    if (lane == 0) {
+        rec.item = item;
+        rec.mg = m * 4 + g;
+        rec.prev = last;
+        rec.next = -1;
+        if (last >= 0) P.unc_rec[last].next = (int)slot;
+    }
+    rec.unc[lane] = (uint8_t)unc;
+    rec.keep[lane] = (uint8_t)keep;
+    last = (int)slot;
+}
+
+// Inverse X stage of step m's output rows, and the store of each lane's row
+// into its overlap class.
+__device__ __forceinline__ void x_inverse_store(const T3Params &P, const LaneConst &LC, const float4 *rows, int m,
+                                                int tileX, int cls)
+{
     float2 CS[8];   // (cosine sum, sine sum) of row i
 #pragma unroll
     for (int x = 0; x < 8; x++) CS[x] = make_float2(0.f, 0.f);
-    const float2 *Rj = LC.j ? RB : RA;
+    const float *yr = reinterpret_cast<const float *>(rows) + 4 * LC.i + LC.j;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        const float2 lo_v = Rj[k * 32 + LC.i];        // R[kk]   (lane kappa^-1(kk) = i)
-        const float2 hi_v = Rj[k * 32 + LC.i + 16];   // R[kk+16]
-        float2 G = LC.y0 ? sub2(lo_v, hi_v) : add2(lo_v, hi_v);
-        G = cmul(G, make_float2(LC.ptw.x, -LC.ptw.y));   // exp(+i pi kk y0 / 16)
-        // 16-point inverse DFT, bit-reversed input -> natural order (DIT)
-        int st = 3;
-#pragma unroll
-        for (int h = 1; h <= 8; h <<= 1, st--) {
-            const bool upper = (LC.i & h) != 0;
-            const float2 w = make_float2(LC.ftw[st].x, -LC.ftw[st].y);   // exp(+2 pi i r/(2h))
-            const float2 o = shfl_xor2(G, h);
-            const float2 t = cmul(upper ? G : o, w);
-            G = upper ? sub2(o, t) : add2(G, t);
-        }
+        const float2 G = make_float2(yr[80 * k], yr[80 * k + 2]);
 #pragma unroll
         for (int x = 0; x < 8; x++) CS[x] = __ffma2_rn(G, c3_xi[k][x], CS[x]);
     }
     // Store row i of field 2m + j.
-    const int L = tileY + LC.y0 + 2 * LC.i;
-    if (L >= P.fafl && L <= P.lafl) {
+    if (LC.row_ok) {
         const int ofield = 2 * (m - P.frame_begin) + LC.j;
         float *dst = P.partial + (long long)cls * P.part_class_stride + (long long)ofield * P.part_field_stride +
-                     (long long)((L >> 1) - P.fl_lo) * P.part_row_stride - P.avs;
+                     (long long)((LC.rowL >> 1) - P.fl_lo) * P.part_row_stride - P.avs;
         // tileX - avs is a multiple of 8, so an interior tile's row starts
         // on a 32-byte boundary whenever the planes' strides are multiples
         // of 4 floats and their base is 16-byte aligned: four vector stores
@@ -577,13 +789,23 @@ __device__ __forceinline__ void walk_store(const T3Params &P, const LaneConst &L
     }
 }
 
+// The record of (step m, kx group g) in the list of `rec`'s item, or -1.
+__device__ __forceinline__ int find_record(const T3Params &P, int rec, int mg)
+{
+    int at = rec;
+    while (at >= 0 && P.unc_rec[at].mg > mg) at = P.unc_rec[at].prev;
+    while (at >= 0 && P.unc_rec[at].mg < mg) at = P.unc_rec[at].next;
+    return at >= 0 && P.unc_rec[at].mg == mg ? at : -1;
+}
+
 // TMODE: 0 = one uniform threshold, 1 = per-bin table, 2 = per-frame
 // thresholds (batches of captures). EXACT = false: the walk over every work
 // item, guard-band decisions taken in FP32 and recorded for
 // tp3_resolve_kernel (an exact path inside this loop, however rarely taken,
-// slows the whole walk by a third). EXACT = true: the walk again over the
-// items tp3_resolve_kernel listed, deciding those bins exactly; it writes
-// the same output locations, so its result replaces the FP32 one.
+// slows the whole walk by a third). EXACT = true: the outputs that
+// tp3_resolve_kernel's corrections reach, walked again with the decisions of
+// the corrected records; it writes the same output locations, so its result
+// replaces the FP32 one.
 template <int TMODE, bool EXACT>
 __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
 {
@@ -591,11 +813,26 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int ntiles = P.ntx * P.nty;
+    extern __shared__ float4 s_dyn[];
+    float4 *win = s_dyn + (size_t)warp * kWarpF4;
+    float4 *carry_base = win + kWinF4;
+    float4 *exch = carry_base + kCarryF4;
+    float4 *R = exch + kExchF4;
+    float2 *bnd = reinterpret_cast<float2 *>(R + kOutF4);
+    float4 *tw = s_dyn + kWarps3 * kWarpF4;
+    float *thr = reinterpret_cast<float *>(tw + kTwF4);   // [g][kz][lane], per-bin walks only
+    if (PER_BIN)
+        for (int i = threadIdx.x; i < 3 * 8 * 32; i += blockDim.x)
+            thr[i] = P.thr_table[3 * ((((i >> 5) & 7) * 32 + kappa(i & 31)) * 3 + (i >> 8))];
+    fill_twiddles(P, tw);
     // Work items (tile position, chunk of frames); a grid smaller than the
-    // item count walks them persistently.
-    const unsigned nitems = EXACT ? min(P.counters[1], P.unc_cap) : (unsigned)(ntiles * P.nchunks);
+    // item count walks them persistently. EXACT: two items per corrected
+    // record, the output of its own step mf and the one its carries feed
+    // (step mf + 2).
+    const unsigned nitems = EXACT ? 2 * min(P.counters[1], P.unc_cap) : (unsigned)(ntiles * P.nchunks);
     for (unsigned w = blockIdx.x * kWarps3 + warp; w < nitems; w += gridDim.x * kWarps3) {
-    const int item = EXACT ? (int)P.rerun[2 * w] : (int)w;
+    const int rec = EXACT ? (int)P.rerun[w >> 1] : -1;
+    const int item = EXACT ? P.unc_rec[rec].item : (int)w;
     const int tile = item % ntiles;
     const int chunk = item / ntiles;
     const int tx = tile % P.ntx, ty = tile / P.ntx;
@@ -604,146 +841,144 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
     int m0 = P.frame_begin + chunk * P.chunk_frames;
     int m1 = min(m0 + P.chunk_frames, P.frame_end);
     if (EXACT) {
-        // only the steps a wrong decision at step mf reached: its own output
-        // (fields 2mf, 2mf+1) and the one its carries feed (step mf + 2)
-        const int mf = (int)P.rerun[2 * w + 1];
-        m0 = max(m0, mf);
-        m1 = min(m1, mf + 3);
+        const int mo = (P.unc_rec[rec].mg >> 2) + 2 * (int)(w & 1);
+        if (mo < m0 || mo >= m1) continue;
+        m0 = mo;
+        m1 = mo + 1;
     }
     const int cls = ((ty & 1) << 1) | (tx & 1);
-
-    // Per-warp shared state (dynamic): window of field spectra, Z carries,
-    // Z-stage output spectra and per-field bound terms.
-    extern __shared__ float4 s_dyn[];
-    float2 *wbase = reinterpret_cast<float2 *>(s_dyn) + (size_t)warp * kWarpSmemF2;
-    float2 *win = wbase;                          // [8 slots][5 kx][32 lanes]
-    float2 *carry_base = wbase + 8 * 5 * 32;      // [2][2 slices][5 kx][32 lanes]
-    float *bnd = reinterpret_cast<float *>(carry_base + 2 * 2 * 5 * 32);   // [8 slots][8]
-
-    const LaneConst LC = lane_const(lane, tileY, P.swap);
-    const int my_ky = kappa(lane);
-    const int kyr = (40 - my_ky) & 31;
-    const int mirror_lane = kappa(kyr);
+    const LaneConst LC = lane_const(P, lane, tileX, tileY);
+    int last = -1;   // the item's latest record
+    RowWords row;
+    load_row(P, m0 - 2, LC, row);
 
     // Steps m0-5 .. m0-3 only fill the window (fields 2(m0-2) .. 2(m0-2)+5);
-    // steps m0-2 and m0-1 also run the Z stage for the carries; the rest output.
-    for (int m = m0 - 5; m < m1; m++) {
+    // steps m0-2 and m0-1 also run the Z stage for the carries; the rest
+    // output, each with the next step's forward stages (step m1: only that).
+    for (int m = m0 - 5; m <= m1; m++) {
         __syncwarp();
-        forward_pair(P, m + 3, tileX, tileY, LC, lane, win, bnd);   // fields 2m+6, 2m+7
+        if (m < m1) x_forward(row, m + 3, LC, exch, bnd);   // fields 2m+6, 2m+7
+        if (m + 1 < m1) load_row(P, m + 4, LC, row);        // the next step's, in flight until then
         __syncwarp();
-        if (m < m0 - 2) continue;
+        if (lane < 20) y_stages<true>(m + 3, LC, lane, win, exch, R, bnd, tw);
+        __syncwarp();
+        if (m > m0) x_inverse_store(P, LC, R + kRowsAt, m - 1, tileX, cls);
+        if (m < m0 - 2 || (EXACT && m == m0 - 1) || m == m1) continue;
+        __syncwarp();   // the output rows have been read: R may be written
 
-        // Per-kx error-bound base (warp-uniform): sum_z w_z (A_z[kx] + R_z / 2)
-        float ek[5];
-#pragma unroll
-        for (int k = 0; k < 5; k++) ek[k] = 0.f;
-#pragma unroll
-        for (int z = 0; z < 8; z++) {
-            const float *b = bnd + 8 * ((2 * m + z) & 7);
-            const float half_r = 0.5f * b[5];
-#pragma unroll
-            for (int k = 0; k < 5; k++) ek[k] = __fmaf_rn(c3_wz[z], b[k] + half_r, ek[k]);
-        }
-        float2 *carry = carry_base + (m & 1) * (2 * 5 * 32);
+        const StepBounds SB = EXACT ? StepBounds{0.f, 0.f} : step_bounds(bnd, m, lane);
+        float4 *carry = carry_base + (m & 1) * (5 * 32);
         const float tf_m = (TMODE == 2) ? P.frame_t2[3 * max(m, 0)] : P.t2f;   // uniform threshold of frame m
 
-        // Z stage per kx pair: column A = kx 2+g (visited by the filter),
-        // column B = its mirror kx 6-g (g = 2: kx 4 mirrors onto itself).
-        // Z-stage outputs for fields 2m, 2m+1 go into those fields' window
-        // slots: each column is written after it has been read.
-        float2 *RA = win + ((2 * m) & 7) * 5 * 32;
-        float2 *RB = win + ((2 * m + 1) & 7) * 5 * 32;
-#pragma unroll 1
-        for (int g = 0; g < 3; g++) {
-            const int ka = g, kb = 4 - g;
-            const int kxa = 2 + g;
-            float rmag[8], rab[8], rE;
-            Col B;
-            if (g < 2) {
-                z_column(win, m, kb, lane, g == 0 ? ek[4] : ek[3], B);
-#pragma unroll
-                for (int kz = 0; kz < 8; kz++) {
-                    rmag[kz] = __shfl_sync(0xffffffffu, B.mag[kz], mirror_lane);
-                    rab[kz] = __shfl_sync(0xffffffffu, B.ab[kz], mirror_lane);
-                }
-                rE = __shfl_sync(0xffffffffu, B.E, mirror_lane);
+        // One decision: bin magnitude a against its mirror's b. Beside it a
+        // screen for the guard band, an upper bound of the bin's band: with
+        // ab <= sqrt(2 a), a band pa + t pb is at most
+        // 2 sqrt(2) E (sqrt a + t sqrt b) + (1 + t) E^2
+        // <= (1 + t) (2 sqrt(2) E sqrt(a + b) + E^2). The nearer margin is
+        // the one of the smaller magnitude against t times the larger (for
+        // t > 1 both tests fail unless both magnitudes are zero). A pair under
+        // the limit of tiny pairs cannot be recorded. Only groups that pass
+        // the screen run the bin-by-bin test (record_group).
+        float e1, e2, lim;
+        bool u;
+        auto bounds = [&](float Em) {
+            const float t1 = PER_BIN ? 1.f : 1.f + tf_m;
+            e1 = 2.83f * t1 * Em;
+            e2 = 1.01f * t1 * Em * Em;
+            lim = kTinyPair - 2.01f * Em * Em;
+            u = false;
+        };
+        auto similar = [&](float a, float b, float t) -> bool {
+            const float d = __fmaf_rn(-fmaxf(a, b), t, fminf(a, b));
+            if (!EXACT) {
+                const float s = a + b;
+                const float band = __fmaf_rn(e1, sqrt_approx(s), e2);
+                u |= (s >= lim) && (fabsf(d) <= (PER_BIN ? (1.f + t) * band : band));
             }
-            Col A;
-            z_column(win, m, ka, lane, g == 0 ? ek[0] : (g == 1 ? ek[1] : ek[2]), A);
-            if (g == 2) {
+            return d >= 0.f;
+        };
+        int fix[3] = {-1, -1, -1};
+        if (EXACT)
+            for (int g = 0; g < 3; g++) fix[g] = find_record(P, rec, m * 4 + g);
+
+        // Pass 1: the pairs (kx 2, kx 6) in half-warp 0, (kx 3, kx 5) in half-warp 1
+        {
+            const int h = lane >> 4;
+            float2 YA[8], YB[8], wz[4];
+            z_window(wz, false);
+            z_dft(win, m, h, LC.posA, wz, YA);
+            z_dft(win, m, 4 - h, LC.posB, LC.wzB, YB);
+            bounds(EXACT ? 0.f : __shfl_sync(0xffffffffu, SB.em, h));
+            float k[8], kh[8], kr[8], khr[8];   // at ky, at ky + 16; the same for the mirror column
+            float ma[8], mb[8];
 #pragma unroll
-                for (int kz = 0; kz < 8; kz++) {
-                    rmag[kz] = __shfl_sync(0xffffffffu, A.mag[kz], mirror_lane);
-                    rab[kz] = __shfl_sync(0xffffffffu, A.ab[kz], mirror_lane);
-                }
-                rE = __shfl_sync(0xffffffffu, A.E, mirror_lane);
+            for (int kz = 0; kz < 8; kz++) {
+                ma[kz] = mag2(YA[kz]);
+                mb[kz] = mag2(YB[kz]);
             }
-            // The mirror of my column-A bin kz is bin kzr of the mirror lane's
-            // column B (its column A when g = 2).
-            unsigned keep = 0, unc = 0;
-            // A pair too small to matter is left to FP32: toggling bins of
-            // magnitudes |Y_b|, |Y_r| moves any output sample by at most
-            // (2/4096)(|Y_b| + |Y_r|) <= (4/4096) sqrt(a + b + E^2 + rE^2)
-            // (true magnitudes within E of the computed ones), so under
-            // kTinyPair the change is below 1/4 of a composite sample unit
-            // (0.38 LSB of yuv444p16, 7e-6 of yuv444ps).
-            const float tiny_lim = kTinyPair - __fmaf_rn(A.E, A.E, rE * rE);
+            unsigned fl = 0, fh = 0;
+            if (EXACT && fix[h] >= 0) {
+                fl = P.unc_rec[fix[h]].keep[lane & 15];
+                fh = P.unc_rec[fix[h]].keep[16 + (lane & 15)];
+            }
 #pragma unroll
             for (int kz = 0; kz < 8; kz++) {
                 const int kzr = (10 - kz) & 7;
-                const float a = A.mag[kz], b = rmag[kzr];
-                const float pa = 2.f * A.E * A.ab[kz] + A.E * A.E;
-                const float pb = 2.f * rE * rab[kzr] + rE * rE;
-                float t = tf_m;
-                if (PER_BIN) t = thr_of(P, m, kz, my_ky, kxa).f;
-                bool sim = fsim(a, b, t);
-                bool u = funcertain(a, b, t, pa, pb);
-                if (PER_BIN && g == 2) {   // kx = 4: the mirror bin visits too, with its own threshold
-                    const float t2 = thr_of(P, m, kzr, kyr, 4).f;
-                    sim |= fsim(a, b, t2);
-                    u |= funcertain(a, b, t2, pa, pb);
-                }
-                // a carrier (its own mirror) is always kept
-                const bool self = (g == 2) && (kz == kzr) && (my_ky == kyr);
-                if (sim || self) keep |= 1u << kz;
-                if (u && !self && !(a + b < tiny_lim)) unc |= 1u << kz;
-            }
-            // Record decisions inside the guard band for the exact passes
-            // (a flat or black tile, whose bound is zero, never has any).
-            if (__any_sync(0xffffffffu, unc != 0)) {
-                if (EXACT) {
-                    keep = resolve_uncertain(P, m, tileX, tileY, g, kxa, lane, keep, unc);
-                } else {
-                    unsigned slot = 0;
-                    if (lane == 0) slot = atomicAdd(P.counters, 1u);
-                    slot = __shfl_sync(0xffffffffu, slot, 0);
-                    if (slot < P.unc_cap) {   // sized for every kx group of the launch
-                        UncRecord &rec = P.unc_rec[slot];
-                        if (lane == 0) {
-                            rec.item = item;
-                            rec.tile = tile;
-                            rec.m = m;
-                            rec.g = g;
-                        }
-                        rec.unc[lane] = (uint8_t)unc;
-                        rec.keep[lane] = (uint8_t)keep;
-                    }
+                bool sim = similar(ma[kz], mb[kzr], PER_BIN ? thr[(8 * h + kz) * 32 + (lane & 15)] : tf_m);
+                if (EXACT && fix[h] >= 0) sim = (fl >> kz) & 1u;
+                k[kz] = sim ? 1.f : 0.f;
+                if (PER_BIN) {
+                    bool simh = similar(ma[kz ^ 4], mb[kzr ^ 4], thr[(8 * h + kz) * 32 + 16 + (lane & 15)]);
+                    if (EXACT && fix[h] >= 0) simh = (fh >> kz) & 1u;
+                    kh[kz] = simh ? 1.f : 0.f;
                 }
             }
-            z_inverse(A.Y, keep, carry, RA, RB, ka, lane);
-            if (g < 2) {
-                // Column B bins are kept exactly when their mirror visit kept them.
-                const unsigned mk = __shfl_sync(0xffffffffu, keep, mirror_lane);
-                unsigned keepB = 0;
 #pragma unroll
-                for (int kz = 0; kz < 8; kz++) keepB |= ((mk >> ((10 - kz) & 7)) & 1u) << kz;
-                z_inverse(B.Y, keepB, carry, RA, RB, kb, lane);
+            for (int kz = 0; kz < 8; kz++) {
+                kr[kz] = k[(10 - kz) & 7];
+                khr[kz] = PER_BIN ? kh[(10 - kz) & 7] : 0.f;
+            }
+            z_inverse<!PER_BIN>(YA, k, kh, carry, R, h, lane & 15);
+            z_inverse<!PER_BIN>(YB, kr, khr, carry, R, 4 - h, LC.laneB);
+            if (!EXACT) {
+                const unsigned hit = __ballot_sync(0xffffffffu, u);
+                for (int g = 0; g < 2; g++)
+                    if (hit & (0xFFFFu << (16 * g))) {
+                        const float ekA = __shfl_sync(0xffffffffu, SB.ek, g), ekB = __shfl_sync(0xffffffffu, SB.ek, 4 - g);
+                        record_group<PER_BIN>(P, LC, win, thr, item, m, g, lane, tf_m, ekA, ekB, last);
+                    }
             }
         }
-        __syncwarp();
-        if (m < m0) continue;   // warm-up step: only the carries are needed
-
-        walk_store(P, LC, RA, RB, m, tileX, tileY, cls);
+        // Pass 2: kx 4, whose mirror bins' magnitudes come from the lanes
+        // that own them; all 32 ky.
+        {
+            const int laneB = LC.laneB ^ (lane & 16);
+            float2 Y[8], wz[4];
+            z_window(wz, lane >= 16);
+            z_dft(win, m, 2, LC.posA, wz, Y);
+            bounds(EXACT ? 0.f : __shfl_sync(0xffffffffu, SB.em, 2));
+            const unsigned f = EXACT && fix[2] >= 0 ? P.unc_rec[fix[2]].keep[lane] : 0u;
+            float2 y[8], o[4];
+#pragma unroll
+            for (int kz = 0; kz < 8; kz++) {
+                const int kzr = (10 - kz) & 7;
+                const float a = mag2(Y[kz]), b = __shfl_sync(0xffffffffu, mag2(Y[kzr]), laneB);
+                bool sim = similar(a, b, PER_BIN ? thr[(16 + kz) * 32 + lane] : tf_m);
+                if (PER_BIN) sim |= similar(a, b, thr[(16 + kzr) * 32 + laneB]);   // the mirror bin visits too
+                if (kz == kzr) sim |= laneB == lane;   // a carrier (its own mirror) is always kept
+                if (EXACT && fix[2] >= 0) sim = (f >> kz) & 1u;
+                const float k = sim ? 1.f : 0.f;
+                y[kz] = __fmul2_rn(Y[kz], make_float2(k, k));
+            }
+            z_rotate(y, o);
+            ZInverse Z;
+            Z.sum(y, o);
+            Z.finish(carry, R, 2, lane);
+            if (!EXACT && __any_sync(0xffffffffu, u)) {
+                const float ek = __shfl_sync(0xffffffffu, SB.ek, 2);
+                record_group<PER_BIN>(P, LC, win, thr, item, m, 2, lane, tf_m, ek, ek, last);
+            }
+        }
     }
     __syncwarp();   // the next item reuses this warp's shared window
     }
@@ -752,29 +987,6 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
 // ---------------------------------------------------------------------------
 // Learned-mask form: feature pass and apply pass
 // ---------------------------------------------------------------------------
-// FP32 threshold decisions of kx group g (the walk's rule without the exact
-// resolution): bits kz of column A kept; the caller derives column B's.
-__device__ __forceinline__ unsigned fp32_keep(const Col &A, const float (&rmag)[8], int g, int my_ky, int kyr, float t)
-{
-    unsigned keep = 0;
-#pragma unroll
-    for (int kz = 0; kz < 8; kz++) {
-        const int kzr = (10 - kz) & 7;
-        const bool self = (g == 2) && (kz == kzr) && (my_ky == kyr);
-        if (fsim(A.mag[kz], rmag[kzr], t) || self) keep |= 1u << kz;
-    }
-    return keep;
-}
-
-__device__ __forceinline__ unsigned mirror_keep(unsigned keep, int mirror_lane)
-{
-    const unsigned mk = __shfl_sync(0xffffffffu, keep, mirror_lane);
-    unsigned keepB = 0;
-#pragma unroll
-    for (int kz = 0; kz < 8; kz++) keepB |= ((mk >> ((10 - kz) & 7)) & 1u) << kz;
-    return keepB;
-}
-
 __device__ __forceinline__ uint16_t bf16_bits(float x)
 {
     const __nv_bfloat16 h = __float2bfloat16_rn(x);
@@ -791,6 +1003,14 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_learned_kernel(T3Param
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int ntiles = P.ntx * P.nty;
+    extern __shared__ float4 s_dyn[];
+    float4 *win = s_dyn + (size_t)warp * kWarpF4;
+    float4 *carry_base = win + kWinF4;
+    float4 *exch = carry_base + kCarryF4;
+    float4 *R = exch + kExchF4;
+    float2 *bnd = reinterpret_cast<float2 *>(R + kOutF4);
+    float4 *tw = s_dyn + kWarps3 * kWarpF4;
+    fill_twiddles(P, tw);
     const unsigned nitems = (unsigned)(ntiles * P.nchunks);
     for (unsigned w = blockIdx.x * kWarps3 + warp; w < nitems; w += gridDim.x * kWarps3) {
     const int item = (int)w;
@@ -802,89 +1022,107 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_learned_kernel(T3Param
     const int m0 = P.frame_begin + chunk * P.chunk_frames;
     const int m1 = min(m0 + P.chunk_frames, P.frame_end);
     const int cls = ((ty & 1) << 1) | (tx & 1);
+    const LaneConst LC = lane_const(P, lane, tileX, tileY);
 
-    extern __shared__ float4 s_dyn[];
-    float2 *wbase = reinterpret_cast<float2 *>(s_dyn) + (size_t)warp * kWarpSmemF2;
-    float2 *win = wbase;
-    float2 *carry_base = wbase + 8 * 5 * 32;
-    float *bnd = reinterpret_cast<float *>(carry_base + 2 * 2 * 5 * 32);
-
-    const LaneConst LC = lane_const(lane, tileY, P.swap);
-    const int my_ky = kappa(lane);
-    const int kyr = (40 - my_ky) & 31;
-    const int mirror_lane = kappa(kyr);
-
-    for (int m = m0 - 5; m < m1; m++) {
+    RowWords row;
+    load_row(P, m0 - 2, LC, row);
+    for (int m = m0 - 5; m <= m1; m++) {
         __syncwarp();
-        forward_pair(P, m + 3, tileX, tileY, LC, lane, win, bnd);
+        if (m < m1) x_forward(row, m + 3, LC, exch, bnd);
+        if (m + 1 < m1) load_row(P, m + 4, LC, row);
         __syncwarp();
-        if (m < m0 - 2) continue;
+        if (lane < 20) y_stages<PASS == 1>(m + 3, LC, lane, win, exch, R, bnd, tw);
+        __syncwarp();
+        if (PASS == 1 && m > m0) x_inverse_store(P, LC, R + kRowsAt, m - 1, tileX, cls);
+        if (m < m0 - 2 || m == m1) continue;
+        __syncwarp();
         const long long base = ((long long)(m - L.z0) * ntiles + tile) * 1280;
-        float2 *carry = carry_base + (m & 1) * (2 * 5 * 32);
-        float2 *RA = win + ((2 * m) & 7) * 5 * 32;
-        float2 *RB = win + ((2 * m + 1) & 7) * 5 * 32;
+        float4 *carry = carry_base + (m & 1) * (5 * 32);
         const bool fb = (PASS == 1) ? (L.fallback[(long long)(m - L.z0) * ntiles + tile] != 0) : false;
+        // the walk's two passes: the column pairs of both half-warps, then
+        // kx 4 (both half-warps at ky < 16; half-warp 0 writes)
 #pragma unroll 1
-        for (int g = 0; g < 3; g++) {
-            const int ka = g, kb = 4 - g;
-            float rmag[8];
-            Col B;
-            if (g < 2) {
-                z_column(win, m, kb, lane, 0.f, B);
+        for (int pass = 0; pass < 2; pass++) {
+            const int h = lane >> 4;
+            const int ka = pass == 0 ? h : 2, kb = 4 - ka;
+            float2 YA[8], YB[8], wz[4];
+            z_window(wz, false);
+            z_dft(win, m, ka, LC.posA, wz, YA);
+            z_dft(win, m, kb, LC.posB, LC.wzB, YB);
+            const int kyr = (40 - LC.ky) & 31;
+            const long long va = base + ka * 256 + LC.ky, vb = base + kb * 256 + kyr;
+            const int hb = kyr < 16 ? 16 : -16;   // from the mirror ky to its other half
+            const bool wa = pass == 0 || h == 0, wb = pass == 0;   // column A, column B written
+            unsigned keep = 0;   // FP32 decisions: bit kz = column A's bin kz and column B's (10 - kz) & 7
+            if (PASS == 0 ? L.plain_p != nullptr : fb) {
 #pragma unroll
-                for (int kz = 0; kz < 8; kz++) rmag[kz] = __shfl_sync(0xffffffffu, B.mag[kz], mirror_lane);
-            }
-            Col A;
-            z_column(win, m, ka, lane, 0.f, A);
-            if (g == 2) {
-#pragma unroll
-                for (int kz = 0; kz < 8; kz++) rmag[kz] = __shfl_sync(0xffffffffu, A.mag[kz], mirror_lane);
+                for (int kz = 0; kz < 8; kz++) {
+                    const int kzr = (10 - kz) & 7;
+                    const bool self = pass == 1 && kz == kzr && LC.ky == kyr;
+                    if (fsim(mag2(YA[kz]), mag2(YB[kzr]), P.t2f) || self) keep |= 1u << kz;
+                }
             }
             if (PASS == 0) {
 #pragma unroll
                 for (int kz = 0; kz < 8; kz++) {
-                    const long long va = base + (ka * 8 + kz) * 32 + my_ky;
-                    L.feat[va] = bf16_bits(log1pf(sqrtf(A.mag[kz])) * 0.0625f);
-                    if (L.spec != nullptr) L.spec[va] = A.Y[kz];
-                    if (g < 2) {
-                        const long long vb = base + (kb * 8 + kz) * 32 + my_ky;
-                        L.feat[vb] = bf16_bits(log1pf(sqrtf(B.mag[kz])) * 0.0625f);
-                        if (L.spec != nullptr) L.spec[vb] = B.Y[kz];
+                    const int v = 32 * kz, vm = 32 * (kz ^ 4);
+                    if (wa) {
+                        const uint16_t f = bf16_bits(log1pf(sqrtf(mag2(YA[kz]))) * 0.0625f);
+                        L.feat[va + v] = f;
+                        L.feat[va + vm + 16] = f;
+                    }
+                    if (wb) {
+                        const uint16_t f = bf16_bits(log1pf(sqrtf(mag2(YB[kz]))) * 0.0625f);
+                        L.feat[vb + v] = f;
+                        L.feat[vb + vm + hb] = f;
+                    }
+                }
+                if (L.spec != nullptr) {
+                    const float s = ((P.swap ^ P.tileY0) & 1) ? -1.f : 1.f;   // the sign of ky >= 16
+                    const float sb = kyr < 16 ? 1.f : s, sm = kyr < 16 ? s : 1.f;
+#pragma unroll
+                    for (int kz = 0; kz < 8; kz++) {
+                        const int v = 32 * kz, vm = 32 * (kz ^ 4);
+                        if (wa) {
+                            L.spec[va + v] = YA[kz];
+                            L.spec[va + vm + 16] = make_float2(s * YA[kz].x, s * YA[kz].y);
+                        }
+                        if (wb) {
+                            L.spec[vb + v] = make_float2(sb * YB[kz].x, sb * YB[kz].y);
+                            L.spec[vb + vm + hb] = make_float2(sm * YB[kz].x, sm * YB[kz].y);
+                        }
                     }
                 }
                 if (L.plain_p != nullptr) {
-                    const unsigned keep = fp32_keep(A, rmag, g, my_ky, kyr, P.t2f);
-                    const unsigned keepB = mirror_keep(keep, mirror_lane);
 #pragma unroll
                     for (int kz = 0; kz < 8; kz++) {
-                        L.plain_p[base + (ka * 8 + kz) * 32 + my_ky] = (float)((keep >> kz) & 1u);
-                        if (g < 2) L.plain_p[base + (kb * 8 + kz) * 32 + my_ky] = (float)((keepB >> kz) & 1u);
+                        const int kzr = (10 - kz) & 7;
+                        const float p = (float)((keep >> kz) & 1u);
+                        if (wa) L.plain_p[va + 32 * kz] = L.plain_p[va + 32 * (kz ^ 4) + 16] = p;
+                        if (wb) L.plain_p[vb + 32 * kzr] = L.plain_p[vb + 32 * (kzr ^ 4) + hb] = p;
                     }
                 }
             } else {
-                if (fb) {
-                    const unsigned keep = fp32_keep(A, rmag, g, my_ky, kyr, P.t2f);
-                    const unsigned keepB = mirror_keep(keep, mirror_lane);
-                    z_inverse(A.Y, keep, carry, RA, RB, ka, lane);
-                    if (g < 2) z_inverse(B.Y, keepB, carry, RA, RB, kb, lane);
-                } else {
+                float k[8], kh[8], kr[8], khr[8];
 #pragma unroll
-                    for (int kz = 0; kz < 8; kz++) {
-                        const float pa = __ldg(L.p + base + (ka * 8 + kz) * 32 + my_ky);
-                        A.Y[kz] = __fmul2_rn(A.Y[kz], make_float2(pa, pa));
-                        if (g < 2) {
-                            const float pb = __ldg(L.p + base + (kb * 8 + kz) * 32 + my_ky);
-                            B.Y[kz] = __fmul2_rn(B.Y[kz], make_float2(pb, pb));
-                        }
+                for (int kz = 0; kz < 8; kz++) {
+                    const int kzr = (10 - kz) & 7;
+                    if (fb) {
+                        k[kz] = (float)((keep >> kz) & 1u);
+                        kh[kz] = (float)((keep >> (kz ^ 4)) & 1u);
+                        kr[kz] = (float)((keep >> kzr) & 1u);
+                        khr[kz] = (float)((keep >> (kzr ^ 4)) & 1u);
+                    } else {
+                        k[kz] = __ldg(L.p + va + 32 * kz);
+                        kh[kz] = __ldg(L.p + va + 32 * kz + 16);
+                        kr[kz] = wb ? __ldg(L.p + vb + 32 * kz) : 0.f;
+                        khr[kz] = wb ? __ldg(L.p + vb + 32 * kz + hb) : 0.f;
                     }
-                    z_inverse(A.Y, 0xFFu, carry, RA, RB, ka, lane);
-                    if (g < 2) z_inverse(B.Y, 0xFFu, carry, RA, RB, kb, lane);
                 }
+                if (wa) z_inverse<false>(YA, k, kh, carry, R, ka, lane & 15);
+                if (wb) z_inverse<false>(YB, kr, khr, carry, R, kb, LC.laneB);
             }
         }
-        __syncwarp();
-        if (PASS == 0 || m < m0) continue;
-        walk_store(P, LC, RA, RB, m, tileX, tileY, cls);
     }
     __syncwarp();
     }
@@ -895,7 +1133,7 @@ int tp3_learned_launch(const T3Params &P, const T3Learn &L, int pass, cudaStream
     const long long items = (long long)P.ntx * P.nty * P.nchunks;
     if (items <= 0) return 0;
     const unsigned blocks = (unsigned)((items + kWarps3 - 1) / kWarps3);
-    const size_t smem = sizeof(float2) * (size_t)kWarpSmemF2 * kWarps3;
+    const size_t smem = walk_smem(false);
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -923,8 +1161,8 @@ int tp3_learned_launch(const T3Params &P, const T3Learn &L, int pass, cudaStream
 // One warp per record: decide its guard-band bins exactly in double-float
 // (the arithmetic of exact_pair, with the X stage of the record's two kx
 // columns computed once for all its bins) and, where an exact decision
-// differs from the FP32 one the walk used, list the record's work item and
-// step for the exact walk.
+// differs from the FP32 one the walk used, correct the record's decisions and
+// list it for the exact walk.
 __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -953,11 +1191,11 @@ __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
     __syncthreads();
     auto as_dfc = [](float4 v) -> dfc { return {{v.x, v.y}, {v.z, v.w}}; };
     for (unsigned rec = blockIdx.x * kWarps3 + warp; rec < n; rec += gridDim.x * kWarps3) {
-        const UncRecord &R = P.unc_rec[rec];
-        const int item = R.item, tile = R.tile, m = R.m, g = R.g;
+        UncRecord &R = P.unc_rec[rec];
+        const int tile = R.item % (P.ntx * P.nty), m = R.mg >> 2, g = R.mg & 3;
         const int tileX = P.tileX0 + 8 * (tile % P.ntx), tileY = P.tileY0 + 16 * (tile / P.ntx);
         const int kxa = 2 + g;
-        const unsigned keep = R.keep[lane];
+        unsigned keep = R.keep[lane];
         unsigned unc = R.unc[lane];
         // X stage of this lane's four rows of field 2m + z, both columns
         const int f = 2 * m + z;
@@ -1014,15 +1252,19 @@ __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
                 n_exact++;
                 if (old != sim) n_flip++;
                 unc &= ~(1u << kz);
+                keep = (keep & ~(1u << kz)) | ((unsigned)sim << kz);
             }
-            if (g == 2 && lane == kappa(kybr)) unc &= ~(1u << kzr);   // kx = 4: the same pair
+            if (g == 2 && lane == kappa(kybr)) {   // kx = 4: the same pair
+                unc &= ~(1u << kzr);
+                keep = (keep & ~(1u << kzr)) | ((unsigned)sim << kzr);
+            }
             any = __ballot_sync(0xffffffffu, unc != 0);
         }
-        if (flipped && lane == 0) {
-            const unsigned at = atomicAdd(P.counters + 1, 1u);
-            if (at < P.unc_cap) {   // at most one entry per record
-                P.rerun[2 * at] = (unsigned)item;
-                P.rerun[2 * at + 1] = (unsigned)m;
+        if (flipped) {   // the exact walk takes this group's decisions from the record
+            R.keep[lane] = (uint8_t)keep;
+            if (lane == 0) {
+                const unsigned at = atomicAdd(P.counters + 1, 1u);
+                if (at < P.unc_cap) P.rerun[at] = rec;   // at most one entry per record
             }
         }
     }
@@ -1115,14 +1357,14 @@ int tp3_launch(const T3Params &P, cudaStream_t stream, int max_blocks)
     if (items <= 0) return 0;
     unsigned blocks = (unsigned)((items + kWarps3 - 1) / kWarps3);
     if (max_blocks > 0 && blocks > (unsigned)max_blocks) blocks = (unsigned)max_blocks;   // persistent grid
-    const size_t smem = sizeof(float2) * (size_t)kWarpSmemF2 * kWarps3;
+    const size_t smem = walk_smem(P.thr_table != nullptr);
     // function attributes are per device
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return -1;
     if (!attr_set[dev]) {
-        const int b = (int)smem;
+        const int b = (int)walk_smem(true);
         const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
         if (cudaFuncSetAttribute(tpal3d_kernel<0, false>, a, b) != cudaSuccess ||
             cudaFuncSetAttribute(tpal3d_kernel<1, false>, a, b) != cudaSuccess ||
@@ -1150,7 +1392,7 @@ int tp3_resolve_launch(const T3Params &P, cudaStream_t stream)
     // the record and item counts are only known on the device: fixed grids
     // walk them
     tp3_resolve_kernel<<<4 * sms, 32 * kWarps3, 0, stream>>>(P);
-    const size_t smem = sizeof(float2) * (size_t)kWarpSmemF2 * kWarps3;
+    const size_t smem = walk_smem(P.thr_table != nullptr);
     const unsigned t = 32 * kWarps3, blocks = 3u * (unsigned)sms;
     if (P.thr_table != nullptr) tpal3d_kernel<1, true><<<blocks, t, smem, stream>>>(P);
     else if (P.frame_t2 != nullptr) tpal3d_kernel<2, true><<<blocks, t, smem, stream>>>(P);

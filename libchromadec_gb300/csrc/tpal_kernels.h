@@ -26,16 +26,17 @@ __device__ __forceinline__ const uint16_t *field_at(const Params &P, int f)
 
 // Deferred exact decisions of the 3D transform. The walk decides every bin
 // in FP32 and, for each kx group with a bin inside the guard band, appends
-// one record; the resolve pass decides those bins exactly and lists the work
-// items where FP32 got one wrong, which the exact walk then runs again with
-// every guard-band decision taken exactly, overwriting their output.
+// one record; the resolve pass decides those bins exactly, corrects the
+// record where FP32 got one wrong and lists it. The exact walk then walks the
+// outputs those decisions reach again, taking the decisions of every recorded
+// group from its record, and overwrites them. One warp walks one item, so an
+// item's records form a list in (m, g) order.
 struct UncRecord {
-    int item;            // work item (tile + ntiles * chunk)
-    int tile;            // tile position, tx + ntx * ty
-    int m;               // the Z tile T(2m)
-    int g;               // kx group: column A is kx = 2 + g
+    int item;            // work item (tile + ntiles * chunk; tile = tx + ntx * ty)
+    int mg;              // 4 m + g: the Z tile T(2m), kx group g (column A is kx = 2 + g)
+    int prev, next;      // the item's neighbouring records, or -1
     uint8_t unc[32];     // per lane (ky = kappa(lane)): kz bits inside the guard band
-    uint8_t keep[32];    // per lane: the FP32 decisions the walk used
+    uint8_t keep[32];    // per lane: the FP32 decisions the walk used, corrected by the resolve pass
 };
 
 struct T3Params {
@@ -59,8 +60,8 @@ struct T3Params {
     unsigned int *stats;         // [0] exact decisions taken, [1] of which FP32 was wrong
     // deferred exact decisions (required)
     UncRecord *unc_rec;
-    unsigned int *rerun;         // (work item, step) pairs to walk again exactly (unc_cap pairs)
-    unsigned int *counters;      // [0] records, [1] items listed in rerun
+    unsigned int *rerun;         // corrected records, whose outputs are walked again (unc_cap entries)
+    unsigned int *counters;      // [0] records, [1] entries of rerun
     unsigned int unc_cap;
 };
 
