@@ -87,6 +87,11 @@ __device__ __forceinline__ float l1(float2 a) { return fabsf(a.x) + fabsf(a.y); 
 // tiny real part is below the rounding of any non-degenerate product
 __device__ __forceinline__ float2 mul_negi(float2 a) { return make_float2(a.y, -a.x); }
 
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
+{
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+
 __device__ __forceinline__ df dfc_abs2(dfc v) { return df_add(df_mul(v.re, v.re), df_mul(v.im, v.im)); }
 
 // Squared threshold of visited bin (z, y, x-2) for x in 2..4.
@@ -212,18 +217,26 @@ __device__ __forceinline__ bool df_sim(df a, df b, df t)
 //
 // Shared memory per warp (float4 units): the window [4 pairs][5 kx][16]
 // as (re0, re1, im0, im1) of the pair's two fields, the Z carries
-// [m & 1][5 kx][32] as (slice 4, slice 5), an exchange buffer of 5 x 20 (rows
-// padded by 4: the columns of a quarter-warp fall on different banks), the
-// output spectra [5][32], and the bound terms.
+// [m & 1][5 kx][32] as (slice 4, slice 5), the buffers of the forward and the
+// inverse Y stage, [5 kx][16] in rows of 20 (the columns of a quarter-warp
+// fall on different banks; the inverse one starts with the output spectra,
+// already folded to 16 positions, and ends with the output rows), and the
+// bound terms: 13.7 KB. With 128 registers a thread 16 warps are resident on
+// an SM; the per-bin walk holds two sets of decisions and takes 168 registers
+// and 12 warps.
 //
 // The inverse Y stage of one step runs together with the forward Y stage of
-// the next: two independent chains through the same two exchanges.
+// the next: two independent chains through the same exchange.
 //
 // Measured against the walk before it (one ky per lane in the Z stage, shuffle
-// DFTs in the Y stages, every bin's guard band in the loop): 2,671 -> 1,551
-// warp instructions a step, 526 -> 363 us for 60 fields. The kx pairs unrolled
-// into straight-line code, four blocks a SM at 128 registers (spills) and two
-// warps a block all measured slower.
+// DFTs in the Y stages, every bin's guard band in the loop): 2,671 -> 1,541
+// warp instructions a step, 526 -> 330 us for 60 fields. Both the issue slots
+// and the shared-memory path are about 65 % busy; what is left is latency
+// (short scoreboard) and instruction fetch: unrolling the kx pairs, a second
+// copy of the rare path or straight-line code for both passes each measured
+// slower. So did samples by asynchronous 16-byte copies (coalesced, but with
+// nine shared loads a lane and the addresses: 413 us) and two or three warps
+// a block.
 constexpr int kWarps3 = 4;
 constexpr float kBoundFactor = 2.0f;   // guard band, in units of the per-bin error estimate
 constexpr float kEps32 = 5.9604645e-8f;
@@ -233,8 +246,7 @@ constexpr float kTinyPair = 65000.0f;
 constexpr int kWinF4 = 4 * 5 * 16;
 constexpr int kCarryF4 = 2 * 5 * 32;
 constexpr int kExchF4 = 5 * 20;
-constexpr int kOutF4 = 5 * 32;         // output spectra; then an exchange at 0, then the output rows at kRowsAt
-constexpr int kRowsAt = kOutF4 - 5 * 20;
+constexpr int kOutF4 = 5 * 20;         // output spectra, the inverse exchange, then the output rows
 constexpr int kBndF4 = 4 * 4;          // [4 pairs][8] float2: kx 0..4 and the row term at 5
 constexpr int kWarpF4 = kWinF4 + kCarryF4 + kExchF4 + kOutF4 + kBndF4;
 constexpr int kTwF4 = 4 * 11;          // Y twiddles per quarter r, per block
@@ -254,7 +266,7 @@ struct LaneConst {
     float wy;             // w_y(y0 + 2i), y0 the parity of the field's rows
     int rowL;             // frame line of this lane's row
     bool row_ok, row_fast;
-    long long row_off;    // its first sample within the field
+    int row_off;          // its first sample within the field (negative before the first line)
     int ky;               // of position lane & 15 (below 16)
     int posA, posB;       // window positions of ky and its mirror
     int laneB;            // position (of 32) of the mirror ky
@@ -275,7 +287,7 @@ __device__ __forceinline__ LaneConst lane_const(const T3Params &P, int lane, int
     // Nine aligned words around the row stay inside the field: the row is not
     // its first, and it is not the last unless the words end inside it.
     c.row_fast = tileX >= 0 && fl >= 1 && (fl + 1 < P.fh || tileX + 18 <= P.fw);
-    c.row_off = (long long)fl * P.fw + tileX;
+    c.row_off = fl * P.fw + tileX;
     c.ky = rev4(c.i);
     c.laneB = kappa((40 - c.ky) & 31);
     c.posA = swz(c.i);
@@ -369,8 +381,8 @@ __device__ __forceinline__ void load_row(const T3Params &P, int q, const LaneCon
     } else {
 #pragma unroll
         for (int k = 0; k < 8; k++) {   // never before the field start
-            const long long e = LC.row_off + 2 * k;
-            r.w[k] = (uint32_t)__ldg(fp + (e < 0 ? 0 : e)) | ((uint32_t)__ldg(fp + (e + 1 < 0 ? 0 : e + 1)) << 16);
+            const int e = LC.row_off + 2 * k;
+            r.w[k] = (uint32_t)__ldg(fp + max(e, 0)) | ((uint32_t)__ldg(fp + max(e + 1, 0)) << 16);
         }
         r.w[8] = 0;
     }
@@ -423,22 +435,25 @@ __device__ __forceinline__ void x_forward(const RowWords &row, int q, const Lane
     if (LC.i == 0) bq[2 * 5 + LC.j] = rowl1;
 
     // column DFT bin kx = k+2 of this row (window and centre phase folded)
+    // rows 8..15 write their imaginary part first: 32 different banks a store
     float *xr = reinterpret_cast<float *>(exch) + 4 * LC.i + LC.j;
+    const bool upper = LC.i >= 8;
+    float *xs = xr + (upper ? 2 : 0), *xt = xr + (upper ? 0 : 2);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         float2 X = make_float2(0.f, 0.f);
 #pragma unroll
         for (int x = 0; x < 8; x++) X = __ffma2_rn(c3_xf[k][x], sd[x], X);
         X = __fmul2_rn(X, make_float2(LC.wy, LC.wy));
-        xr[80 * k] = X.x;
-        xr[80 * k + 2] = X.y;
+        xs[80 * k] = upper ? X.y : X.x;
+        xt[80 * k] = upper ? X.x : X.y;
     }
 }
 
 // Y stages, lanes 0..19: the forward one of fields 2q and 2q+1 from their
 // rows in `exch` to window slot q & 3 (and A per kx, the L1 norm of the
 // column-DFT outputs over the rows, into bnd); with INV the inverse one of the
-// output spectra R (re0, re1, im0, im1), their rows into R + kRowsAt.
+// folded output spectra R (re0, re1, im0, im1), in place.
 template <bool INV>
 __device__ __forceinline__ void y_stages(int q, const LaneConst &LC, int lane, float4 *win, float4 *exch, float4 *R,
                                          float2 *bnd, const float4 *tw)
@@ -452,11 +467,8 @@ __device__ __forceinline__ void y_stages(int q, const LaneConst &LC, int lane, f
     if (INV) {
 #pragma unroll
         for (int n = 0; n < 4; n++) {
-            // fold ky = kk and kk + 16, then exp(+i pi kk / 16) for the odd field
-            const float4 *s = R + 32 * k + 4 * r + (n ^ r);
-            const cp2 lo = cp_of(s[0]), hi = cp_of(s[16]);
-            G[n] = ctw({__ffma2_rn(hi.re, make_float2(1.f, -1.f), lo.re), __ffma2_rn(hi.im, make_float2(1.f, -1.f), lo.im)},
-                       twiddle(tw, r, 3 + n), true);
+            // exp(+i pi kk / 16) for the odd field
+            G[n] = ctw(cp_of(y[4 * r + (n ^ r)]), twiddle(tw, r, 3 + n), true);
         }
     }
     float A0 = 0.f, A1 = 0.f;
@@ -496,7 +508,6 @@ __device__ __forceinline__ void y_stages(int q, const LaneConst &LC, int lane, f
         a[n] = cp_of(x[4 * r + (n ^ r)]);
         if (INV) G[n] = cp_of(y[4 * n + (r ^ n)]);
     }
-    if (INV) __syncwarp(kYLanes);   // the output rows overlap the exchange
     const cp2 w0 = cadd(a[0], a[2]), w1 = cadd(a[1], a[3]), w2 = csub(a[0], a[2]), d3 = csub(a[1], a[3]);
     // the odd branch of span 2 times exp(-i pi/2): (d3.im, -d3.re)
     const cp2 o[4] = {cadd(w0, w1), csub(w0, w1), {add2(w2.re, d3.im), sub2(w2.im, d3.re)},
@@ -509,11 +520,11 @@ __device__ __forceinline__ void y_stages(int q, const LaneConst &LC, int lane, f
         const cp2 f1 = ctw(G[1], t2, true), f3 = ctw(G[3], t2, true);
         const cp2 g0 = cadd(G[0], f1), g1 = csub(G[0], f1);
         const cp2 g2 = ctw(cadd(G[2], f3), t0, true), g3 = ctw(csub(G[2], f3), t1, true);
-        float4 *z = y + kRowsAt;
-        z[r] = f4_of(cadd(g0, g2));
-        z[r + 4] = f4_of(cadd(g1, g3));
-        z[r + 8] = f4_of(csub(g0, g2));
-        z[r + 12] = f4_of(csub(g1, g3));
+        __syncwarp(kYLanes);   // the exchange has been read
+        y[r] = f4_of(cadd(g0, g2));
+        y[r + 4] = f4_of(cadd(g1, g3));
+        y[r + 8] = f4_of(csub(g0, g2));
+        y[r + 12] = f4_of(csub(g1, g3));
     }
 }
 
@@ -572,19 +583,28 @@ struct ZInverse {
         sum(ym, om);
         O1 = make_float2(-O1.x, -O1.y);
     }
-    // R(field 2m) = slice 0 + carried slice 4 of tile 2m-4, R(2m+1) = slice 1
-    // + carried slice 5; then carry this tile's slices 4, 5 for frame m+2.
-    __device__ __forceinline__ void finish(float4 *carry, float4 *R, int k, int at) const
+    // The output spectra at one ky, field 2m: slice 0 + carried slice 4 of
+    // tile 2m-4, field 2m+1: slice 1 + carried slice 5; then this tile's
+    // slices 4, 5 are carried for frame m+2.
+    __device__ __forceinline__ cp2 finish(float4 *carry) const
     {
-        const float4 c = carry[32 * k + at];
+        const float4 c = *carry;
         const float2 s0 = add2(E0, O0), d0 = sub2(E0, O0);
         const float2 s1 = make_float2(__fadd_rn(E1.x, O1.x), __fadd_rn(E1.y, O1.y));
         const float2 d1 = make_float2(__fsub_rn(E1.x, O1.x), __fsub_rn(E1.y, O1.y));
-        R[32 * k + swz(at)] = make_float4(__fadd_rn(s0.x, c.x), __fadd_rn(s1.x, c.z), __fadd_rn(s0.y, c.y),
-                                          __fadd_rn(s1.y, c.w));
-        carry[32 * k + at] = make_float4(d0.x, d0.y, d1.x, d1.y);
+        *carry = make_float4(d0.x, d0.y, d1.x, d1.y);
+        return {make_float2(__fadd_rn(s0.x, c.x), __fadd_rn(s1.x, c.z)),
+                make_float2(__fadd_rn(s0.y, c.y), __fadd_rn(s1.y, c.w))};
     }
 };
+
+// The inverse Y stage's first step: ky and ky + 16 of the two fields added
+// (even rows) or subtracted (odd rows).
+__device__ __forceinline__ cp2 fold_ky(cp2 lo, cp2 hi)
+{
+    const float2 s = make_float2(1.f, -1.f);
+    return {__ffma2_rn(hi.re, s, lo.re), __ffma2_rn(hi.im, s, lo.im)};
+}
 
 __device__ __forceinline__ void z_rotate(const float2 (&y)[8], float2 (&o)[4])
 {
@@ -592,9 +612,9 @@ __device__ __forceinline__ void z_rotate(const float2 (&y)[8], float2 (&o)[4])
     for (int i = 0; i < 4; i++) o[i] = cmulc(y[2 * i + 1], c3_tw32[4 * (2 * i + 1)]);
 }
 
-// Masks column Y at ky (position `at`) by k and at ky + 16 by kh, inverse Z
-// and overlap-add of both. MOVED: kh is k moved by 4, the sums share the
-// masked bins.
+// Masks column Y at ky (position `at` of 32) by k and at ky +- 16 by kh,
+// inverse Z and overlap-add of both, and their folded output spectrum into R.
+// MOVED: kh is k moved by 4, the sums share the masked bins.
 template <bool MOVED>
 __device__ __forceinline__ void z_inverse(const float2 (&Y)[8], const float (&k)[8], const float (&kh)[8],
                                           float4 *carry, float4 *R, int col, int at)
@@ -605,7 +625,7 @@ __device__ __forceinline__ void z_inverse(const float2 (&Y)[8], const float (&k)
     z_rotate(y, o);
     ZInverse Z;
     Z.sum(y, o);
-    Z.finish(carry, R, col, at);
+    const cp2 a = Z.finish(carry + 32 * col + at);
     if (MOVED) {
         Z.sum_moved(y, o);
     } else {
@@ -615,7 +635,13 @@ __device__ __forceinline__ void z_inverse(const float2 (&Y)[8], const float (&k)
         z_rotate(yh, o);
         Z.sum(yh, o);
     }
-    Z.finish(carry, R, col, at ^ 16);
+    const cp2 b = Z.finish(carry + 32 * col + (at ^ 16));
+    cp2 g = fold_ky(a, b);
+    if (at >= 16) {   // a is the upper half: component 1 is b - a
+        g.re.y = -g.re.y;
+        g.im.y = -g.im.y;
+    }
+    R[20 * col + swz(at & 15)] = f4_of(g);
 }
 
 __device__ __forceinline__ bool fsim(float a, float b, float t) { return (__fmaf_rn(-b, t, a) >= 0.f) && (__fmaf_rn(-a, t, b) >= 0.f); }
@@ -751,9 +777,12 @@ __device__ __forceinline__ void x_inverse_store(const T3Params &P, const LaneCon
 #pragma unroll
     for (int x = 0; x < 8; x++) CS[x] = make_float2(0.f, 0.f);
     const float *yr = reinterpret_cast<const float *>(rows) + 4 * LC.i + LC.j;
+    const bool upper = LC.i >= 8;   // reads its imaginary part first: 32 different banks a load
+    const float *ys = yr + (upper ? 2 : 0), *yt = yr + (upper ? 0 : 2);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        const float2 G = make_float2(yr[80 * k], yr[80 * k + 2]);
+        const float u = ys[80 * k], v = yt[80 * k];
+        const float2 G = make_float2(upper ? v : u, upper ? u : v);
 #pragma unroll
         for (int x = 0; x < 8; x++) CS[x] = __ffma2_rn(G, c3_xi[k][x], CS[x]);
     }
@@ -807,7 +836,7 @@ __device__ __forceinline__ int find_record(const T3Params &P, int rec, int mg)
 // the corrected records; it writes the same output locations, so its result
 // replaces the FP32 one.
 template <int TMODE, bool EXACT>
-__global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
+__global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpal3d_kernel(T3Params P)
 {
     constexpr bool PER_BIN = (TMODE == 1);
     const int lane = threadIdx.x & 31;
@@ -858,11 +887,11 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
     for (int m = m0 - 5; m <= m1; m++) {
         __syncwarp();
         if (m < m1) x_forward(row, m + 3, LC, exch, bnd);   // fields 2m+6, 2m+7
-        if (m + 1 < m1) load_row(P, m + 4, LC, row);        // the next step's, in flight until then
         __syncwarp();
+        if (m + 1 < m1) load_row(P, m + 4, LC, row);   // the next step's
         if (lane < 20) y_stages<true>(m + 3, LC, lane, win, exch, R, bnd, tw);
         __syncwarp();
-        if (m > m0) x_inverse_store(P, LC, R + kRowsAt, m - 1, tileX, cls);
+        if (m > m0) x_inverse_store(P, LC, R, m - 1, tileX, cls);
         if (m < m0 - 2 || (EXACT && m == m0 - 1) || m == m1) continue;
         __syncwarp();   // the output rows have been read: R may be written
 
@@ -897,6 +926,7 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
             }
             return d >= 0.f;
         };
+        unsigned hits = 0;   // kx groups that reached the screen's bound
         int fix[3] = {-1, -1, -1};
         if (EXACT)
             for (int g = 0; g < 3; g++) fix[g] = find_record(P, rec, m * 4 + g);
@@ -941,12 +971,8 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
             z_inverse<!PER_BIN>(YA, k, kh, carry, R, h, lane & 15);
             z_inverse<!PER_BIN>(YB, kr, khr, carry, R, 4 - h, LC.laneB);
             if (!EXACT) {
-                const unsigned hit = __ballot_sync(0xffffffffu, u);
-                for (int g = 0; g < 2; g++)
-                    if (hit & (0xFFFFu << (16 * g))) {
-                        const float ekA = __shfl_sync(0xffffffffu, SB.ek, g), ekB = __shfl_sync(0xffffffffu, SB.ek, 4 - g);
-                        record_group<PER_BIN>(P, LC, win, thr, item, m, g, lane, tf_m, ekA, ekB, last);
-                    }
+                const unsigned b = __ballot_sync(0xffffffffu, u);
+                hits = ((b & 0xFFFFu) != 0 ? 1u : 0u) | (b >> 16 != 0 ? 2u : 0u);
             }
         }
         // Pass 2: kx 4, whose mirror bins' magnitudes come from the lanes
@@ -973,10 +999,17 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_kernel(T3Params P)
             z_rotate(y, o);
             ZInverse Z;
             Z.sum(y, o);
-            Z.finish(carry, R, 2, lane);
-            if (!EXACT && __any_sync(0xffffffffu, u)) {
-                const float ek = __shfl_sync(0xffffffffu, SB.ek, 2);
-                record_group<PER_BIN>(P, LC, win, thr, item, m, 2, lane, tf_m, ek, ek, last);
+            const cp2 own = Z.finish(carry + 32 * 2 + lane);
+            const cp2 high = {shfl_xor2(own.re, 16), shfl_xor2(own.im, 16)};
+            if (lane < 16) R[20 * 2 + LC.posA] = f4_of(fold_ky(own, high));
+            if (!EXACT && __any_sync(0xffffffffu, u)) hits |= 4u;
+        }
+        if (!EXACT && hits != 0) {   // one copy of the rare path
+#pragma unroll 1
+            for (int g = 0; g < 3; g++) {
+                if (!(hits >> g & 1)) continue;
+                const float ekA = __shfl_sync(0xffffffffu, SB.ek, g), ekB = __shfl_sync(0xffffffffu, SB.ek, 4 - g);
+                record_group<PER_BIN>(P, LC, win, thr, item, m, g, lane, tf_m, ekA, ekB, last);
             }
         }
     }
@@ -1029,11 +1062,11 @@ __global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_learned_kernel(T3Param
     for (int m = m0 - 5; m <= m1; m++) {
         __syncwarp();
         if (m < m1) x_forward(row, m + 3, LC, exch, bnd);
-        if (m + 1 < m1) load_row(P, m + 4, LC, row);
         __syncwarp();
+        if (m + 1 < m1) load_row(P, m + 4, LC, row);
         if (lane < 20) y_stages<PASS == 1>(m + 3, LC, lane, win, exch, R, bnd, tw);
         __syncwarp();
-        if (PASS == 1 && m > m0) x_inverse_store(P, LC, R + kRowsAt, m - 1, tileX, cls);
+        if (PASS == 1 && m > m0) x_inverse_store(P, LC, R, m - 1, tileX, cls);
         if (m < m0 - 2 || m == m1) continue;
         __syncwarp();
         const long long base = ((long long)(m - L.z0) * ntiles + tile) * 1280;
