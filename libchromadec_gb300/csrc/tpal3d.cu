@@ -36,6 +36,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
+#include <vector>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -57,13 +58,14 @@ __constant__ float c3_wx[16];      // w_x(x)
 __constant__ float c3_wz[8];       // w_z(z)
 __constant__ float2 c3_tw16[16];   // exp(-2 pi i r / 16)
 __constant__ float2 c3_tw32[32];   // exp(-2 pi i r / 32)
-// double-float tables for the exact decision path
-// w_x(x) exp(-2 pi i kx x/16) as 60-bit fixed point, c * 2^60 = hi * 2^30 + lo
-// (lo in [0, 2^30)): re.hi, re.lo, im.hi, im.lo
+// Fixed-point tables of the exact decision path:
+// w_x(x) exp(-2 pi i kx x/16), c * 2^60 = hi * 2^30 + lo (lo in [0, 2^30)):
+// re.hi, re.lo, im.hi, im.lo
 __constant__ int c3_qx[5][16][4];
-__constant__ float c3_dfwy[32][2];     // w_y(y)
-__constant__ float c3_dfwz[8][2];      // w_z(z)
-__constant__ float c3_dftw32[32][4];   // exp(-2 pi i r/32)
+// w_z(z) w_y(y) exp(-2 pi i r/32), c * 2^59 = hi * 2^29 + lo (lo in [0, 2^29)),
+// for z < 4 and y < 16 (both windows are symmetric): [z][y][r], the same order
+constexpr int kQYZ = 4 * 16 * 32;
+__device__ int4 g3_qyz[kQYZ];
 
 static bool g_tp3_constants_ready[64];
 
@@ -92,8 +94,6 @@ __device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
     return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
 
-__device__ __forceinline__ df dfc_abs2(dfc v) { return df_add(df_mul(v.re, v.re), df_mul(v.im, v.im)); }
-
 // Squared threshold of visited bin (z, y, x-2) for x in 2..4.
 struct Thr {
     float f;
@@ -114,43 +114,38 @@ __device__ __forceinline__ Thr thr_of(const T3Params &P, int m, int kz, int ky, 
 }
 
 // ---------------------------------------------------------------------------
-// Double-float X stage of one row for columns kx and 8 - kx. The second
-// column's coefficients are the first's conjugated with sign (-1)^x
-// (w(x) exp(-2 pi i (8-k) x / 16) = (-1)^x conj(w(x) exp(-2 pi i k x / 16))),
-// so the products are formed once and summed twice.
+// Exact decisions in fixed point
 // ---------------------------------------------------------------------------
-// An integer below 2^51 in magnitude as double-float, through 32-bit
-// conversions (the 64-bit ones run on the FP64 pipe, which this GPU has
-// little of): v = hi * 2^32 + mid * 2^16 + low, each part exact in FP32.
-__device__ __forceinline__ df df_from_i51(long long v)
-{
-    const float fh = (float)(int)(v >> 32) * 4294967296.0f;   // |v >> 32| < 2^19: exact
-    const unsigned lo = (unsigned)v;
-    const float fm = (float)(lo >> 16) * 65536.0f, fl = (float)(lo & 0xFFFFu);
-    return df_add(two_sum(fh, fm), df_make(fl));
-}
+// A bin is a sum over 8 fields x 16 rows of a row's X-stage value times
+// w_z w_y exp(-2 pi i (ky y + 4 kz z) / 32). Both factors are integers of two
+// words, every product an exact 64-bit integer product, the sums exact; what
+// is rounded is each row's value (at 2^-39), the product of the two low words
+// (dropped, below 2^-40) and each lane's sum (at 2^-38), against bins of 2^8 and
+// more: the result is at least as near the true spectrum as FP64's.
+struct fx2 {
+    int rh, rl, ih, il;   // value * 2^39 = hi * 2^29 + lo, lo in [0, 2^29)
+};
 
-__device__ __forceinline__ df df_from_fixed60(long long hi_acc, long long lo_acc)
+__device__ __forceinline__ void fx_split(long long hi_acc, long long lo_acc, int &h, int &l)
 {
     // v = hi_acc * 2^-30 + lo_acc * 2^-60; hi_acc and lo_acc are below 2^51
-    const df v = df_add(df_from_i51(hi_acc), df_make((float)(int)(lo_acc >> 30) + (float)(int)(lo_acc & 0x3FFFFFFF) *
-                                                                                    9.3132257461547852e-10f));
-    return {v.hi * 9.3132257461547852e-10f, v.lo * 9.3132257461547852e-10f};   // 2^-30
+    const long long v = (hi_acc << 9) + ((lo_acc + (1 << 20)) >> 21);
+    h = (int)(v >> 29);
+    l = (int)v & ((1 << 29) - 1);
 }
 
-// The X stage in 60-bit fixed point: each sample times each coefficient
-// word is an exact 64-bit integer product, so the sums are exact and the one
-// rounding is the conversion to double-float (about 2^-47 of the sum).
+// X stage of one row for columns kx and 8 - kx. The second column's
+// coefficients are the first's conjugated with sign (-1)^x
+// (w(x) exp(-2 pi i (8-k) x / 16) = (-1)^x conj(w(x) exp(-2 pi i k x / 16))),
+// so the products are formed once: even and odd samples summed apart, column
+// kx is even + odd, column 8 - kx the conjugate of even - odd.
 __device__ __forceinline__ void x_row_pair(const uint16_t *field, long long base, long long field_len, int black,
-                                           int kx, dfc &xa, dfc &xb)
+                                           int kx, fx2 &xa, fx2 &xb)
 {
-    // even and odd samples summed apart: column kx is even + odd, column
-    // 8 - kx ((-1)^x times the conjugate) is the conjugate of even - odd --
-    // the same integers as summing each column's products directly
     long long e[4] = {0, 0, 0, 0}, o[4] = {0, 0, 0, 0};   // re.hi, re.lo, im.hi, im.lo
     int a[16];
     if (base >= 1 && base + 18 <= field_len) {
-        // nine aligned 32-bit words and a funnel shift, as in forward_pair
+        // nine aligned 32-bit words and a funnel shift, as the walk's rows
         const uintptr_t pa = reinterpret_cast<uintptr_t>(field + base);
         const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
         const unsigned sh = (unsigned)(pa & 2) * 8u;
@@ -177,8 +172,48 @@ __device__ __forceinline__ void x_row_pair(const uint16_t *field, long long base
 #pragma unroll
         for (int k = 0; k < 4; k++) acc[k] += (long long)a[x] * c[k];
     }
-    xa = {df_from_fixed60(e[0] + o[0], e[1] + o[1]), df_from_fixed60(e[2] + o[2], e[3] + o[3])};
-    xb = {df_from_fixed60(e[0] - o[0], e[1] - o[1]), df_from_fixed60(o[2] - e[2], o[3] - e[3])};
+    fx_split(e[0] + o[0], e[1] + o[1], xa.rh, xa.rl);
+    fx_split(e[2] + o[2], e[3] + o[3], xa.ih, xa.il);
+    fx_split(e[0] - o[0], e[1] - o[1], xb.rh, xb.rl);
+    fx_split(o[2] - e[2], o[3] - e[3], xb.ih, xb.il);
+}
+
+// (high, middle) sums of complex products: high counts 2^-40, middle 2^-69.
+struct fxsum {
+    long long rh, rm, ih, im;
+    __device__ __forceinline__ void mac(const fx2 &x, int4 c)   // c: re.hi, re.lo, im.hi, im.lo
+    {
+        const int nh = -c.z, nl = -c.w;
+        rh += (long long)x.rh * c.x;
+        rh += (long long)x.ih * nh;
+        rm += (long long)x.rh * c.y;
+        rm += (long long)x.rl * c.x;
+        rm += (long long)x.ih * nl;
+        rm += (long long)x.il * nh;
+        ih += (long long)x.rh * c.z;
+        ih += (long long)x.ih * c.x;
+        im += (long long)x.rh * c.w;
+        im += (long long)x.rl * c.z;
+        im += (long long)x.ih * c.y;
+        im += (long long)x.il * c.x;
+    }
+};
+
+// a 64-bit integer below 2^63 in magnitude as double-float (about 2^-48 of
+// it), through 32-bit conversions (the 64-bit ones run on the FP64 pipe,
+// which this GPU has little of)
+__device__ __forceinline__ df df_from_i64(long long v)
+{
+    const float fh = (float)(int)(v >> 40) * 1099511627776.0f;              // below 2^23: exact
+    const float fm = (float)(int)((v >> 20) & 0xFFFFF) * 1048576.0f;        // 20 bits: exact
+    const float fl = (float)(int)(v & 0xFFFFF);
+    return df_add(two_sum(fh, fm), df_make(fl));
+}
+
+__device__ __forceinline__ long long shfl_xor_i64(long long v, int m)
+{
+    const int lo = __shfl_xor_sync(0xffffffffu, (int)v, m), hi = __shfl_xor_sync(0xffffffffu, (int)(v >> 32), m);
+    return (long long)(((unsigned long long)(unsigned)hi << 32) | (unsigned)lo);
 }
 
 // sim(a, b, t) = !(a < b t || b < a t) evaluated in double-float
@@ -1191,109 +1226,121 @@ int tp3_learned_launch(const T3Params &P, const T3Learn &L, int pass, cudaStream
 // ---------------------------------------------------------------------------
 // Deferred exact decisions
 // ---------------------------------------------------------------------------
-// One warp per record: decide its guard-band bins exactly in double-float
-// (the arithmetic of exact_pair, with the X stage of the record's two kx
-// columns computed once for all its bins) and, where an exact decision
-// differs from the FP32 one the walk used, correct the record's decisions and
-// list it for the exact walk.
+// One warp per record: decide its guard-band bins exactly and, where an exact
+// decision differs from the FP32 one the walk used, correct the record's
+// decisions and list it for the exact walk. The X stage of the record's two kx
+// columns is computed once for all its bins; lane (z, part) owns rows
+// 4 part .. 4 part + 3 of field 2m + z. A bin at (kz + 4, ky + 16) has the
+// magnitudes of the bin at (kz, ky) (see the walk), so both are decided from
+// one evaluation.
+//
+// Bound by integer multiplies: 256 for a record's X stage, 96 a bin a lane.
+// 615 -> 258 us for a 500-field capture (90 -> 38 us for 60); double-float Y
+// and Z stages, which this replaces, took about 1,500 instructions a bin, and
+// ran twice, for ky and ky + 16.
 __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned n = min(P.counters[0], P.unc_cap);
+    if (blockIdx.x * kWarps3 >= n) return;
     unsigned n_exact = 0, n_flip = 0;
     const int z = lane >> 2, part = lane & 3;
-    // Window-scaled double-float twiddles, w_y(y) exp(-2 pi i r/32) for every
-    // (y, r) and w_z(z) exp(-2 pi i 4 r/32) for every (z, r), formed once per
-    // block with the same df_mul the products would use (the same values),
-    // read from shared memory: a warp reads them with 8 distinct indices,
-    // which the constant cache would serialise. Rows padded by one entry.
-    __shared__ float4 s_yw[32][33], s_zw[8][8];
-    for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
-        const int y = i >> 5, r = i & 31;
-        const df w = {c3_dfwy[y][0], c3_dfwy[y][1]};
-        const df re = df_mul({c3_dftw32[r][0], c3_dftw32[r][1]}, w), im = df_mul({c3_dftw32[r][2], c3_dftw32[r][3]}, w);
-        s_yw[y][r] = make_float4(re.hi, re.lo, im.hi, im.lo);
-    }
-    for (int i = threadIdx.x; i < 8 * 8; i += blockDim.x) {
-        const int zz = i >> 3, r = i & 7;
-        const df w = {c3_dfwz[zz][0], c3_dfwz[zz][1]};
-        const df re = df_mul({c3_dftw32[4 * r][0], c3_dftw32[4 * r][1]}, w);
-        const df im = df_mul({c3_dftw32[4 * r][2], c3_dftw32[4 * r][3]}, w);
-        s_zw[zz][r] = make_float4(re.hi, re.lo, im.hi, im.lo);
-    }
+    extern __shared__ int4 s_qyz[];
+    for (int i = threadIdx.x; i < kQYZ; i += blockDim.x) s_qyz[i] = g3_qyz[i];
     __syncthreads();
-    auto as_dfc = [](float4 v) -> dfc { return {{v.x, v.y}, {v.z, v.w}}; };
     for (unsigned rec = blockIdx.x * kWarps3 + warp; rec < n; rec += gridDim.x * kWarps3) {
         UncRecord &R = P.unc_rec[rec];
         const int tile = R.item % (P.ntx * P.nty), m = R.mg >> 2, g = R.mg & 3;
         const int tileX = P.tileX0 + 8 * (tile % P.ntx), tileY = P.tileY0 + 16 * (tile / P.ntx);
         const int kxa = 2 + g;
         unsigned keep = R.keep[lane];
-        unsigned unc = R.unc[lane];
-        // X stage of this lane's four rows of field 2m + z, both columns
+        const unsigned unc = R.unc[lane];
         const int f = 2 * m + z;
         const int p = (f & 1) ^ P.swap;
         const int y0 = (p - tileY) & 1;
-        dfc xa[4], xb[4];
+        fx2 xa[4], xb[4];
         const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
 #pragma unroll
         for (int r4 = 0; r4 < 4; r4++) {
-            xa[r4] = xb[r4] = {{0.f, 0.f}, {0.f, 0.f}};
+            xa[r4] = xb[r4] = {0, 0, 0, 0};
             const int L = tileY + y0 + 2 * (part * 4 + r4);
             if (fp == nullptr || L < P.fafl || L > P.lafl) continue;
             const long long base = (long long)(L >> 1) * P.fw + tileX;   // within the field
             x_row_pair(fp, base, (long long)P.fh * P.fw, P.black, kxa, xa[r4], xb[r4]);
         }
+        // bins of ky < 16 to evaluate: this lane's own and those of ky + 16 moved by 4
+        const unsigned up = __shfl_xor_sync(0xffffffffu, unc, 16);
+        unsigned todo = lane < 16 ? unc | ((up << 4 | up >> 4) & 0xFFu) : 0u;
         bool flipped = false;
-        unsigned any = __ballot_sync(0xffffffffu, unc != 0);
+        unsigned any = __ballot_sync(0xffffffffu, todo != 0);
         while (any) {
             const int src = __ffs(any) - 1;
-            const unsigned su = __shfl_sync(0xffffffffu, unc, src);
-            const int kz = __ffs(su) - 1;
-            const int kyb = kappa(src);
-            const int kzr = (10 - kz) & 7, kybr = (40 - kyb) & 31;
-            // Y stage over this lane's rows, then the 4 row groups, then Z
-            dfc accb = {{0.f, 0.f}, {0.f, 0.f}}, accr = accb;
+            const int kz = __ffs(__shfl_sync(0xffffffffu, todo, src)) - 1;
+            const int ky = kappa(src), kzr = (10 - kz) & 7, kyr = (40 - ky) & 31;
+            fxsum b = {0, 0, 0, 0}, r = b;
+            const int4 *q = s_qyz + (z < 4 ? z : 7 - z) * (16 * 32);
 #pragma unroll
             for (int r4 = 0; r4 < 4; r4++) {
                 const int y = y0 + 2 * (part * 4 + r4);
-                const dfc cb = as_dfc(s_yw[y][(kyb * y) & 31]), cr = as_dfc(s_yw[y][(kybr * y) & 31]);
-                accb = dfc_add(accb, dfc_mul(xa[r4], cb));
-                accr = dfc_add(accr, dfc_mul(xb[r4], cr));
+                const int4 *c = q + (y < 16 ? y : 31 - y) * 32;
+                b.mac(xa[r4], c[(ky * y + 4 * kz * z) & 31]);
+                r.mac(xb[r4], c[(kyr * y + 4 * kzr * z) & 31]);
             }
-            accb = dfc_add(accb, dfc_shfl_xor(accb, 1));
-            accb = dfc_add(accb, dfc_shfl_xor(accb, 2));
-            accr = dfc_add(accr, dfc_shfl_xor(accr, 1));
-            accr = dfc_add(accr, dfc_shfl_xor(accr, 2));
-            {
-                const dfc tb = as_dfc(s_zw[z][(kz * z) & 7]), tr = as_dfc(s_zw[z][(kzr * z) & 7]);
-                accb = dfc_mul(accb, tb);
-                accr = dfc_mul(accr, tr);
+            // the sums of the 32 lanes, in units of 2^-38: lanes 0-7 end with
+            // the bin's real part, 8-15 its imaginary part, 16-31 the mirror's
+            const long long v0 = (b.rh >> 2) + (b.rm >> 31), v1 = (b.ih >> 2) + (b.im >> 31);
+            const long long v2 = (r.rh >> 2) + (r.rm >> 31), v3 = (r.ih >> 2) + (r.im >> 31);
+            const bool h16 = lane & 16, h8 = lane & 8;
+            const long long s0 = (h16 ? v2 : v0) + shfl_xor_i64(h16 ? v0 : v2, 16);
+            const long long s1 = (h16 ? v3 : v1) + shfl_xor_i64(h16 ? v1 : v3, 16);
+            long long s = (h8 ? s1 : s0) + shfl_xor_i64(h8 ? s0 : s1, 8);
+#pragma unroll
+            for (int h = 4; h >= 1; h >>= 1) s += shfl_xor_i64(s, h);
+            const df v = df_from_i64(s);
+            const df sq = df_mul({v.hi * 3.637978807091713e-12f, v.lo * 3.637978807091713e-12f},   // 2^-38
+                                 {v.hi * 3.637978807091713e-12f, v.lo * 3.637978807091713e-12f});
+            const df mag = df_add(sq, df_shfl_xor(sq, 8));
+            const df oth = df_shfl_xor(mag, 16);
+            const df mb = h16 ? oth : mag, mr = h16 ? mag : oth;
+            bool sim = df_sim(mb, mr, thr_of(P, m, kz, ky, kxa).d);
+            if (kxa == 4) sim |= df_sim(mb, mr, thr_of(P, m, kzr, kyr, 4).d);
+            bool simh = sim;   // of (kz + 4, ky + 16)
+            if (P.thr_table != nullptr) {
+                simh = df_sim(mb, mr, thr_of(P, m, kz ^ 4, ky + 16, kxa).d);
+                if (kxa == 4) simh |= df_sim(mb, mr, thr_of(P, m, kzr ^ 4, kyr ^ 16, 4).d);
             }
-            accb = dfc_add(accb, dfc_shfl_xor(accb, 4));
-            accb = dfc_add(accb, dfc_shfl_xor(accb, 8));
-            accb = dfc_add(accb, dfc_shfl_xor(accb, 16));
-            accr = dfc_add(accr, dfc_shfl_xor(accr, 4));
-            accr = dfc_add(accr, dfc_shfl_xor(accr, 8));
-            accr = dfc_add(accr, dfc_shfl_xor(accr, 16));
-            const df mb = dfc_abs2(accb), mr = dfc_abs2(accr);
-            bool sim = df_sim(mb, mr, thr_of(P, m, kz, kyb, kxa).d);
-            if (kxa == 4) sim |= df_sim(mb, mr, thr_of(P, m, kzr, kybr, 4).d);
-            const bool old = ((__shfl_sync(0xffffffffu, keep, src) >> kz) & 1u) != 0;
-            flipped |= (old != sim);
+            // the bins decided: this one, its copy at ky + 16, and for kx = 4
+            // the mirrors of both, which visit too
+            const int lr = kappa(kyr);
+            const unsigned bit = 1u << kz, bith = 1u << (kz ^ 4), bitr = 1u << kzr, bitrh = 1u << (kzr ^ 4);
+            if (g == 2) {
+                if (lane == lr) todo &= ~bitr;
+                if (lane == (lr ^ 16)) todo &= ~bitrh;
+            }
             if (lane == src) {
-                n_exact++;
-                if (old != sim) n_flip++;
-                unc &= ~(1u << kz);
-                keep = (keep & ~(1u << kz)) | ((unsigned)sim << kz);
+                todo &= ~bit;
+                const bool was = keep & bit;
+                n_exact += (unc & bit) != 0;
+                if (was != sim) {
+                    n_flip++;
+                    keep ^= bit;
+                    flipped = true;
+                }
             }
-            if (g == 2 && lane == kappa(kybr)) {   // kx = 4: the same pair
-                unc &= ~(1u << kzr);
-                keep = (keep & ~(1u << kzr)) | ((unsigned)sim << kzr);
+            if (lane == src + 16) {
+                const bool was = keep & bith;
+                n_exact += (unc & bith) != 0;
+                if (was != simh) {
+                    n_flip++;
+                    keep ^= bith;
+                    flipped = true;
+                }
             }
-            any = __ballot_sync(0xffffffffu, unc != 0);
+            if (g == 2 && lane == lr) keep = sim ? keep | bitr : keep & ~bitr;
+            if (g == 2 && lane == (lr ^ 16)) keep = simh ? keep | bitrh : keep & ~bitrh;
+            any = __ballot_sync(0xffffffffu, todo != 0);
         }
-        if (flipped) {   // the exact walk takes this group's decisions from the record
+        if (__any_sync(0xffffffffu, flipped)) {   // the exact walk takes this group's decisions from the record
             R.keep[lane] = (uint8_t)keep;
             if (lane == 0) {
                 const unsigned at = atomicAdd(P.counters + 1, 1u);
@@ -1311,12 +1358,6 @@ __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
 // Host side
 // ---------------------------------------------------------------------------
 static double rc_window(int n, int N) { return 0.5 - (0.5 * cos((2 * M_PI * (n + 0.5)) / N)); }
-
-static void split_df(double v, float &hi, float &lo)
-{
-    hi = (float)v;
-    lo = (float)(v - (double)hi);
-}
 
 int tp3_init_constants(int device)
 {
@@ -1341,7 +1382,7 @@ int tp3_init_constants(int device)
     float2 tw16[16], tw32[32];
     for (int r = 0; r < 16; r++) tw16[r] = make_float2((float)cos(-2 * M_PI * r / 16), (float)sin(-2 * M_PI * r / 16));
     for (int r = 0; r < 32; r++) tw32[r] = make_float2((float)cos(-2 * M_PI * r / 32), (float)sin(-2 * M_PI * r / 32));
-    float dfwy[32][2], dfwz[8][2], dftw32[32][4];
+    std::vector<int4> qyz(kQYZ);
     int qx[5][16][4];
     for (int k = 0; k < 5; k++)
         for (int x = 0; x < 16; x++) {
@@ -1354,11 +1395,17 @@ int tp3_init_constants(int device)
                 qx[k][x][2 * c + 1] = (int)(q & ((1LL << 30) - 1));
             }
         }
-    for (int y = 0; y < 32; y++) split_df(rc_window(y, 32), dfwy[y][0], dfwy[y][1]);
-    for (int z = 0; z < 8; z++) split_df(rc_window(z, 8), dfwz[z][0], dfwz[z][1]);
-    for (int r = 0; r < 32; r++) {
-        split_df(cos(-2 * M_PI * r / 32), dftw32[r][0], dftw32[r][1]);
-        split_df(sin(-2 * M_PI * r / 32), dftw32[r][2], dftw32[r][3]);
+    for (int e = 0; e < kQYZ; e++) {
+        const int z = e / (16 * 32), y = (e / 32) % 16, r = e % 32;
+        const double w = rc_window(z, 8) * rc_window(y, 32), an = -2.0 * M_PI * r / 32;
+        int w4[4];
+        const double parts[2] = {w * cos(an), w * sin(an)};
+        for (int c = 0; c < 2; c++) {
+            const long long q = llround(parts[c] * 576460752303423488.0);   // 2^59
+            w4[2 * c] = (int)(q >> 29);
+            w4[2 * c + 1] = (int)(q & ((1LL << 29) - 1));
+        }
+        qyz[e] = make_int4(w4[0], w4[1], w4[2], w4[3]);
     }
 #define TPAL_CPY(sym, src)                                                  \
     if (cudaMemcpyToSymbol(sym, src, sizeof(src)) != cudaSuccess) return -1;
@@ -1376,9 +1423,7 @@ int tp3_init_constants(int device)
     TPAL_CPY(c3_tw16, tw16);
     TPAL_CPY(c3_tw32, tw32);
     TPAL_CPY(c3_qx, qx);
-    TPAL_CPY(c3_dfwy, dfwy);
-    TPAL_CPY(c3_dfwz, dfwz);
-    TPAL_CPY(c3_dftw32, dftw32);
+    if (cudaMemcpyToSymbol(g3_qyz, qyz.data(), sizeof(int4) * kQYZ) != cudaSuccess) return -1;
 #undef TPAL_CPY
     if (device >= 0 && device < 64) g_tp3_constants_ready[device] = true;
     return 0;
@@ -1424,7 +1469,7 @@ int tp3_resolve_launch(const T3Params &P, cudaStream_t stream)
     if (sms <= 0) sms = 1;
     // the record and item counts are only known on the device: fixed grids
     // walk them
-    tp3_resolve_kernel<<<4 * sms, 32 * kWarps3, 0, stream>>>(P);
+    tp3_resolve_kernel<<<4 * sms, 32 * kWarps3, sizeof(int4) * kQYZ, stream>>>(P);
     const size_t smem = walk_smem(P.thr_table != nullptr);
     const unsigned t = 32 * kWarps3, blocks = 3u * (unsigned)sms;
     if (P.thr_table != nullptr) tpal3d_kernel<1, true><<<blocks, t, smem, stream>>>(P);
