@@ -27,9 +27,20 @@
 //  * Every output format of the ABI is packed here: yuv444p16/ps, rgb48
 //    (interleaved, truncating), rgbs, gray16, grays.
 //
-// One block: 16 field lines (8 with yNR) of one output field, 256 threads; a
-// work item produces 8 consecutive samples of one line from a register window
-// of the four vertically combined chroma rows.
+// One block: up to 16 field lines (8 with yNR) of one output field, 256
+// threads; a work item produces 8 consecutive samples of one line from a
+// register window of the four vertically combined chroma rows. Items start at
+// the first active sample, so an item's samples are 8 aligned output pixels;
+// XO, the carrier phase of that sample, is a template parameter.
+//
+// Measured on a 500-field capture against the kernel before it (items on the
+// carrier phase, scalar FIR, run-time format): 1.85 -> 1.33 ms, 2,124 -> 1,395
+// warp instructions per 32 items, 634 -> about 400 wavefronts; 160 fields of
+// packed rgb48 with its border 1,460 -> 540 us. What bounds it now is the
+// latency of the plane loads at the start of a block (two blocks of 8 warps a
+// SM: 128 registers for the window). Four blocks of 8 lines (halo 1.75x),
+// three of 10 or 14, two of 192 threads, L2 prefetches of the block 304 ahead
+// and eight loads in flight a lane instead of four all measured slower.
 #include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -43,7 +54,7 @@ __constant__ float cd_nrpal[25];     // doYNR high-pass (c_nrpal_b)
 static bool g_demod_ready[64];
 
 constexpr int kDemodThreads = 256;
-constexpr int kPad = 8;
+constexpr int kLead = 8;                 // samples a row in shared memory starts before the first active one
 constexpr int kNrHalf = 12;              // half length of the yNR filter
 // Field lines per block: 16 (a 6-line halo re-read per 16 lines), 8 with
 // yNR, whose luma lines also live in shared memory.
@@ -52,69 +63,131 @@ __host__ __device__ constexpr int demod_lines(bool ynr) { return ynr ? 8 : 16; }
 __device__ __forceinline__ int first_line(int fafl, int off) { return (fafl + 1 - off) / 2; }
 __device__ __forceinline__ int last_line(int lafl, int off) { return ((lafl - off) / 2) + 1; }
 
-__host__ __device__ __forceinline__ int demod_span(int avs, int ave) { return ((ave - (avs & ~3)) + 7) & ~7; }
+// Shared rows: samples avs - 8 .. avs + 8 n + 7 for n items, in 16-byte chunks;
+// chunk c is stored at c ^ ((c >> 3) & 1), which spreads the chunks of
+// consecutive items (2 apart) over all banks. The row length keeps the pattern
+// the same in every row.
+__host__ __device__ __forceinline__ int demod_items(int avs, int ave) { return (ave - avs + 7) / 8; }
+__host__ __device__ __forceinline__ int demod_row(int avs, int ave) { return (8 * demod_items(avs, ave) + 2 * kLead + 63) & ~63; }
+__device__ __forceinline__ int chunk_at(int c) { return c ^ ((c >> 3) & 1); }
+__device__ __forceinline__ int float_at(int i) { return 4 * chunk_at(i >> 2) + (i & 3); }
 
 // 4fsc reference carrier at sample x: sine {0, 1, 0, -1}, cosine {1, 0, -1, 0}.
 __device__ __forceinline__ float carrier_sin(int x) { return (x & 1) ? ((x & 2) ? -1.f : 1.f) : 0.f; }
 __device__ __forceinline__ float carrier_cos(int x) { return (x & 1) ? 0.f : ((x & 2) ? -1.f : 1.f); }
 
-// The 2D FIR of one work item: PU, QU, PV, QV (and PY, QY from the luma
-// taps when WITH_Y) for 8 samples from the 4 vertical combinations v.
-// Taps b = 0..7 of the launch's filter (a filter of size 6, at PAL-M's
-// sample rate, has zero taps at b = 7). swap: the reference's PAL-M tables
-// (sine and cosine exchanged at fieldHeight 263, palcolour.cpp:158-173) make
-// each P sum the other table's Q sum and vice versa: (PU, QU, PV, QV)
-// become (QV, PV, QU, PU); the luma resynthesis is unchanged.
-template <bool WITH_Y>
-__device__ __forceinline__ void item_fir(const DemodParams &P, const float (&v)[4][22], float (&PU)[8], float (&QU)[8],
-                                         float (&PV)[8], float (&QV)[8], float (&PY)[8], float (&QY)[8])
+// The vertical combinations (palcolour.cpp:557-567 without the carrier) of 22
+// columns, sample s of the item at column s + 7:
+//   v0 = c0, v1 = -c(-2) - c(+2), v2 = c(-1) - c(+1), v3 = -c(-3) + c(+3)
+// as the pairs (v0, v2) and (v1, v3) for the f32x2 instructions.
+struct Window {
+    float2 v02[22], v13[22];
+};
+
+// Chunks N0 .. N1 - 1 of the six an item's window spans. ch: the row three
+// lines above the item's; the item's first chunk is 2 seg. Samples 0..3 need
+// chunks 0..4 only.
+template <int N0, int N1>
+__device__ __forceinline__ void load_window(const float *ch, int row_floats, int seg, Window &W)
 {
 #pragma unroll
-    for (int s = 0; s < 8; s++) {
-        float PA = 0.f, PB = 0.f, QA = 0.f, QB = 0.f, PYs = 0.f, QYs = 0.f;
+    for (int n = N0; n < N1; n++) {
+        const float *p = ch + 4 * chunk_at(2 * seg + n);
+        float4 r[7];
 #pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const int r = s + b + 7, l = s - b + 7;
-            float sg[4];
+        for (int k = 0; k < 7; k++) r[k] = *reinterpret_cast<const float4 *>(p + k * row_floats);
 #pragma unroll
-            for (int k = 0; k < 4; k++) sg[k] = (b & 1) ? v[k][r] - v[k][l] : v[k][r] + v[k][l];
-            const float A = __fmaf_rn(P.cfilt[b][1], sg[1], P.cfilt[b][0] * sg[0]);
-            const float B = __fmaf_rn(P.cfilt[b][3], sg[3], P.cfilt[b][2] * sg[2]);
-            float AY = 0.f;
-            if (WITH_Y) AY = __fmaf_rn(P.yfilt[b][1], sg[1], P.yfilt[b][0] * sg[0]);
-            switch ((s + b) & 3) {
-            case 1: PA += A; PB += B; if (WITH_Y) PYs += AY; break;
-            case 3: PA -= A; PB -= B; if (WITH_Y) PYs -= AY; break;
-            case 0: QA += A; QB += B; if (WITH_Y) QYs += AY; break;
-            default: QA -= A; QB -= B; if (WITH_Y) QYs -= AY; break;
-            }
+        for (int i = 0; i < 4; i++) {
+            const int q = 4 * n + i - 1;
+            if (q < 0 || q >= 22) continue;
+            auto at = [&](int k) { return i == 0 ? r[k].x : i == 1 ? r[k].y : i == 2 ? r[k].z : r[k].w; };
+            W.v02[q] = make_float2(at(3), at(2) - at(4));
+            W.v13[q] = make_float2(-at(1) - at(5), -at(0) + at(6));
         }
-        if (P.swap_carrier) {
-            PU[s] = QA + PB;
-            PV[s] = QA - PB;
-            QU[s] = PA - QB;
-            QV[s] = PA + QB;
-        } else {
-            PU[s] = PA + QB;
-            PV[s] = PA - QB;
-            QU[s] = QA - PB;
-            QV[s] = QA + PB;
-        }
-        PY[s] = PYs;
-        QY[s] = QYs;
     }
 }
 
-// Vertical combinations (palcolour.cpp:557-567 without the carrier):
-//   v0 = c0, v1 = -c(-2) - c(+2), v2 = c(-1) - c(+1), v3 = -c(-3) + c(+3)
-__device__ __forceinline__ void item_window(const float *rw, int SW, float (&v)[4][22])
+// The 2D FIR at sample s of an item: (PU, QU, PV, QV), and (PY, QY) from the
+// luma taps with WITH_Y. Taps b = 0..7 of the launch's filter (a filter of
+// size 6, at PAL-M's sample rate, has zero taps at b = 7). Each tap touches
+// either the sine or the cosine products. swap: the reference's PAL-M tables
+// (sine and cosine exchanged at fieldHeight 263, palcolour.cpp:158-173) make
+// each P sum the other table's Q sum and vice versa: (PU, QU, PV, QV)
+// become (QV, PV, QU, PU); the luma resynthesis is unchanged.
+template <int N>
+struct Num {
+    static constexpr int value = N;
+};
+struct FirOut {
+    float PU, QU, PV, QV, PY, QY;
+};
+
+template <int XO, int S, bool CHROMA, bool WITH_Y>
+__device__ __forceinline__ FirOut fir(const DemodParams &P, const Window &W)
 {
+    float2 Pab = make_float2(0.f, 0.f), Qab = Pab;   // (A, B): the v0, v1 and the v2, v3 parts
+    float PY = 0.f, QY = 0.f;
 #pragma unroll
-    for (int q = 0; q < 22; q++) {
-        v[0][q] = rw[3 * SW + q];
-        v[1][q] = -rw[1 * SW + q] - rw[5 * SW + q];
-        v[2][q] = rw[2 * SW + q] - rw[4 * SW + q];
-        v[3][q] = -rw[q] + rw[6 * SW + q];
+    for (int b = 0; b < 8; b++) {
+        const int r = S + b + 7, l = S - b + 7, phase = (S + XO + b) & 3;
+        float2 s02, s13;
+        if (CHROMA) {
+            s02 = (b & 1) ? sub2(W.v02[r], W.v02[l]) : add2(W.v02[r], W.v02[l]);
+            s13 = (b & 1) ? sub2(W.v13[r], W.v13[l]) : add2(W.v13[r], W.v13[l]);
+            const float2 ab = __ffma2_rn(make_float2(P.cfilt[b][2], P.cfilt[b][3]), s13,
+                                         __fmul2_rn(make_float2(P.cfilt[b][0], P.cfilt[b][1]), s02));
+            if (phase == 1) Pab = add2(Pab, ab);
+            if (phase == 3) Pab = sub2(Pab, ab);
+            if (phase == 0) Qab = add2(Qab, ab);
+            if (phase == 2) Qab = sub2(Qab, ab);
+        } else {
+            s02.x = (b & 1) ? W.v02[r].x - W.v02[l].x : W.v02[r].x + W.v02[l].x;
+            s13.x = (b & 1) ? W.v13[r].x - W.v13[l].x : W.v13[r].x + W.v13[l].x;
+        }
+        if (WITH_Y) {
+            const float y = __fmaf_rn(P.yfilt[b][1], s13.x, P.yfilt[b][0] * s02.x);
+            if (phase == 1) PY += y;
+            if (phase == 3) PY -= y;
+            if (phase == 0) QY += y;
+            if (phase == 2) QY -= y;
+        }
+    }
+    FirOut o;
+    o.PY = PY;
+    o.QY = QY;
+    if (P.swap_carrier) {
+        o.PU = Qab.x + Pab.y;
+        o.PV = Qab.x - Pab.y;
+        o.QU = Pab.x - Qab.y;
+        o.QV = Pab.x + Qab.y;
+    } else {
+        o.PU = Pab.x + Qab.y;
+        o.PV = Pab.x - Qab.y;
+        o.QU = Qab.x - Pab.y;
+        o.QV = Qab.x + Pab.y;
+    }
+    return o;
+}
+
+// 4 samples of a composite row, at any 2-byte boundary, as floats: three
+// aligned words and a funnel shift, the bits 2^23 + a, less `off` + 2^23
+// (exact). first: the first sample's index within the field.
+__device__ __forceinline__ void samples4(const uint16_t *field, int first, int field_len, float off, float (&v)[4])
+{
+    const float bias = 8388608.0f + off;
+    if (first >= 1 && first + 6 <= field_len) {
+        const uintptr_t pa = reinterpret_cast<uintptr_t>(field + first);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
+        const unsigned sh = (unsigned)(pa & 2) * 8u;
+        const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
+        const uint32_t a = __funnelshift_r(w0, w1, sh), b = __funnelshift_r(w1, w2, sh);
+        v[0] = __uint_as_float(__byte_perm(a, 0x4B000000u, 0x7610)) - bias;
+        v[1] = __uint_as_float(__byte_perm(a, 0x4B000000u, 0x7632)) - bias;
+        v[2] = __uint_as_float(__byte_perm(b, 0x4B000000u, 0x7610)) - bias;
+        v[3] = __uint_as_float(__byte_perm(b, 0x4B000000u, 0x7632)) - bias;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = (float)__ldg(field + min(max(first + i, 0), field_len - 1)) - off;
     }
 }
 
@@ -126,113 +199,122 @@ __device__ __forceinline__ void item_window(const float *rw, int SW, float (&v)[
 // (p - n) + e, below one in magnitude, rounded. zero is an integer, so
 // zero + n + Floor(r + 1/2) is H.273's Round of the whole sum wherever that
 // sum is non-negative; below zero both clamp to the bound lo >= 0. Returns
-// the clamped code as a float (exact).
+// the clamped code plus 2^23, exact, so the code is the low half of its bits
+// (conversions run on a quarter-rate pipe; rounding to the nearest integer is
+// the addition of 3 * 2^22, exact for |p| below 2^22 -- beyond the code's range
+// by a factor of 64 -- and clamped to it).
+constexpr float kCode0 = 8388608.0f;
 __device__ __forceinline__ float code_of(float zero, float v_hi, float v_lo, float k_hi, float k_lo, float lo, float hi)
 {
-    const float p = v_hi * k_hi;
+    const float p = fminf(fmaxf(v_hi * k_hi, -4194304.0f), 4194303.0f);
     const float e = __fmaf_rn(v_hi, k_hi, -p) + __fmaf_rn(v_hi, k_lo, v_lo * k_hi);
-    const float n = rintf(p);
+    const float n = __fsub_rn(__fadd_rn(p, 12582912.0f), 12582912.0f);
     const float r = (p - n) + e;   // p - n is exact
-    return fminf(fmaxf(zero + n + floorf(r + 0.5f), lo), hi);
+    return fminf(fmaxf((kCode0 + zero) + n + floorf(r + 0.5f), kCode0 + lo), kCode0 + hi);
+}
+__device__ __forceinline__ uint32_t code_pair(float a, float b)
+{
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x5410);
 }
 
-// Pack one sample in the output format (OutputWriter::convertLine,
-// convertToFloat, convertToFloatRGB; output_writer.cpp:402-486, 670-779).
-// Luma arrives as Y - black = yb.hi + yb.lo (exact for the Transform kinds:
-// an integer composite sample minus the FP32 chroma, by two-sum).
-__device__ __forceinline__ void pack_sample(const DemodParams &P, void *out, long long frame, long long pix, df yb,
-                                            float U, float V)
+// One sample's outputs in the units its format stores: the codes of code_of
+// (yuv444p16, gray16), 0..65535 before truncation (rgb48) or the float value.
+// OutputWriter::convertLine, convertToFloat, convertToFloatRGB
+// (output_writer.cpp:402-486, 670-779). Luma arrives as Y - black = yb.hi +
+// yb.lo (exact for the Transform kinds: an integer composite sample minus the
+// FP32 chroma, by two-sum).
+__device__ __forceinline__ float luma_value(const DemodParams &P, int format, df yb)
 {
-    const long long plane = (long long)P.out_w * P.out_h;
-    const long long e = frame * P.out_frame_stride + pix;
-    const float ey = (yb.hi + yb.lo) * P.ey_scale;
-    switch (P.format) {
-    case 0: {
-        uint16_t *o = (uint16_t *)out;
-        o[e] = (uint16_t)code_of(16.0f * 256.0f, yb.hi, yb.lo, P.qy_hi, P.qy_lo, P.y_lo, P.y_hi);
-        o[e + plane] = (uint16_t)code_of(128.0f * 256.0f, U, 0.f, P.qcb_hi, P.qcb_lo, P.c_lo, P.c_hi);
-        o[e + 2 * plane] = (uint16_t)code_of(128.0f * 256.0f, V, 0.f, P.qcr_hi, P.qcr_lo, P.c_lo, P.c_hi);
-        break;
-    }
-    case 1: {
-        float *o = (float *)out;
-        o[e] = fminf(fmaxf(ey, P.y_lo), P.y_hi);
-        o[e + plane] = fminf(fmaxf(U * P.ecb_scale, P.c_lo), P.c_hi);
-        o[e + 2 * plane] = fminf(fmaxf(V * P.ecr_scale, P.c_lo), P.c_hi);
-        break;
-    }
-    case 2: {   // interleaved R'G'B' 0..65535, truncating stores
-        uint16_t *o = (uint16_t *)out + frame * P.out_frame_stride + 3 * pix;
-        const float rY = fminf(fmaxf((yb.hi + yb.lo) * P.rgb_y_scale, 0.f), 65535.f);
-        const float rU = U * P.rgb_uv_scale, rV = V * P.rgb_uv_scale;
-        o[0] = (uint16_t)__float2uint_rz(fminf(fmaxf(__fmaf_rn(P.r_from_v, rV, rY), 0.f), 65535.f));
-        o[1] = (uint16_t)__float2uint_rz(
-            fminf(fmaxf(__fmaf_rn(P.g_from_v, rV, __fmaf_rn(P.g_from_u, rU, rY)), 0.f), 65535.f));
-        o[2] = (uint16_t)__float2uint_rz(fminf(fmaxf(__fmaf_rn(P.b_from_u, rU, rY), 0.f), 65535.f));
-        break;
-    }
-    case 3: {
-        float *o = (float *)out;
-        const float rU = U * P.rgb_uv_scale, rV = V * P.rgb_uv_scale;
-        o[e] = fminf(fmaxf(__fmaf_rn(P.r_from_v, rV, ey), P.r_lo), P.r_hi);
-        o[e + plane] = fminf(fmaxf(__fmaf_rn(P.g_from_v, rV, __fmaf_rn(P.g_from_u, rU, ey)), P.g_lo), P.g_hi);
-        o[e + 2 * plane] = fminf(fmaxf(__fmaf_rn(P.b_from_u, rU, ey), P.b_lo), P.b_hi);
-        break;
-    }
-    case 4:
-        ((uint16_t *)out)[e] = (uint16_t)code_of(16.0f * 256.0f, yb.hi, yb.lo, P.qy_hi, P.qy_lo, P.y_lo, P.y_hi);
-        break;
-    default:
-        ((float *)out)[e] = fminf(fmaxf(ey, P.y_lo), P.y_hi);
-        break;
-    }
+    if (format == 0 || format == 4)
+        return code_of(16.0f * 256.0f, yb.hi, yb.lo, P.qy_hi, P.qy_lo, P.y_lo, P.y_hi);
+    return fminf(fmaxf((yb.hi + yb.lo) * P.ey_scale, P.y_lo), P.y_hi);
 }
-
-// The three outputs of one sample in the units yuv444p16 (the quantised
-// code, exact in FP32) or yuv444ps (E'Y, E'Cb, E'Cr) stores -- the
-// arithmetic of pack_sample's cases 0 and 1.
-__device__ __forceinline__ void yuv_values(const DemodParams &P, df yb, float U, float V, float &o0, float &o1,
-                                           float &o2)
+__device__ __forceinline__ void chroma_values(const DemodParams &P, int format, float U, float V, float &o1, float &o2)
 {
-    if (P.format == 0) {
-        o0 = code_of(16.0f * 256.0f, yb.hi, yb.lo, P.qy_hi, P.qy_lo, P.y_lo, P.y_hi);
+    if (format == 0) {
         o1 = code_of(128.0f * 256.0f, U, 0.f, P.qcb_hi, P.qcb_lo, P.c_lo, P.c_hi);
         o2 = code_of(128.0f * 256.0f, V, 0.f, P.qcr_hi, P.qcr_lo, P.c_lo, P.c_hi);
     } else {
-        o0 = fminf(fmaxf((yb.hi + yb.lo) * P.ey_scale, P.y_lo), P.y_hi);
         o1 = fminf(fmaxf(U * P.ecb_scale, P.c_lo), P.c_hi);
         o2 = fminf(fmaxf(V * P.ecr_scale, P.c_lo), P.c_hi);
     }
 }
-
-__device__ __forceinline__ void store_yuv(const DemodParams &P, void *out, long long e, long long plane, float o0,
-                                          float o1, float o2)
+__device__ __forceinline__ void rgb_values(const DemodParams &P, int format, df yb, float U, float V, float &o0,
+                                           float &o1, float &o2)
 {
-    if (P.format == 0) {
-        uint16_t *o = (uint16_t *)out;
-        o[e] = (uint16_t)o0;
-        o[e + plane] = (uint16_t)o1;
-        o[e + 2 * plane] = (uint16_t)o2;
+    const float rU = U * P.rgb_uv_scale, rV = V * P.rgb_uv_scale;
+    if (format == 2) {
+        const float rY = fminf(fmaxf((yb.hi + yb.lo) * P.rgb_y_scale, 0.f), 65535.f);
+        o0 = fminf(fmaxf(__fmaf_rn(P.r_from_v, rV, rY), 0.f), 65535.f);
+        o1 = fminf(fmaxf(__fmaf_rn(P.g_from_v, rV, __fmaf_rn(P.g_from_u, rU, rY)), 0.f), 65535.f);
+        o2 = fminf(fmaxf(__fmaf_rn(P.b_from_u, rU, rY), 0.f), 65535.f);
     } else {
-        float *o = (float *)out;
-        o[e] = o0;
-        o[e + plane] = o1;
-        o[e + 2 * plane] = o2;
+        const float ey = (yb.hi + yb.lo) * P.ey_scale;
+        o0 = fminf(fmaxf(__fmaf_rn(P.r_from_v, rV, ey), P.r_lo), P.r_hi);
+        o1 = fminf(fmaxf(__fmaf_rn(P.g_from_v, rV, __fmaf_rn(P.g_from_u, rU, ey)), P.g_lo), P.g_hi);
+        o2 = fminf(fmaxf(__fmaf_rn(P.b_from_u, rU, ey), P.b_lo), P.b_hi);
     }
 }
 
-// 8 consecutive outputs of one plane at element e (a multiple of 4): two
-// 8-byte stores (yuv444p16) or two 16-byte stores (yuv444ps)
-__device__ __forceinline__ void store8(const DemodParams &P, void *out, long long e, const float (&a)[8])
+// 4 consecutive outputs of one plane at element e, `n` of them inside the
+// picture; align: the elements by which every such e is aligned (4, 2 or 1).
+__device__ __forceinline__ void store4(bool wide, void *out, long long e, int n, int align, const float (&a)[4])
 {
-    if (P.format == 0) {
-        uint2 *o = reinterpret_cast<uint2 *>((uint16_t *)out + e);
-        o[0] = make_uint2((uint32_t)a[0] | ((uint32_t)a[1] << 16), (uint32_t)a[2] | ((uint32_t)a[3] << 16));
-        o[1] = make_uint2((uint32_t)a[4] | ((uint32_t)a[5] << 16), (uint32_t)a[6] | ((uint32_t)a[7] << 16));
+    if (wide) {   // FP32 planes
+        float *o = (float *)out + e;
+        if (n == 4 && align == 4) {
+            *reinterpret_cast<float4 *>(o) = make_float4(a[0], a[1], a[2], a[3]);
+        } else if (n == 4 && align == 2) {
+            reinterpret_cast<float2 *>(o)[0] = make_float2(a[0], a[1]);
+            reinterpret_cast<float2 *>(o)[1] = make_float2(a[2], a[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i < n) o[i] = a[i];
+        }
     } else {
-        float4 *o = reinterpret_cast<float4 *>((float *)out + e);
-        o[0] = make_float4(a[0], a[1], a[2], a[3]);
-        o[1] = make_float4(a[4], a[5], a[6], a[7]);
+        uint16_t *o = (uint16_t *)out + e;
+        const uint32_t p0 = code_pair(a[0], a[1]), p1 = code_pair(a[2], a[3]);
+        if (n == 4 && align == 4) {
+            *reinterpret_cast<uint2 *>(o) = make_uint2(p0, p1);
+        } else if (n == 4 && align == 2) {
+            reinterpret_cast<uint32_t *>(o)[0] = p0;
+            reinterpret_cast<uint32_t *>(o)[1] = p1;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i < n) o[i] = (uint16_t)__float_as_uint(a[i]);
+        }
+    }
+}
+
+// 4 pixels of interleaved R'G'B' (truncating) at pixel pix, the same rules
+__device__ __forceinline__ void store_rgb48(void *out, long long e, int n, int align, const float (&r)[4],
+                                            const float (&g)[4], const float (&b)[4])
+{
+    uint16_t *o = (uint16_t *)out + e;
+    uint32_t c[12];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        c[3 * i] = __float2uint_rz(r[i]);
+        c[3 * i + 1] = __float2uint_rz(g[i]);
+        c[3 * i + 2] = __float2uint_rz(b[i]);
+    }
+    if (n == 4 && align >= 2) {
+        uint32_t w[6];
+#pragma unroll
+        for (int i = 0; i < 6; i++) w[i] = c[2 * i] | (c[2 * i + 1] << 16);
+        if (align == 4) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) reinterpret_cast<uint2 *>(o)[i] = make_uint2(w[2 * i], w[2 * i + 1]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 6; i++) reinterpret_cast<uint32_t *>(o)[i] = w[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 12; i++)
+            if (i < 3 * n) o[i] = (uint16_t)c[i];
     }
 }
 
@@ -268,30 +350,33 @@ __device__ __forceinline__ df df_div_f(float a, df d)
 
 __device__ __forceinline__ float df_round(df v) { return __fadd_rn(v.hi, v.lo); }
 
-template <bool COMPOSITE, bool YNR>
+// FMT: the output format as a constant (yuv444p16 0, yuv444ps 1), or -1: the
+// launch's, any. With the format known the item loop has no branches and half
+// the code (instruction fetch stalled it).
+template <int XO, int FMT, bool COMPOSITE, bool YNR>
 __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_constant__ DemodParams P)
 {
-    constexpr int kDemodLines = demod_lines(YNR);
-    constexpr int kRows = kDemodLines + 6;   // input lines fl0-3 .. fl0+L+2
-    extern __shared__ float smem[];
-    const int nblk_per_field = (P.fh + kDemodLines - 1) / kDemodLines;   // upper bound; invalid lines skip
-    const int o = blockIdx.x / nblk_per_field;
-    const int blk = blockIdx.x % nblk_per_field;
-    if (o >= P.nout) return;
+    const int format = FMT >= 0 ? FMT : P.format;
+    extern __shared__ float4 smem4[];
+    constexpr int kMaxLines = demod_lines(YNR);
+    const int lines = P.lines;                        // field lines of a block, at most kMaxLines
+    const int o = blockIdx.x / P.blocks_per_field;
+    const int blk = blockIdx.x % P.blocks_per_field;
     const int f = P.field_begin + o;
     const int off = (f & 1) ^ P.swap;   // SourceField::getOffset
     const int fl_first = first_line(P.fafl, off);
     const int fl_last = last_line(P.lafl, off);
-    const int fl0 = fl_first + blk * kDemodLines;
+    const int fl0 = fl_first + blk * lines;
     if (fl0 >= fl_last) return;
 
-    const int base4 = P.avs & ~3;                     // absolute sample of local index 0
-    const int span = demod_span(P.avs, P.ave);        // samples covered by threads (multiple of 8)
-    const int SW = span + 2 * kPad;                   // smem row length
-    const int YW = span + 2 * kNrHalf;                // luma line length (yNR)
-    float *ch = smem;                                  // [kRows][SW] rows fl0-3 .. fl0+L+2
-    float *ys = smem + kRows * SW;                     // [kDemodLines][YW] luma before coring (yNR only)
-    __shared__ float s_bp[kDemodLines], s_bq[kDemodLines], s_vsw[kDemodLines];
+    const int cols = P.ave - P.avs;
+    const int items = demod_items(P.avs, P.ave);      // per line
+    const int SW = demod_row(P.avs, P.ave);           // floats per shared row
+    const int YW = 8 * items + 2 * kNrHalf;           // luma line length (yNR)
+    const int rows = lines + 6;                       // input lines fl0-3 .. fl0+lines+2
+    float *ch = reinterpret_cast<float *>(smem4);     // [rows][SW]
+    float *ys = ch + rows * SW;                       // [lines][YW] luma before coring (yNR only)
+    __shared__ float s_bp[kMaxLines], s_bq[kMaxLines], s_vsw[kMaxLines];
 
     // where this field's frame goes: the frame slot of the output array, or
     // (batches of captures) the frame's own pointer, absent for the black
@@ -305,87 +390,88 @@ __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_co
     }
     const uint16_t *field = field_at(P, f);
     if (field == nullptr) return;   // a black batch gap: nothing to write
-    const int cols = P.ave - P.avs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kWarps = kDemodThreads / 32;
+    const int field_len = P.fw * P.fh;
 
     // 1. input rows, zero outside the field's active lines: the summed
     //    overlap-class chroma planes (zero outside the active window, the
     //    reference's zero-initialised chroma buffer), or the composite
     //    itself for the PALcolour filter (blackLine = 0, palcolour.cpp:466-473).
-    for (int idx = threadIdx.x; idx < kRows * SW; idx += blockDim.x) ch[idx] = 0.f;
-    if (YNR)
-        for (int idx = threadIdx.x; idx < kDemodLines * YW; idx += blockDim.x) ys[idx] = 0.f;
-    __syncthreads();
-    if (COMPOSITE) {
-        for (int idx = threadIdx.x; idx < kRows * SW; idx += blockDim.x) {
-            const int r = idx / SW, c = idx % SW;
-            const int fl = fl0 - 3 + r;
-            const int x = base4 - kPad + c;
-            if (fl < fl_first || fl >= fl_last || x < 0 || x >= P.fw) continue;
-            ch[idx] = (float)field[(long long)fl * P.fw + x];
-        }
-    } else {
-        const float *part = P.partial + (long long)o * P.part_field_stride;
-        const int c4 = cols >> 2;   // float4 per row (cols is a multiple of 4 when avs is)
-        const bool vec = ((cols & 3) == 0) && ((P.part_row_stride & 3) == 0) && ((P.part_class_stride & 3) == 0) &&
-                         ((P.part_field_stride & 3) == 0);
-        if (vec) {
+    const bool vec = !COMPOSITE && ((cols | P.part_row_stride) & 3) == 0 &&
+                     ((P.part_class_stride | P.part_field_stride) & 3) == 0;
+    const int chunks = 2 * items + 4;
+    for (int r = warp; r < rows; r += kWarps) {
+        const int fl = fl0 - 3 + r;
+        float4 *dst = reinterpret_cast<float4 *>(ch + r * SW);
+        if (fl < fl_first || fl >= fl_last) {
+            for (int c = lane; c < chunks; c += 32) dst[chunk_at(c)] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else if (COMPOSITE) {
+            for (int c = lane; c < chunks; c += 32) {
+                const int x = P.avs - kLead + 4 * c;
+                float v[4];
+                samples4(field, fl * P.fw + x, field_len, 0.f, v);
+                if (x < 0 || x + 4 > P.fw)
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (x + i < 0 || x + i >= P.fw) v[i] = 0.f;
+                dst[chunk_at(c)] = make_float4(v[0], v[1], v[2], v[3]);
+            }
+        } else if (vec) {
+            const int c4 = cols >> 2;
+            const long long cs4 = P.part_class_stride >> 2;
+            const float4 *src = reinterpret_cast<const float4 *>(P.partial + (long long)o * P.part_field_stride +
+                                                                 (long long)(fl - P.fl_lo) * P.part_row_stride);
+            if (lane < 2) dst[chunk_at(lane)] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane < chunks - 2 - c4) dst[chunk_at(2 + c4 + lane)] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-            for (int idx = threadIdx.x; idx < kRows * c4; idx += blockDim.x) {
-                const int r = idx / c4, q = idx % c4;
-                const int fl = fl0 - 3 + r;
-                if (fl < fl_first || fl >= fl_last) continue;
-                const float4 *src =
-                    reinterpret_cast<const float4 *>(part + (long long)(fl - P.fl_lo) * P.part_row_stride) + q;
-                const long long cs4 = P.part_class_stride >> 2;
-                float4 a = __ldg(src), b = __ldg(src + cs4), c = __ldg(src + 2 * cs4), d = __ldg(src + 3 * cs4);
-                float *dst = ch + r * SW + kPad + (P.avs - base4) + 4 * q;
-                dst[0] = (a.x + b.x) + (c.x + d.x);
-                dst[1] = (a.y + b.y) + (c.y + d.y);
-                dst[2] = (a.z + b.z) + (c.z + d.z);
-                dst[3] = (a.w + b.w) + (c.w + d.w);
+            for (int q = lane; q < c4; q += 32) {
+                const float4 a = __ldg(src + q), b = __ldg(src + cs4 + q), c = __ldg(src + 2 * cs4 + q),
+                             d = __ldg(src + 3 * cs4 + q);
+                dst[chunk_at(2 + q)] = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y),
+                                                   (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
             }
         } else {
-            for (int idx = threadIdx.x; idx < kRows * cols; idx += blockDim.x) {
-                const int r = idx / cols, c = idx % cols;
-                const int fl = fl0 - 3 + r;
-                if (fl < fl_first || fl >= fl_last) continue;
-                const long long e = (long long)(fl - P.fl_lo) * P.part_row_stride + c;
+            const float *src = P.partial + (long long)o * P.part_field_stride +
+                               (long long)(fl - P.fl_lo) * P.part_row_stride - kLead;
+            for (int i = lane; i < 4 * chunks; i += 32) {
                 float v = 0.f;
-                for (int k = 0; k < P.nclasses; k++) v += part[(long long)k * P.part_class_stride + e];
-                ch[r * SW + kPad + (P.avs - base4) + c] = v;
+                if (i >= kLead && i < kLead + cols)
+                    for (int k = 0; k < P.nclasses; k++) v += src[(long long)k * P.part_class_stride + i];
+                ch[r * SW + float_at(i)] = v;
             }
         }
     }
+    if (YNR)
+        for (int idx = threadIdx.x; idx < lines * YW; idx += blockDim.x) ys[idx] = 0.f;
 
-    // 2. burst detection: one warp per line (detectBurst, palcolour.cpp:344-409)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int ln = warp; ln < kDemodLines; ln += kDemodThreads / 32) {
+    // 2. burst detection: one warp per line (detectBurst, palcolour.cpp:344-409).
+    //    At most 1,135 samples of at most 2^18: the sums fit 32 bits.
+    const bool gray = format >= 4;
+    if (!gray)
+    for (int ln = warp; ln < lines; ln += kWarps) {
         const int fl = fl0 + ln;
-        long long Ps = 0, Qs = 0, POs = 0, QOs = 0;
-        if (fl < fl_last) {
-            auto px = [&](int line, int i) -> int {
-                return (line < 0 || line >= P.fh) ? 0 : (int)field[(long long)line * P.fw + i];
-            };
-            for (int i = P.burst_start + lane; i < P.burst_end; i += 32) {
-                const int d = 2 * px(fl, i) - px(fl - 2, i) - px(fl + 2, i);   // 4 * ((in0 - (in3+in4)/2) / 2)
-                const int e = px(fl + 1, i) - px(fl - 1, i);                   // 2 * ((in2 - in1) / 2)
-                switch (i & 3) {
-                case 0: Qs += d; QOs += e; break;    // cosine +1
-                case 1: Ps += d; POs += e; break;    // sine +1
-                case 2: Qs -= d; QOs -= e; break;    // cosine -1
-                default: Ps -= d; POs -= e; break;   // sine -1
-                }
+        if (fl >= fl_last) continue;
+        int Ps = 0, Qs = 0, POs = 0, QOs = 0;
+        auto px = [&](int line, int i) -> int {
+            return (line < 0 || line >= P.fh) ? 0 : (int)__ldg(field + line * P.fw + i);
+        };
+        for (int i = P.burst_start + lane; i < P.burst_end; i += 32) {
+            const int d = 2 * px(fl, i) - px(fl - 2, i) - px(fl + 2, i);   // 4 * ((in0 - (in3+in4)/2) / 2)
+            const int e = px(fl + 1, i) - px(fl - 1, i);                   // 2 * ((in2 - in1) / 2)
+            switch (i & 3) {
+            case 0: Qs += d; QOs += e; break;    // cosine +1
+            case 1: Ps += d; POs += e; break;    // sine +1
+            case 2: Qs -= d; QOs -= e; break;    // cosine -1
+            default: Ps -= d; POs -= e; break;   // sine -1
             }
         }
-#pragma unroll
-        for (int h = 16; h >= 1; h >>= 1) {
-            Ps += __shfl_xor_sync(0xffffffffu, Ps, h);
-            Qs += __shfl_xor_sync(0xffffffffu, Qs, h);
-            POs += __shfl_xor_sync(0xffffffffu, POs, h);
-            QOs += __shfl_xor_sync(0xffffffffu, QOs, h);
-        }
+        Ps = __reduce_add_sync(0xffffffffu, Ps);
+        Qs = __reduce_add_sync(0xffffffffu, Qs);
+        POs = __reduce_add_sync(0xffffffffu, POs);
+        QOs = __reduce_add_sync(0xffffffffu, QOs);
         if (P.swap_carrier) {   // the PAL-M tables: the sine sums are the cosine sums and vice versa
-            const long long t0 = Ps, t1 = POs;
+            const int t0 = Ps, t1 = POs;
             Ps = Qs;
             Qs = t0;
             POs = QOs;
@@ -393,14 +479,14 @@ __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_co
         }
         if (lane == 0) {
             // bp = P/(4 len), bpo = PO/(2 len): the V-switch test scaled by (4 len)^2
-            const long long a = Ps - 2 * POs, b = Qs - 2 * QOs;
-            const bool vpos = (a * a + b * b) < 2 * (Ps * Ps + Qs * Qs);
+            const long long a = (long long)Ps - 2 * (long long)POs, b = (long long)Qs - 2 * (long long)QOs;
+            const bool vpos = (a * a + b * b) < 2 * ((long long)Ps * Ps + (long long)Qs * Qs);
             // bp / max(|(bp, bq)|, 130000/128) with bp = pn / (8 len): the
             // 8 len cancels, leaving pn / max(|(pn, qn)|, 8 len 130000/128).
             // pn, qn are integers below 2^23 (exact in FP32); the rest runs
             // in double-float (about 2^-46), so the rounded results are the
             // double computation's.
-            const float pn = (float)(Ps - 2 * QOs), qn = (float)(Qs + 2 * POs);
+            const float pn = (float)((long long)Ps - 2 * (long long)QOs), qn = (float)((long long)Qs + 2 * (long long)POs);
             const df n = burst_norm(pn, qn, 8.0f * (float)(P.burst_end - P.burst_start) * (130000.0f / 128.0f));
             const df nbp = df_div_f(pn, n), nbq = df_div_f(qn, n);
             s_bp[ln] = df_round(df_sub(df_mul_f(nbp, P.gain_cos), df_mul_f(nbq, P.gain_sin)));
@@ -410,144 +496,131 @@ __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_co
     }
     __syncthreads();
 
-    const int per_line = span / 8;
-
     // 3. yNR pre-pass: the block's luma lines (zero outside the active window)
     if (YNR) {
-        for (int item = threadIdx.x; item < kDemodLines * per_line; item += blockDim.x) {
-            const int t = item / per_line, seg = item % per_line;
+        for (int item = threadIdx.x; item < lines * items; item += blockDim.x) {
+            const int t = item / items, seg = item % items;
             const int fl = fl0 + t;
             if (fl >= fl_last) continue;
-            const int xl0 = seg * 8;
-            const uint16_t *comp = field + (long long)fl * P.fw;
-            float Yv[8];
+            float cv[8], Yv[8];
+            samples4(field, fl * P.fw + P.avs + 8 * seg, field_len, 0.f, reinterpret_cast<float(&)[4]>(cv[0]));
+            samples4(field, fl * P.fw + P.avs + 8 * seg + 4, field_len, 0.f, reinterpret_cast<float(&)[4]>(cv[4]));
             if (COMPOSITE) {
-                float v[4][22];
-                item_window(ch + t * SW + kPad + xl0 - 7, SW, v);
-                float PU[8], QU[8], PV[8], QV[8], PY[8], QY[8];
-                item_fir<true>(P, v, PU, QU, PV, QV, PY, QY);
-#pragma unroll
-                for (int s = 0; s < 8; s++) {
-                    const int x = base4 + xl0 + s;
-                    Yv[s] = (float)comp[x < P.fw ? x : P.fw - 1] -
-                            2.0f * __fmaf_rn(PY[s], carrier_sin(x), QY[s] * carrier_cos(x));
-                }
+                Window W;
+                load_window<0, 6>(ch + t * SW, SW, seg, W);
+                auto luma = [&](auto S) {
+                    constexpr int s = decltype(S)::value;
+                    const FirOut q = fir<XO, s, false, true>(P, W);
+                    Yv[s] = cv[s] - 2.0f * __fmaf_rn(q.PY, carrier_sin(s + XO), q.QY * carrier_cos(s + XO));
+                };
+                luma(Num<0>{}), luma(Num<1>{}), luma(Num<2>{}), luma(Num<3>{});
+                luma(Num<4>{}), luma(Num<5>{}), luma(Num<6>{}), luma(Num<7>{});
             } else {
 #pragma unroll
-                for (int s = 0; s < 8; s++) {
-                    const int x = base4 + xl0 + s;
-                    Yv[s] = (float)comp[x < P.fw ? x : P.fw - 1] - ch[(t + 3) * SW + kPad + xl0 + s];
-                }
+                for (int s = 0; s < 8; s++) Yv[s] = cv[s] - ch[(t + 3) * SW + float_at(kLead + 8 * seg + s)];
             }
 #pragma unroll
-            for (int s = 0; s < 8; s++) {
-                const int x = base4 + xl0 + s;
-                if (x >= P.avs && x < P.ave) ys[t * YW + kNrHalf + xl0 + s] = Yv[s];
-            }
+            for (int s = 0; s < 8; s++)
+                if (8 * seg + s < cols) ys[t * YW + kNrHalf + 8 * seg + s] = Yv[s];
         }
         __syncthreads();
     }
 
-    // 4. 2D FIR + rotation + pack; work item = (line, 8-sample segment).
-    // Sample s of an item is output pixel 8 seg + s - xoff. For yuv444p16 /
-    // yuv444ps with 4-element-aligned rows, planes and frames, a lane stores
-    // pixels 8 seg .. 8 seg + 7 with vector stores: its samples xoff..7 and
-    // (xoff = 1) the next lane's sample 0, passed by a shuffle; edges and the
-    // other formats store per sample. Every lane runs every round, so the
-    // shuffles see the whole warp.
-    const int total = kDemodLines * per_line;
-    const int xoff = P.avs - base4;
-    const int aw = P.ave - P.avs;
+    // 4. 2D FIR + rotation + pack; work item = (line, 8-sample segment), 4
+    // pixels stored at a time: vectors where the output's rows, planes and
+    // frames allow, else element by element.
+    const bool wide = format == 1 || format == 3 || format == 5;
     const long long plane = (long long)P.out_w * P.out_h;
-    const bool vout = (P.format == 0 || P.format == 1) && xoff <= 1 && ((P.out_w | P.left_pad) & 3) == 0 &&
-                      (P.out_frame_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(out_base) & 15) == 0;
-    for (int ib = 0; ib < total; ib += blockDim.x) {
-        const int item = ib + threadIdx.x;
-        const int t = item / per_line;
-        const int seg = item % per_line;
+    int align = 4;
+    {
+        const int elem = wide ? 4 : 2;
+        const uintptr_t u = reinterpret_cast<uintptr_t>(out_base);
+        const long long units = format == 2 ? P.out_frame_stride / 3 : P.out_frame_stride;
+        const long long all = P.out_w | P.left_pad | units | plane;
+        if ((all & 3) != 0 || u % (4 * elem) != 0) align = 2;
+        if ((all & 1) != 0 || u % (2 * elem) != 0) align = 1;
+    }
+    int t = threadIdx.x / items, seg = threadIdx.x % items;
+    const int dt = kDemodThreads / items, dseg = kDemodThreads % items;
+    for (int item = threadIdx.x; item < lines * items;
+         item += kDemodThreads, t += dt, seg += dseg, t += seg >= items, seg -= seg >= items ? items : 0) {
         const int fl = fl0 + t;
-        const bool live = item < total && fl < fl_last;
-        float o0[8], o1[8], o2[8];
-        long long rowpix = 0;
-        if (live) {
-            const int xl0 = seg * 8;   // local index of the first sample (absolute base4 + xl0, a multiple of 4)
-            // the composite samples luma needs, loaded before the FIR so their
-            // latency hides behind it
-            const uint16_t *comp = field + (long long)fl * P.fw;
-            float cv[8];
+        if (fl >= fl_last) break;
+        // the composite samples luma needs, less black, loaded before the FIR
+        // so their latency hides behind it
+        float cb[8];
+        if (!YNR) {
+            samples4(field, fl * P.fw + P.avs + 8 * seg, field_len, (float)P.black, reinterpret_cast<float(&)[4]>(cb[0]));
+            samples4(field, fl * P.fw + P.avs + 8 * seg + 4, field_len, (float)P.black, reinterpret_cast<float(&)[4]>(cb[4]));
+        }
+        const int orow = P.top_pad + 2 * fl + off - P.fafl;
+        const long long pix = (long long)orow * P.out_w + P.left_pad + 8 * seg;
+        const long long e0 = frame_slot * P.out_frame_stride + (format == 2 ? 3 * pix : pix);
+        // Y - black of sample s
+        auto luma = [&](int s, float v0, float PY, float QY) -> df {
+            if (YNR) {
+                // doYNR: a = sum_i b_i Y[x + 12 - i], cored to +-nr_y, subtracted
+                const float *yl = ys + t * YW + kNrHalf + 8 * seg + s;
+                float a = 0.f;
 #pragma unroll
-            for (int s = 0; s < 8; s++) {
-                const int x = base4 + xl0 + s;
-                cv[s] = (float)comp[x < P.fw ? x : P.fw - 1];
+                for (int i = 0; i < 25; i++) a = __fmaf_rn(cd_nrpal[i], yl[kNrHalf - i], a);
+                a = fminf(fmaxf(a, -P.nr_y), P.nr_y);
+                return two_sum(yl[0] - (float)P.black, -a);
             }
-            float v[4][22];
-            item_window(ch + t * SW + kPad + xl0 - 7, SW, v);
-            float PU[8], QU[8], PV[8], QV[8], PY[8], QY[8];
-            item_fir<COMPOSITE && !YNR>(P, v, PU, QU, PV, QV, PY, QY);
-
-            const float bp = s_bp[t], bq = s_bq[t], vsw = s_vsw[t];
-            const int orow = P.top_pad + 2 * fl + off - P.fafl;
-            rowpix = (long long)orow * P.out_w + P.left_pad;
+            if (COMPOSITE)
+                return two_sum(cb[s], -2.0f * __fmaf_rn(PY, carrier_sin(s + XO), QY * carrier_cos(s + XO)));
+            return two_sum(cb[s], -v0);
+        };
+        constexpr bool kLumaFir = COMPOSITE && !YNR;   // luma needs the window
+        if (gray && !kLumaFir) {
 #pragma unroll
-            for (int s = 0; s < 8; s++) {
-                const int x = base4 + xl0 + s;
-                df yb;   // Y - black
-                const float cb = cv[s] - (float)P.black;   // exact: an integer sample
-                if (YNR) {
-                    // doYNR: a = sum_i b_i Y[x + 12 - i], cored to +-nr_y, subtracted
-                    const float *yl = ys + t * YW + kNrHalf + xl0 + s;
-                    float a = 0.f;
+            for (int h = 0; h < 2; h++) {
+                const int n = min(4, cols - 8 * seg - 4 * h);
+                if (n <= 0) break;
+                float y[4];
 #pragma unroll
-                    for (int i = 0; i < 25; i++) a = __fmaf_rn(cd_nrpal[i], yl[kNrHalf - i], a);
-                    a = fminf(fmaxf(a, -P.nr_y), P.nr_y);
-                    yb = two_sum(yl[0] - (float)P.black, -a);
-                } else if (COMPOSITE) {
-                    yb = two_sum(cb, -2.0f * __fmaf_rn(PY[s], carrier_sin(x), QY[s] * carrier_cos(x)));
+                for (int i = 0; i < 4; i++)
+                    y[i] = luma_value(P, format, luma(4 * h + i, YNR ? 0.f : ch[(t + 3) * SW + float_at(kLead + 8 * seg + 4 * h + i)], 0.f, 0.f));
+                store4(wide, out_base, e0 + 4 * h, n, align, y);
+            }
+            continue;
+        }
+        Window W;
+        load_window<0, 5>(ch + t * SW, SW, seg, W);
+        const float bp = gray ? 0.f : s_bp[t], bq = gray ? 0.f : s_bq[t], vsw = gray ? 1.f : s_vsw[t];
+        auto half = [&](auto H) {
+            constexpr int h = decltype(H)::value;
+            const int n = min(4, cols - 8 * seg - 4 * h);
+            if (n <= 0) return;
+            float o0[4], o1[4], o2[4];
+            auto sample = [&](auto I) {
+                constexpr int i = decltype(I)::value, s = 4 * h + i;
+                const FirOut q = fir<XO, s, true, kLumaFir>(P, W);
+                const df yb = luma(s, W.v02[s + 7].x, q.PY, q.QY);
+                const float U = -(q.PU * bp + q.QU * bq) * 2.0f;
+                const float V = vsw * -(q.QV * bp - q.PV * bq) * 2.0f;
+                if (format == 2 || format == 3) {
+                    rgb_values(P, format, yb, U, V, o0[i], o1[i], o2[i]);
                 } else {
-                    yb = two_sum(cb, -v[0][s + 7]);
+                    o0[i] = luma_value(P, format, yb);
+                    chroma_values(P, format, U, V, o1[i], o2[i]);
                 }
-                const float U = -(PU[s] * bp + QU[s] * bq) * 2.0f;
-                const float V = vsw * -(QV[s] * bp - PV[s] * bq) * 2.0f;
-                if (vout) {
-                    yuv_values(P, yb, U, V, o0[s], o1[s], o2[s]);
-                } else if (x >= P.avs && x < P.ave) {
-                    pack_sample(P, out_base, frame_slot, rowpix + (x - P.avs), yb, U, V);
+            };
+            sample(Num<0>{}), sample(Num<1>{}), sample(Num<2>{}), sample(Num<3>{});
+            if (format == 2) {
+                store_rgb48(out_base, e0 + 12 * h, n, align, o0, o1, o2);
+            } else {
+                const long long e = e0 + 4 * h;
+                store4(wide, out_base, e, n, align, o0);
+                if (!gray) {
+                    store4(wide, out_base, e + plane, n, align, o1);
+                    store4(wide, out_base, e + 2 * plane, n, align, o2);
                 }
             }
-        }
-        if (!vout) continue;
-        const float n0 = __shfl_down_sync(0xffffffffu, o0[0], 1);
-        const float n1 = __shfl_down_sync(0xffffffffu, o1[0], 1);
-        const float n2 = __shfl_down_sync(0xffffffffu, o2[0], 1);
-        const int nitem = __shfl_down_sync(0xffffffffu, live ? item : -1, 1);
-        const bool full = live && 8 * seg + 8 <= aw &&
-                          (xoff == 0 || (lane < 31 && nitem == item + 1 && seg + 1 < per_line));
-        const bool prev_full = (__shfl_up_sync(0xffffffffu, full ? 1 : 0, 1) != 0) && lane > 0;
-        if (!live) continue;
-        const long long e0 = frame_slot * P.out_frame_stride + rowpix;
-        if (full) {
-            float a0[8], a1[8], a2[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {   // xoff is 0 or 1 here; constant indices keep o* in registers
-                a0[j] = xoff == 0 ? o0[j] : (j < 7 ? o0[j < 7 ? j + 1 : 7] : n0);
-                a1[j] = xoff == 0 ? o1[j] : (j < 7 ? o1[j < 7 ? j + 1 : 7] : n1);
-                a2[j] = xoff == 0 ? o2[j] : (j < 7 ? o2[j < 7 ? j + 1 : 7] : n2);
-            }
-            const long long e = e0 + 8 * seg;
-            store8(P, out_base, e, a0);
-            store8(P, out_base, e + plane, a1);
-            store8(P, out_base, e + 2 * plane, a2);
-        }
-        // samples no vector store covered: edges, and sample 0 unless the
-        // previous lane stored it
-#pragma unroll
-        for (int s = 0; s < 8; s++) {
-            const int p = 8 * seg + s - xoff;
-            if (p < 0 || p >= aw) continue;
-            if (full && s >= xoff) continue;
-            if (xoff == 1 && s == 0 && prev_full) continue;
-            store_yuv(P, out_base, e0 + p, plane, o0[s], o1[s], o2[s]);
-        }
+        };
+        half(Num<0>{});
+        load_window<5, 6>(ch + t * SW, SW, seg, W);
+        half(Num<1>{});
     }
 }
 
@@ -581,7 +654,8 @@ int demod_taps(double sample_rate, float (&cfilt)[8][4], float (&yfilt)[8][2])
         ydiv += 2 * (1 * yf[f][0] + 2 * yf[f][1]);
     }
     for (int f = 0; f < 8; f++) {
-        for (int i = 0; i < 4; i++) cfilt[f][i] = (float)(cf[f][i] / cdiv);
+        static const int order[4] = {0, 2, 1, 3};
+        for (int i = 0; i < 4; i++) cfilt[f][i] = (float)(cf[f][order[i]] / cdiv);
         for (int i = 0; i < 2; i++) yfilt[f][i] = (float)(yf[f][i] / ydiv);
     }
     return 0;
@@ -607,50 +681,67 @@ int demod_init_constants(int device)
     return 0;
 }
 
-size_t demod_smem_bytes(int avs, int ave, bool ynr)
+static size_t demod_smem_bytes(int avs, int ave, int lines, bool ynr)
 {
-    const int span = demod_span(avs, ave);
-    const int lines = demod_lines(ynr);
-    const size_t rows = sizeof(float) * (size_t)(lines + 6) * (span + 2 * kPad);
-    return rows + (ynr ? sizeof(float) * (size_t)lines * (span + 2 * kNrHalf) : 0);
+    const size_t rows = sizeof(float) * (size_t)(lines + 6) * demod_row(avs, ave);
+    return rows + (ynr ? sizeof(float) * (size_t)lines * (8 * demod_items(avs, ave) + 2 * kNrHalf) : 0);
 }
 
-int demod_launch(const DemodParams &P, cudaStream_t stream)
+template <int XO, int FMT, bool COMPOSITE, bool YNR>
+static int demod_start(const DemodParams &P, unsigned blocks, size_t smem, cudaStream_t stream)
 {
-    if (P.nout <= 0) return 0;
-    const bool composite = P.partial == nullptr;
-    const bool ynr = P.nr_y > 0.f;
-    const size_t smem = demod_smem_bytes(P.avs, P.ave, ynr);
-    if (smem > 110 * 1024) return -1;   // two blocks per SM
     // function attributes are per device
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return -1;
     if (!attr_set[dev]) {
-        const int lim = 110 * 1024;
-        if (cudaFuncSetAttribute(demod_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(demod_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(demod_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(demod_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) !=
-                cudaSuccess)
+        if (cudaFuncSetAttribute(demod_kernel<XO, FMT, COMPOSITE, YNR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 110 * 1024) != cudaSuccess)
             return -1;
         attr_set[dev] = true;
     }
-    const int lines = demod_lines(ynr);
-    const int nblk_per_field = (P.fh + lines - 1) / lines;
-    const dim3 grid((unsigned)(P.nout * nblk_per_field));
-    if (composite) {
-        if (ynr) demod_kernel<true, true><<<grid, kDemodThreads, smem, stream>>>(P);
-        else demod_kernel<true, false><<<grid, kDemodThreads, smem, stream>>>(P);
-    } else {
-        if (ynr) demod_kernel<false, true><<<grid, kDemodThreads, smem, stream>>>(P);
-        else demod_kernel<false, false><<<grid, kDemodThreads, smem, stream>>>(P);
-    }
+    demod_kernel<XO, FMT, COMPOSITE, YNR><<<blocks, kDemodThreads, smem, stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// The kernels with a constant format: the two Y'CbCr planar formats at the
+// carrier phases of the PAL (1) and PAL-M (0) presets, without yNR.
+template <int XO, bool COMPOSITE>
+static int demod_launch_xo(const DemodParams &P, unsigned blocks, size_t smem, bool ynr, cudaStream_t stream)
+{
+    if (ynr) return demod_start<XO, -1, COMPOSITE, true>(P, blocks, smem, stream);
+    if constexpr (XO < 2) {
+        if (P.format == 0) return demod_start<XO, 0, COMPOSITE, false>(P, blocks, smem, stream);
+        if (P.format == 1) return demod_start<XO, 1, COMPOSITE, false>(P, blocks, smem, stream);
+    }
+    return demod_start<XO, -1, COMPOSITE, false>(P, blocks, smem, stream);
+}
+
+int demod_launch(const DemodParams &launch, cudaStream_t stream)
+{
+    if (launch.nout <= 0) return 0;
+    DemodParams P = launch;
+    const bool composite = P.partial == nullptr;
+    const bool ynr = P.nr_y > 0.f;
+    // a few fields: shorter blocks, so that every SM has one
+    const int field_lines = (P.lafl - P.fafl) / 2 + 1;
+    P.lines = demod_lines(ynr);
+    while (P.lines > 4 && (long long)P.nout * ((field_lines + P.lines - 1) / P.lines) < 152) P.lines /= 2;
+    P.blocks_per_field = (field_lines + P.lines - 1) / P.lines;
+    const size_t smem = demod_smem_bytes(P.avs, P.ave, P.lines, ynr);
+    if (smem > 110 * 1024) return -1;   // two blocks per SM
+    const unsigned blocks = (unsigned)(P.nout * P.blocks_per_field);
+    auto launch_kind = [&](auto C) {
+        constexpr bool c = decltype(C)::value != 0;
+        switch (P.avs & 3) {
+        case 0: return demod_launch_xo<0, c>(P, blocks, smem, ynr, stream);
+        case 1: return demod_launch_xo<1, c>(P, blocks, smem, ynr, stream);
+        case 2: return demod_launch_xo<2, c>(P, blocks, smem, ynr, stream);
+        default: return demod_launch_xo<3, c>(P, blocks, smem, ynr, stream);
+        }
+    };
+    return composite ? launch_kind(Num<1>{}) : launch_kind(Num<0>{});
 }
 
 }  // namespace tpal

@@ -491,14 +491,21 @@ int Engine::run_demod(const uint16_t *fields, long long stride, int field_base, 
 // Black border of padded frames (OutputWriter::fillBlack, output_writer.cpp:371-400):
 // Y 16*256 and Cb/Cr 128*256 for yuv444p16, 16*256 for gray16, zero for
 // rgb48 and every float format.
-__global__ void fill_frames_kernel(uint16_t *o16, float *o32, long long frame_elems, long long plane, long long nframes,
-                                   uint16_t y, uint16_t c)
+// Only the border: the demodulator writes every active sample (one block per
+// row of a plane; interleaved R'G'B' is one plane of 3-element pixels).
+template <typename T>
+__global__ void fill_border_kernel(T *out, long long frame_elems, int planes, int w, int h, int per_pixel, int left,
+                                   int top, int aw, int ah, T first, T rest)
 {
-    const long long n = nframes * frame_elems;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        if (o16) o16[i] = (((i % frame_elems) / plane) == 0) ? y : c;
-        else o32[i] = 0.f;
-    }
+    const long long row = blockIdx.x;
+    const int y = (int)(row % h), p = (int)(row / h % planes);
+    T *o = out + row / h / planes * frame_elems + ((long long)p * h + y) * w * per_pixel;
+    const T v = p == 0 ? first : rest;
+    const bool active = y >= top && y < top + ah;
+    const int skip0 = active ? left * per_pixel : w * per_pixel, skip1 = (left + aw) * per_pixel;
+    for (int i = threadIdx.x; i < skip0; i += blockDim.x) o[i] = v;
+    if (active)
+        for (int i = skip1 + threadIdx.x; i < w * per_pixel; i += blockDim.x) o[i] = v;
 }
 
 int Engine::fill_border(void *out, int nframes, cudaStream_t s)
@@ -506,12 +513,17 @@ int Engine::fill_border(void *out, int nframes, cudaStream_t s)
     const int fmt = c_.output_format;
     const long long plane = (long long)out_w_ * out_h_;
     const long long elems = plane * (long long)format_planes(fmt);
+    const int aw = g_.active_end - g_.active_start;
+    const int ah = g_.last_active_frame_line - g_.first_active_frame_line + 1;
+    const int planes = fmt == 2 ? 1 : (int)format_planes(fmt), per_pixel = fmt == 2 ? 3 : 1;
+    const unsigned rows = (unsigned)((long long)nframes * planes * out_h_);
     if (format_elem(fmt) == sizeof(float))
-        fill_frames_kernel<<<1024, 256, 0, s>>>(nullptr, (float *)out, elems, plane, nframes, 0, 0);
-    else if (fmt == 2)
-        fill_frames_kernel<<<1024, 256, 0, s>>>((uint16_t *)out, nullptr, elems, plane, nframes, 0, 0);
+        fill_border_kernel<float><<<rows, 64, 0, s>>>((float *)out, elems, planes, out_w_, out_h_, per_pixel, left_pad_,
+                                                      top_pad_, aw, ah, 0.f, 0.f);
     else
-        fill_frames_kernel<<<1024, 256, 0, s>>>((uint16_t *)out, nullptr, elems, plane, nframes, 16 * 256, 128 * 256);
+        fill_border_kernel<uint16_t><<<rows, 64, 0, s>>>((uint16_t *)out, elems, planes, out_w_, out_h_, per_pixel,
+                                                         left_pad_, top_pad_, aw, ah, fmt == 2 ? 0 : 16 * 256,
+                                                         fmt == 2 ? 0 : 128 * 256);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : cuda_fail("fill", e);
 }

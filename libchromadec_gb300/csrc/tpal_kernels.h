@@ -116,7 +116,8 @@ struct DemodParams {
     float rgb_y_scale, rgb_uv_scale;        // rgb48: 65535/range; rgbs: 1/range
     float r_from_v, g_from_u, g_from_v, b_from_u;
     float r_lo, r_hi, g_lo, g_hi, b_lo, b_hi;   // R'G'B' clamp bounds
-    float cfilt[8][4];           // chroma FIR taps of the sample rate (PalColour::buildLookUpTables)
+    int lines, blocks_per_field; // field lines per block (set by demod_launch)
+    alignas(16) float cfilt[8][4];   // chroma FIR taps of the sample rate (PalColour::buildLookUpTables), rows 0, 2, 1, 3
     float yfilt[8][2];           // luma-extraction taps
     int swap_carrier;            // 1 at fieldHeight 263: the reference's PAL-M sine/cosine exchange
 };
