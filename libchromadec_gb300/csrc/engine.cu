@@ -586,7 +586,7 @@ int Engine::run_learned(const tpal::T3Params &P, cudaStream_t s)
     L.feat = lfeat_;
     L.z0 = P.frame_begin - 2;
     if (tpal::tp3_learned_launch(P, L, 0, s) != 0) return cuda_fail("learned features", cudaGetLastError());
-    if (const int rc = net_->forward(lfeat_, ntiles, lp_, lfb_, s); rc != 0) return rc;
+    if (const int rc = net_->forward(lfeat_, ntiles, lp_, lfb_, s, true); rc != 0) return rc;
     count_fallback_kernel<<<64, 256, 0, s>>>(lfb_, ntiles, lcount_);
     L.p = lp_;
     L.fallback = lfb_;

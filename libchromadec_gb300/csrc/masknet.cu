@@ -513,10 +513,19 @@ __global__ void mn_round_kernel(const float *master, float *used)
 //    tile's features into one of two stages.
 // All waits are bounded; a wait that runs out raises the error flag and the
 // CTA leaves after its copies and MMAs in flight have completed.
+//
+// HALF: features that repeat, f(kz + 4, ky + 16) = f(kz, ky), as every
+// spectrum of a tile does (the walk's Z stage says why). The network commutes
+// with shifts along its periodic axes, so its output repeats the same way, bit
+// for bit, and 128 of the 256 rows suffice: the two M blocks are the ky < 16
+// of two tiles. Each block has its own 18 row groups; its halo groups are its
+// own ky = 15 and ky = 0 with kz moved by 4, so nothing needs the stash. The
+// schedule is the same. 62,160 tiles: 3.80 -> 1.88 ms.
 constexpr int kEpiWarps = 8;
 constexpr int kTcThreads = 32 * (kEpiWarps + 2);
 constexpr int kGroupsA = 34;                       // 32 ky groups + one halo group on each side
-constexpr int A_BYTES = kGroupsA * 8 * 160;        // a layer's input, K up to 80
+constexpr int kGroupsH = 18;                       // HALF: 16 + 2, a tile
+constexpr int A_BYTES = 2 * kGroupsH * 8 * 160;    // a layer's input, K up to 80
 constexpr int NCOL = 3 * 80;                       // accumulator columns of one M block: (q, dz, co)
 constexpr int kSlots = 8;                          // weight-piece ring (a layer's 5 pieces stay for both blocks)
 constexpr int SLOT_BYTES = 3 * 144 * 32;           // the largest piece: three ky taps x 144 rows x K 16
@@ -524,9 +533,9 @@ constexpr int FEAT_BYTES = NV * 2;
 constexpr int kPieces = 10;                        // streamed weight pieces of one tile (layers 2 and 3)
 constexpr int W1_BYTES = 3 * NCOL * 32;            // layer 1's weights, resident
 constexpr int STASH_BYTES = 2 * 8 * 160;           // row groups 16 and 33 of the next layer's input
-constexpr int IN_BYTES = kGroupsA * 8 * 32;        // layer 1's input, K = 16
-// shared memory: layers 2 and 3's input [34 groups][8 rows][K 80] and layer
-// 1's [34][8][K 16], both canonical (apart, so a tile's input can be written
+constexpr int IN_BYTES = 2 * kGroupsH * 8 * 32;    // layer 1's input, K = 16
+// shared memory: layers 2 and 3's input [36 groups][8 rows][K 80] and layer
+// 1's [36][8][K 16] (34 used unless HALF), both canonical (apart, so a tile's input can be written
 // while the previous layers' operands are read), the ring, two feature
 // stages, the stash, the barriers
 constexpr int SM_A = 0;
@@ -534,7 +543,7 @@ constexpr int SM_IN = A_BYTES;
 constexpr int SM_W1 = SM_IN + IN_BYTES;
 constexpr int SM_SLOT = SM_W1 + W1_BYTES;
 constexpr int SM_FEAT = SM_SLOT + kSlots * SLOT_BYTES;
-constexpr int SM_STASH = SM_FEAT + 2 * FEAT_BYTES;
+constexpr int SM_STASH = SM_FEAT + 4 * FEAT_BYTES;   // two stages of up to two tiles
 constexpr int SM_BAR = SM_STASH + STASH_BYTES;
 // barriers: an M block's MMAs of a layer done (2); a release of the MMAs (5:
 // chunk q of the next layer's input written, and for layer 1 the input (0)
@@ -621,6 +630,17 @@ __device__ __forceinline__ void put_row(uint8_t *A, int KB, int ky, int kz, int 
     if (ky == 0) *reinterpret_cast<uint4 *>(base + (kGroupsA - 1) * grp) = v;
 }
 
+// The same for HALF's tile b: group 18 b + ky + 1, and the halo groups at
+// ky = -1 and 16, which repeat ky = 15 and 0 with kz moved by 4.
+__device__ __forceinline__ void put_row_half(uint8_t *A, int KB, int b, int ky, int kz, int c, uint4 v)
+{
+    const int grp = 8 * KB;
+    uint8_t *base = A + b * kGroupsH * grp + c * 128;
+    *reinterpret_cast<uint4 *>(base + (ky + 1) * grp + kz * 16) = v;
+    if (ky == 15) *reinterpret_cast<uint4 *>(base + (kz ^ 4) * 16) = v;
+    if (ky == 0) *reinterpret_cast<uint4 *>(base + (kGroupsH - 1) * grp + (kz ^ 4) * 16) = v;
+}
+
 // OR of a predicate over the epilogue's 256 threads (named barrier 1).
 __device__ __forceinline__ bool epi_or(bool v)
 {
@@ -679,6 +699,7 @@ __device__ __forceinline__ void mma_band_any(int ks, uint32_t d, uint64_t ab, ui
 // The MMA warp's thread. Per tile and layer: block 0's MMAs (each chunk once
 // released), then block 1's with the same weight pieces, whose slots are then
 // freed.
+template <bool HALF>
 __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, long long step, long long ntiles)
 {
     using namespace tpal::tc;
@@ -686,10 +707,11 @@ __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, l
              *sfree = S.bars + B_SFREE;
     // operand descriptors at the bases: A with 8-row groups 256 bytes apart
     // (layer 1) or 1280 (layers 2 and 3), the weight slots 256; block 1's A
-    // starts 16 row groups in
+    // starts 16 row groups in (HALF: the second tile's 18)
+    constexpr int kBlock1 = HALF ? kGroupsH : 16;
     const uint64_t a1 = sdesc(smem_addr(S.in), 256), a2 = sdesc(smem_addr(S.A), 1280),
                    b0 = sdesc(smem_addr(S.slots), 256);
-    const uint64_t a1b[2] = {a1, desc_at(a1, 16 * 256)}, a2b[2] = {a2, desc_at(a2, 16 * 1280)};
+    const uint64_t a1b[2] = {a1, desc_at(a1, kBlock1 * 256)}, a2b[2] = {a2, desc_at(a2, kBlock1 * 1280)};
     uint32_t rbits = 0;   // parity of each release barrier's next phase
     long long sc = 0;     // weight pieces taken
     bool ok = true;
@@ -759,8 +781,9 @@ __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, l
 
 // The copy warp's thread: weight pieces through the ring, features of the
 // next tile into the other stage.
+template <bool HALF>
 __device__ bool tc_copy_role(const TcShared &S, const uint8_t *img, const uint16_t *feat, long long first,
-                             long long step, long long ntiles)
+                             long long step, long long ntiles, long long count)
 {
     using namespace tpal::tc;
     uint64_t *sfull = S.bars + B_SFULL, *sfree = S.bars + B_SFREE, *ffull = S.bars + B_FFULL,
@@ -772,8 +795,10 @@ __device__ bool tc_copy_role(const TcShared &S, const uint8_t *img, const uint16
         const int b = (int)(js & 1);
         const long long use = js >> 1;   // earlier fills of this stage
         if (use >= 1 && !bar_wait(ffree + b, (uint32_t)((use - 1) & 1))) return false;
-        bar_arrive_expect_tx(ffull + b, FEAT_BYTES);
-        bulk_g2s(S.stage + b * FEAT_BYTES, feat + tile * NV, FEAT_BYTES, ffull + b);
+        // HALF: the pair's tiles 2 tile and, unless it is past the last, 2 tile + 1
+        const uint32_t bytes = HALF && 2 * tile + 1 < count ? 2 * FEAT_BYTES : FEAT_BYTES;
+        bar_arrive_expect_tx(ffull + b, bytes);
+        bulk_g2s(S.stage + b * 2 * FEAT_BYTES, feat + (HALF ? 2 : 1) * tile * NV, bytes, ffull + b);
         js++;
         return true;
     };
@@ -851,9 +876,10 @@ __device__ __forceinline__ void combine_block(const uint32_t (&d)[48], int lane,
                 __shfl_sync(0xffffffffu, __uint_as_float(d[32 + co]), lp);
 }
 
-template <bool TRAIN>
+// HALF: `tile` below counts pairs of tiles, M block b is tile 2 tile + b.
+template <bool TRAIN, bool HALF>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    mn_tc_forward_kernel(const uint8_t *img, const float *params, const uint16_t *feat, long long ntiles,
+    mn_tc_forward_kernel(const uint8_t *img, const float *params, const uint16_t *feat, long long count,
                          float conf_limit, float *p_out, uint8_t *fallback, __nv_bfloat16 *a1g, __nv_bfloat16 *a2g,
                          __nv_bfloat16 *a3g, int *err)
 {
@@ -870,7 +896,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint8_t *stash = smem + SM_STASH;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + SM_TSLOT);
     __shared__ float s_par[4 * NC + 1];   // b1, b2, b3, wh, bh
-    __shared__ float red[2][kEpiWarps];
+    __shared__ float red[2][2][kEpiWarps];   // [block, HALF][parity of the tile][warp]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     for (int i = t; i < 4 * NC + 1; i += kTcThreads) {
         const int off[5] = {OFF_B1, OFF_B2, OFF_B3, OFF_WH, OFF_BH};
@@ -888,13 +914,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
+    static_assert(!(TRAIN && HALF), "training takes any features");
+    const long long ntiles = HALF ? (count + 1) / 2 : count;
     const long long first = blockIdx.x, step = gridDim.x;
     bool ok = true;
     if (warp == kEpiWarps) {
-        if (lane == 0) ok = tc_mma_role(S, tmem, first, step, ntiles);
+        if (lane == 0) ok = tc_mma_role<HALF>(S, tmem, first, step, ntiles);
         __syncwarp();
     } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) ok = tc_copy_role(S, img, feat, first, step, ntiles);
+        if (lane == 0) ok = tc_copy_role<HALF>(S, img, feat, first, step, ntiles, count);
         __syncwarp();
     } else {
         uint64_t *full = S.bars + B_FULL, *ready = S.bars + B_READY, *ffull = S.bars + B_FFULL,
@@ -909,16 +937,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // thread): row r = (ky, kz), k = 2 q + c (c = 0: the bin, 1: its
         // mirror), zero-padded to 16. Every epilogue warp releases the stage
         // and the first layer's block-0 MMAs.
-        auto write_input = [&]() {
+        auto write_input = [&](bool both) {
             const int b = (int)(js & 1);
             bool done = true;
             if (h == 1) {
                 done = bar_wait(ffull + b, (fbits >> b) & 1);
                 if (done) {
                     fbits ^= 1u << b;
-                    const __nv_bfloat16 *f = reinterpret_cast<const __nv_bfloat16 *>(S.stage + b * FEAT_BYTES);
+                    const __nv_bfloat16 *f0 = reinterpret_cast<const __nv_bfloat16 *>(S.stage + b * 2 * FEAT_BYTES);
                     for (int r = t - 128; r < 256; r += 128) {
-                        const int ky = r >> 3, rz = r & 7;
+                        // HALF: row r of block r >> 7; a pair without a second tile runs its first twice
+                        const int ky = HALF ? (r >> 3) & 15 : r >> 3, rz = r & 7;
+                        const __nv_bfloat16 *f = HALF && both && r >= 128 ? f0 + NV : f0;
                         __align__(16) __nv_bfloat16 v[16];
 #pragma unroll
                         for (int q = 0; q < NQ; q++) {
@@ -927,8 +957,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         }
 #pragma unroll
                         for (int k = 10; k < 16; k++) v[k] = __float2bfloat16_rn(0.f);
-                        put_row(S.in, 32, ky, rz, 0, reinterpret_cast<const uint4 *>(v)[0]);
-                        put_row(S.in, 32, ky, rz, 1, reinterpret_cast<const uint4 *>(v)[1]);
+#pragma unroll
+                        for (int c = 0; c < 2; c++) {
+                            const uint4 u = reinterpret_cast<const uint4 *>(v)[c];
+                            if (HALF) put_row_half(S.in, 32, r >> 7, ky, rz, c, u);
+                            else put_row(S.in, 32, ky, rz, c, u);
+                        }
                     }
                     fence_async_smem();
                 }
@@ -942,13 +976,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             return done;
         };
         if (first < ntiles) {
-            bad = !write_input();
+            bad = !write_input(2 * first + 1 < count);
             // block 1's columns are free for the first tile
             if (lane == 0) bar_arrive(ready + 1);
         }
         long long it = 0;
         for (long long tile = first; tile < ntiles; tile += step, it++) {
-            float conf = 0.f;
+            float conf = 0.f, conf1 = 0.f;   // HALF: block 0's tile, block 1's
             const bool more = tile + step < ntiles;
             for (int L = 0; L < 3; L++) {
                 for (int b = 0; b < 2; b++) {
@@ -960,7 +994,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     pfull ^= 1u << b;
                     fence_after();
                     const int erow = b * 128 + qd * 32 + lane;   // the row: ky = erow >> 3, kz
-                    const int ky = erow >> 3;
+                    const int ky = HALF ? (erow >> 3) & 15 : erow >> 3;
                     if (L < 2) {
                         const uint32_t tl = tq + b * 256 + h * 8;
                         float bias[8];
@@ -981,7 +1015,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 o[c] = __float2bfloat16_rn(fmaxf(y[c] + bias[c], 0.f));
                             const uint4 ov = *reinterpret_cast<const uint4 *>(o);
                             const int ch = 2 * q + h;   // the 16-byte chunk of the input row
-                            if (b == 0) {
+                            if (HALF) {
+                                put_row_half(S.A, 160, b, ky, kz, ch, ov);
+                            } else if (b == 0) {
                                 // groups 16 (ky = 15) and 33 (the halo copy of
                                 // ky = 0) are still read by block 1's MMAs
                                 if (ky == 15)
@@ -1051,8 +1087,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 zh = __fmaf_rn(a, s_par[3 * NC + co], zh);
                             }
                             const float p = 1.0f / (1.0f + expf(-zh));
-                            p_out[tile * NV + vox] = p;
-                            conf += fabsf(p - 0.5f);
+                            if (HALF) {
+                                if (2 * tile + b < count) {
+                                    float *po = p_out + (2 * tile + b) * NV;
+                                    po[vox] = p;
+                                    po[(q * 8 + (kz ^ 4)) * 32 + ky + 16] = p;
+                                }
+                                (b ? conf1 : conf) += 2.f * fabsf(p - 0.5f);
+                            } else {
+                                p_out[tile * NV + vox] = p;
+                                conf += fabsf(p - 0.5f);
+                            }
                         };
                         uint32_t ba[48], bb[48];
                         if (h == 0) {
@@ -1074,7 +1119,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         __syncwarp();
                         if (more) {
                             if (b == 0) {
-                                if (!write_input()) bad = true;
+                                if (!write_input(2 * (tile + step) + 1 < count)) bad = true;
                             } else if (lane == 0) {
                                 bar_arrive(ready + 1);
                             }
@@ -1084,17 +1129,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
             // the tile's confidence; a failure anywhere stops every epilogue warp here
 #pragma unroll
-            for (int hh = 16; hh >= 1; hh >>= 1) conf += __shfl_xor_sync(0xffffffffu, conf, hh);
-            if (lane == 0) red[it & 1][warp] = conf;
+            for (int hh = 16; hh >= 1; hh >>= 1) {
+                conf += __shfl_xor_sync(0xffffffffu, conf, hh);
+                if (HALF) conf1 += __shfl_xor_sync(0xffffffffu, conf1, hh);
+            }
+            if (lane == 0) {
+                red[0][it & 1][warp] = conf;
+                if (HALF) red[1][it & 1][warp] = conf1;
+            }
             if (epi_or(bad || *S.abort_flag != 0)) {
                 bad = true;
                 break;
             }
-            if (t == 0 && fallback != nullptr) {
+            if (t < (HALF ? 2 : 1) && fallback != nullptr) {
                 float sum = 0.f;
 #pragma unroll
-                for (int w = 0; w < kEpiWarps; w++) sum += red[it & 1][w];
-                fallback[tile] = (sum * (1.0f / NV) < conf_limit) ? 1 : 0;
+                for (int w = 0; w < kEpiWarps; w++) sum += red[t][it & 1][w];
+                const long long at = HALF ? 2 * tile + t : tile;
+                if (at < count) fallback[at] = (sum * (1.0f / NV) < conf_limit) ? 1 : 0;
             }
         }
         if (bad) *S.abort_flag = 1;
@@ -1155,8 +1207,9 @@ int MaskNet::init()
         if (cudaFuncSetAttribute(mn::mn_forward_kernel<false>, a, (int)mn::kFwdSmem) != cudaSuccess ||
             cudaFuncSetAttribute(mn::mn_forward_kernel<true>, a, (int)mn::kFwdSmem) != cudaSuccess ||
             cudaFuncSetAttribute(mn::mn_backward_kernel, a, (int)mn::kBwdSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false>, a, mn::kTcSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<true>, a, mn::kTcSmem) != cudaSuccess)
+            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false, false>, a, mn::kTcSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false, true>, a, mn::kTcSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<true, false>, a, mn::kTcSmem) != cudaSuccess)
             return mn_cuda("cudaFuncSetAttribute", cudaGetLastError());
         attr[dev] = true;
     }
@@ -1201,15 +1254,20 @@ int MaskNet::get_weights(float *host, size_t n) const
     return e == cudaSuccess ? 0 : mn_cuda("cudaMemcpy", e);
 }
 
-int MaskNet::forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8_t *d_fallback, cudaStream_t s) const
+int MaskNet::forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8_t *d_fallback, cudaStream_t s,
+                     bool repeating) const
 {
     if (ntiles <= 0) return 0;
     if (d_feat == nullptr || d_p == nullptr) return mn_fail("forward: null buffer");
     if (tc_ && reinterpret_cast<uintptr_t>(d_feat) % 16 != 0)
         return mn_fail("forward: the feature buffer must be 16-byte aligned");
     const unsigned blocks = (unsigned)std::min<long long>(ntiles, (long long)grid_ * 1);
-    if (tc_)
-        mn::mn_tc_forward_kernel<false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
+    if (tc_ && repeating)
+        mn::mn_tc_forward_kernel<false, true><<<(unsigned)std::min<long long>((ntiles + 1) / 2, grid_), mn::kTcThreads,
+                                                mn::kTcSmem, s>>>(img_, used_, d_feat, ntiles, conf_limit_, d_p,
+                                                                  d_fallback, nullptr, nullptr, nullptr, err_);
+    else if (tc_)
+        mn::mn_tc_forward_kernel<false, false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
             img_, used_, d_feat, ntiles, conf_limit_, d_p, d_fallback, nullptr, nullptr, nullptr, err_);
     else
         mn::mn_forward_kernel<false><<<blocks, mn::kThreads, mn::kFwdSmem, s>>>(used_, d_feat, ntiles, conf_limit_,
@@ -1249,7 +1307,7 @@ int MaskNet::train_step(const uint16_t *d_feat, const float2 *d_ac, long long nt
     const unsigned blocks = (unsigned)std::min<long long>(ntiles, grid_);
     cudaMemsetAsync(scal_, 0, 2 * sizeof(double), s);
     if (tc_)
-        mn::mn_tc_forward_kernel<true><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
+        mn::mn_tc_forward_kernel<true, false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
             img_, used_, d_feat, ntiles, conf_limit_, p_, nullptr, (__nv_bfloat16 *)a1_, (__nv_bfloat16 *)a2_,
             (__nv_bfloat16 *)a3_, err_);
     else

@@ -26,8 +26,11 @@ public:
     // wait for `s` and report a tensor-core completion wait that ran out
     int sync(cudaStream_t s) const;
     float confidence() const { return conf_limit_; }
-    // p (and fallback flags) of ntiles tiles of features, [tile][1280]
-    int forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8_t *d_fallback, cudaStream_t s) const;
+    // p (and fallback flags) of ntiles tiles of features, [tile][1280].
+    // repeating: every tile's features repeat along (kz + 4, ky + 16), as those
+    // of the walk's feature pass do (on the tensor cores half the work).
+    int forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8_t *d_fallback, cudaStream_t s,
+                bool repeating = false) const;
     // Loss and gradients of a batch (ac: per bin |X|^2 and Re(C conj X));
     // lr > 0 then takes one Adam step. loss / host_grad (NPARAM floats), when
     // given, are filled after a stream synchronisation.
