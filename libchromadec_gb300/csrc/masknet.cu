@@ -27,12 +27,12 @@
 //  * mn_forward_kernel<TRAIN>: features -> p (+ fallback flags), the
 //    cross-check of the tensor-core pass; the training variant also keeps
 //    each layer's activations for the backward pass.
-//  * mn_loss_kernel: dL/dz of the head for L = sum |p X - C|^2 / sum |X|^2.
-//  * mn_backward_kernel: the head, then per layer the weight gradient (thread
-//    (ci, co) sums over the tile's voxels for all 27 taps) and the input
-//    gradient (the transposed convolution), each CTA adding into its own
-//    slice of a partial-gradient buffer; mn_adam_kernel reduces the slices
-//    and takes one Adam step on the FP32 master weights.
+// Training:
+//  * mn_backward_kernel: dL/dz of the head for L = sum |p X - C|^2 / sum |X|^2,
+//    the head, then per layer the weight and input gradients as tensor-core
+//    contractions; described where it is defined. Each CTA writes its own
+//    slice of a partial-gradient buffer; mn_adam_kernel reduces the slices and
+//    takes one Adam step on the FP32 master weights.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -113,19 +113,6 @@ struct WFwd {
     }
 };
 
-// Transposed, flipped rows for the input gradient: input channel = the
-// layer's output channel co, outputs = its input channels ci:
-// w[ci] = W[26 - t][ci][co]
-struct WTrans {
-    const float *W;
-    __device__ __forceinline__ void operator()(int t, int co, float (&w)[NC]) const
-    {
-        const float *p = W + (26 - t) * NC * NC + co;
-#pragma unroll
-        for (int ci = 0; ci < NC; ci++) w[ci] = p[ci * NC];
-    }
-};
-
 struct InBf16 {
     const __nv_bfloat16 *a;   // [16][CS]
     __device__ __forceinline__ float operator()(int c, int v) const { return __bfloat162float(a[c * CS + v]); }
@@ -166,13 +153,20 @@ __device__ __forceinline__ void load_input(const uint16_t *feat_tile, float *x0,
     }
 }
 
-__device__ __forceinline__ void copy_act_out(const __nv_bfloat16 *s, __nv_bfloat16 *g, int zy)
+// Activations kept for the backward pass: [tile][channel half][voxel][8]
+// bf16, the backward pass's shared layout.
+__device__ __forceinline__ size_t act_at(long long tile, int c, int v)
 {
-    // [16][CS] shared -> [16][NV] global, the thread's column
+    return ((size_t)tile * 2 + (c >> 3)) * (NV * 8) + (size_t)v * 8 + (c & 7);
+}
+
+__device__ __forceinline__ void copy_act_out(const __nv_bfloat16 *s, __nv_bfloat16 *g, long long tile, int zy)
+{
+    // [16][CS] shared -> the thread's column
 #pragma unroll
     for (int c = 0; c < NC; c++)
 #pragma unroll
-        for (int q = 0; q < NQ; q++) g[c * NV + q * NZY + zy] = s[c * CS + q * NZY + zy];
+        for (int q = 0; q < NQ; q++) g[act_at(tile, c, q * NZY + zy)] = s[c * CS + q * NZY + zy];
 }
 
 __device__ __forceinline__ float block_sum(float v, float *red)
@@ -191,7 +185,7 @@ __device__ __forceinline__ float block_sum(float v, float *red)
 constexpr size_t kFwdSmem = sizeof(float) * (NPARAM_PAD + 2 * NV) + 2 * sizeof(__nv_bfloat16) * NC * CS;
 
 // params: the network's weights as used (weights bf16-rounded, biases FP32).
-// TRAIN: also write A1, A2, A3 ([tile][16][NV] bf16 each) for the backward pass.
+// TRAIN: also write A1, A2, A3 (act_at) for the backward pass.
 template <bool TRAIN>
 __global__ void __launch_bounds__(kThreads, 1)
     mn_forward_kernel(const float *params, const uint16_t *feat, long long ntiles, float conf_limit, float *p_out,
@@ -221,8 +215,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         acc_init(acc, wsm + OFF_B3);
         conv_acc<NC>(InBf16{act1}, WFwd<NC>{wsm + OFF_W3}, z, y, acc);
         if (TRAIN) {
-            copy_act_out(act0, a1g + tile * NC * NV, zy);
-            copy_act_out(act1, a2g + tile * NC * NV, zy);
+            copy_act_out(act0, a1g, tile, zy);
+            copy_act_out(act1, a2g, tile, zy);
         }
         float conf = 0.f;
 #pragma unroll
@@ -231,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int co = 0; co < NC; co++) {
                 const float a = bfr(fmaxf(acc[q][co], 0.f));
-                if (TRAIN) a3g[tile * NC * NV + co * NV + q * NZY + zy] = __float2bfloat16_rn(a);
+                if (TRAIN) a3g[act_at(tile, co, q * NZY + zy)] = __float2bfloat16_rn(a);
                 zh = __fmaf_rn(a, wsm[OFF_WH + co], zh);
             }
             const float p = 1.0f / (1.0f + expf(-zh));
@@ -254,193 +248,486 @@ __global__ void mn_sum_kernel(const float2 *ac, long long n, double *out)
     if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
 }
 
-// dz = dL/dz_head = 2 (p a - c) / S * p (1 - p); loss partial sums
-__global__ void mn_loss_kernel(const float *p, const float2 *ac, long long n, const double *S, float *dz, double *loss)
+// ---------------------------------------------------------------------------
+// Backward pass
+// ---------------------------------------------------------------------------
+// One CTA of 9 warps a tile, two CTAs a SM. Activations and pre-activation
+// gradients are bf16 (the gradients rounded once, as they enter the next
+// contraction) in shared memory as [channel half][voxel][8], 16 bytes a row:
+// ldmatrix reads any 8 voxels, so a tap's shift is only another row address,
+// and the same rows serve both contractions of a layer:
+//  * weight gradient g[tap][ci][co] = sum_v in[ci][v + tap] d[co][v]: M = ci,
+//    N = co, K = 16 voxels along ky, both operands transposed by ldmatrix.
+//    Warp w owns the (dz, dy) of that index and its three dq taps; per (kz, ky
+//    half) it loads the five q rows of each operand once for 13 pairs.
+//  * input gradient dA[v][ci] = sum_tap,co d[v - tap][co] W[tap][ci][co]: M = 16
+//    voxels along ky, N = ci, K = co; a (kz, ky half) is one unit of work, its
+//    five q accumulated together. The result is rounded to bf16, and a few
+//    bright bins carry most of a gradient, so a value near a rounding boundary
+//    that falls on the other side moves the gradient by up to 1e-4 of it:
+//    values within a bound of both sums' rounding errors of a boundary are summed
+//    again one product after another, in the order (dz, dy,
+//    co, dq), so what is rounded does not depend on the tensor cores' order.
+// The contractions have N = 16 a tap and operands that shift by single rows, so
+// they are m16n8k16 mma.sync on registers: a tcgen05 tile (M 128, N 16, K 16 a
+// tap) would leave its accumulator almost empty. FP32 accumulation; the weight
+// gradient's tensor-core sums are five products long and then added in FP32.
+//
+// 256 tiles: 622 us on the CUDA cores (thread (ci, co) walking the voxels, two
+// rounds of 152 CTAs) -> 133 us, of which the values summed again are about
+// half; the whole step 764 -> 225 us.
+constexpr int kBwdThreads = 288;
+constexpr int kActBytes = 2 * NV * 16;
+constexpr int kNearCap = 2048;              // values to sum again that are listed; more are summed at once
+constexpr size_t kBwdSmem = 2 * kActBytes + sizeof(float) * (2 * NV + 9 * 20 + 32) + sizeof(uint16_t) * kNearCap + 16;
+constexpr int kWFragBytes = 27 * 32 * 16;   // a layer's weights as B fragments of the input gradient
+
+__device__ __forceinline__ void ldsm4(uint32_t a, uint32_t (&r)[4])
 {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t a, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm2t(uint32_t a, uint32_t &r0, uint32_t &r1)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void load_act(uint32_t dst, const __nv_bfloat16 *g)
+{
+    const char *src = reinterpret_cast<const char *>(g);
+    for (int i = threadIdx.x; i < kActBytes / 16; i += kBwdThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// first: store, else add (the CTA's own slice)
+__device__ __forceinline__ void put_grad(float *g, float v, bool first) { *g = first ? v : *g + v; }
+
+// Weight gradient of a 16-channel layer: `in` and `d` in shared memory.
+__device__ __forceinline__ void wgrad16(uint32_t in, uint32_t d, float *gw, bool first)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int dz = warp / 3 - 1, dy = warp % 3 - 1;
+    // lane's row and channel half of the four 8x8 matrices of an operand
+    const int mi = lane >> 3;
+    const int ra = (lane & 7) + (mi >> 1) * 8, ha = mi & 1;   // A: (half 0, rows 0-7), (1, 0-7), (0, 8-15), (1, 8-15)
+    const int rb = (lane & 7) + (mi & 1) * 8, hb = mi >> 1;   // B: (0, 0-7), (0, 8-15), (1, 0-7), (1, 8-15)
+    float acc[3][2][4] = {};
+#pragma unroll 1
+    for (int u = 0; u < 16; u++) {
+        const int kz = u >> 1, blk = u & 1;
+        const int va = (((kz + dz) & 7) << 5) | ((16 * blk + ra + dy) & 31), vb = (kz << 5) | (16 * blk + rb);
+        const uint32_t pa = in + (ha * NV + va) * 16, pb = d + (hb * NV + vb) * 16;
+        uint32_t A[NQ][4], B[NQ][4];
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            ldsm4t(pa + q * NZY * 16, A[q]);
+            ldsm4t(pb + q * NZY * 16, B[q]);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            float c[2][4] = {};
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {
+                const int qi = q + j - 1;
+                if (qi < 0 || qi >= NQ) continue;
+                mma16816(c[0], A[qi][0], A[qi][1], A[qi][2], A[qi][3], B[q][0], B[q][1]);
+                mma16816(c[1], A[qi][0], A[qi][1], A[qi][2], A[qi][3], B[q][2], B[q][3]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[j][n][i] += c[n][i];
+        }
+    }
+    const int g = lane >> 2, tq = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                put_grad(gw + ((warp * 3 + j) * NC + g + 8 * (i >> 1)) * NC + 8 * n + 2 * tq + (i & 1), acc[j][n][i], first);
+}
+
+// One input-gradient value, voxel and channel id = 16 v + ci, as one chain of
+// FP32 FMAs; W: the layer's weights.
+__device__ __noinline__ float dgrad_one(const __nv_bfloat16 *d, const float *W, int id)
+{
+    const int v = id >> 4, ci = id & 15, q = v >> 8, z = (v >> 5) & 7, y = v & 31;
+    float acc = 0.f;
+#pragma unroll 1
+    for (int zy = 0; zy < 9; zy++) {
+        const int at = (((z + zy / 3 - 1) & 7) << 5) | ((y + zy % 3 - 1) & 31);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {   // eight co at a time
+            uint4 x[3];
+            float4 w[3][2];
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int qi = q + j - 1;
+                x[j] = qi >= 0 && qi < NQ ? reinterpret_cast<const uint4 *>(d)[h * NV + qi * NZY + at] : make_uint4(0, 0, 0, 0);
+                const float4 *row = reinterpret_cast<const float4 *>(W + ((26 - (zy * 3 + j)) * NC + ci) * NC + 8 * h);
+                w[j][0] = __ldg(row);
+                w[j][1] = __ldg(row + 1);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    acc = __fmaf_rn(__bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(&x[j])[c]),
+                                    reinterpret_cast<const float *>(&w[j])[c], acc);
+        }
+    }
+    return acc;
+}
+
+// Values near a rounding boundary: reach[v] = the 2-norm of the 27 x 16
+// gradients the value is a sum of, wmax[ci] the layer's largest |W|, near the list and its count.
+struct DgradNear {
+    const float *reach, *wmax;
+    uint16_t *list;
+    int *count;
+};
+
+// Input gradient of a 16-channel layer from `d`, masked by the activations in
+// `act` (> 0) and rounded to bf16 in their place.
+__device__ __forceinline__ void dgrad16(const __nv_bfloat16 *dbuf, uint32_t d, __nv_bfloat16 *act, const uint4 *wfrag,
+                                        const float *W0, const DgradNear &N)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int mi = lane >> 3, r = (lane & 7) + (mi & 1) * 8, h = mi >> 1;
+    const int g = lane >> 2, tq = lane & 3;
+#pragma unroll 1
+    for (int u = warp; u < 16; u += 9) {
+        const int kz = u >> 1, blk = u & 1;
+        float acc[NQ][2][4] = {};
+#pragma unroll 1
+        for (int zy = 0; zy < 9; zy++) {
+            const int dz = zy / 3 - 1, dy = zy % 3 - 1;
+            const int v = (((kz - dz) & 7) << 5) | ((16 * blk + r - dy) & 31);
+            const uint32_t pa = d + (h * NV + v) * 16;
+            uint32_t A[NQ][4];
+            uint4 W[3];
+#pragma unroll
+            for (int q = 0; q < NQ; q++) ldsm4(pa + q * NZY * 16, A[q]);
+#pragma unroll
+            for (int j = 0; j < 3; j++) W[j] = __ldg(wfrag + (zy * 3 + j) * 32 + lane);
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+#pragma unroll
+                for (int q = 0; q < NQ; q++) {
+                    const int qd = q - (j - 1);
+                    if (qd < 0 || qd >= NQ) continue;
+                    mma16816(acc[q][0], A[qd][0], A[qd][1], A[qd][2], A[qd][3], W[j].x, W[j].y);
+                    mma16816(acc[q][1], A[qd][0], A[qd][1], A[qd][2], A[qd][3], W[j].z, W[j].w);
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {   // rows g, g + 8
+                const int v = ((q * 8 + kz) << 5) | (16 * blk + g + 8 * i);
+                const float reach = N.reach[v];
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    __nv_bfloat162 *at = reinterpret_cast<__nv_bfloat162 *>(act + (n * NV + v) * 8 + 2 * tq);
+                    const float2 a = __bfloat1622float2(*at);
+                    float o[2] = {0.f, 0.f};
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        if (!((k ? a.y : a.x) > 0.f)) continue;
+                        float x = acc[q][n][2 * i + k];
+                        // distance to the midpoint of two bf16 values, in
+                        // units of 2^(exponent - 23), against 2^-18 of a bound of
+                        // the products' 2-norm: each of the 432 sums is rounded
+                        // by 2^-25 of a partial sum of about that norm, so this is
+                        // several times the error of either order
+                        const uint32_t bits = __float_as_uint(x);
+                        const int ci = 8 * n + 2 * tq + k;
+                        const float dist = (float)abs((int)(bits & 0xFFFFu) - 0x8000);
+                        if (dist * __uint_as_float(bits & 0x7F800000u) <= 32.0f * N.wmax[ci] * reach) {
+                            const int slot = atomicAdd(N.count, 1);
+                            if (slot < kNearCap) N.list[slot] = (uint16_t)(v * 16 + ci);
+                            else x = dgrad_one(dbuf, W0, v * 16 + ci);
+                        }
+                        o[k] = x;
+                    }
+                    __nv_bfloat162 w;
+                    w.x = __float2bfloat16_rn(o[0]);
+                    w.y = __float2bfloat16_rn(o[1]);
+                    *at = w;
+                }
+            }
+    }
+}
+
+// sum over the voxels of each channel of a gradient buffer -> red[warp][8] for
+// the channel half warp / 4 (8 warps)
+__device__ __forceinline__ void channel_sums(const __nv_bfloat16 *buf, float *red)
+{
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    if (t >= 256) return;
+    const int h = t >> 7;
+    float s[8] = {};
+    for (int v = t & 127; v < NV; v += 128) {
+        const uint4 raw = reinterpret_cast<const uint4 *>(buf)[h * NV + v];
+        const __nv_bfloat16 *a = reinterpret_cast<const __nv_bfloat16 *>(&raw);
+#pragma unroll
+        for (int c = 0; c < 8; c++) s[c] += __bfloat162float(a[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], m);
+    if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 8; c++) red[warp * 20 + c] = s[c];
+}
+
+__global__ void __launch_bounds__(kBwdThreads, 2)
+    mn_backward_kernel(const float *params, const uint8_t *wfrag, const uint16_t *feat, const __nv_bfloat16 *a1g,
+                       const __nv_bfloat16 *a2g, const __nv_bfloat16 *a3g, const float *pg, const float2 *acg,
+                       const double *S, long long ntiles, float *gpart, double *loss)
+{
+    extern __shared__ __align__(128) uint8_t bsm[];
+    __nv_bfloat16 *bufA = reinterpret_cast<__nv_bfloat16 *>(bsm), *bufB = bufA + 2 * NV * 8;
+    float *dzs = reinterpret_cast<float *>(bsm + 2 * kActBytes);   // [NV]
+    float *reach = dzs + NV;                                       // [NV]
+    float *red = reach + NV;                                       // [9][20]
+    float *wmax = red + 9 * 20;                                    // [2 layers][16]
+    int *near_count = reinterpret_cast<int *>(wmax + 32);
+    uint16_t *near_list = reinterpret_cast<uint16_t *>(near_count + 4);
+    const uint32_t sA = (uint32_t)__cvta_generic_to_shared(bufA), sB = (uint32_t)__cvta_generic_to_shared(bufB);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    float *gp = gpart + (size_t)blockIdx.x * NPARAM;
     const float inv = (float)(1.0 / *S);
     double l = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float pv = p[i];
-        const float2 v = ac[i];
-        const float dp = 2.0f * (pv * v.x - v.y) * inv;
-        dz[i] = dp * pv * (1.0f - pv);
-        l += (double)((pv * pv * v.x - 2.0f * pv * v.y) * inv);
+    const uint4 *w2 = reinterpret_cast<const uint4 *>(wfrag), *w3 = w2 + kWFragBytes / 16;
+    // the largest |weight| of layers 2 and 3 per input channel
+    if (t < 32) wmax[t] = 0.f;
+    __syncthreads();
+    {
+        const int pair = t / 9, layer = pair >> 4, ci = pair & 15;
+        const float *W = params + (layer == 0 ? OFF_W2 : OFF_W3);
+        float m = 0.f;
+        for (int k = 0; k < 48; k++) {
+            const int e = (t % 9) * 48 + k;   // (tap, co)
+            m = fmaxf(m, fabsf(W[((e >> 4) * NC + ci) * NC + (e & 15)]));
+        }
+        atomicMax(reinterpret_cast<int *>(wmax + pair), __float_as_int(m));
+    }
+    // Input gradient of layer L (1: layer 2, 2: layer 3) from d into act, and
+    // its channel sums, the previous layer's bias gradient, into gp + off.
+    auto input_gradient = [&](int L, const __nv_bfloat16 *dbuf, uint32_t d, __nv_bfloat16 *act, int off, bool first) {
+        const float *W = params + (L == 1 ? OFF_W2 : OFF_W3);
+        for (int v = t; v < NV; v += kBwdThreads) {
+            float s = 0.f;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint4 raw = reinterpret_cast<const uint4 *>(dbuf)[h * NV + v];
+                const __nv_bfloat16 *a = reinterpret_cast<const __nv_bfloat16 *>(&raw);
+#pragma unroll
+                for (int c = 0; c < 8; c++) s = __fmaf_rn(__bfloat162float(a[c]), __bfloat162float(a[c]), s);
+            }
+            dzs[v] = s;
+        }
+        if (t == 0) *near_count = 0;
+        __syncthreads();
+        for (int v = t; v < NV; v += kBwdThreads) {
+            const int q = v >> 8, z = (v >> 5) & 7, y = v & 31;
+            float s = 0.f;
+            for (int zy = 0; zy < 9; zy++) {
+                const int at = (((z + zy / 3 - 1) & 7) << 5) | ((y + zy % 3 - 1) & 31);
+                for (int qi = max(q - 1, 0); qi <= min(q + 1, NQ - 1); qi++) s += dzs[qi * NZY + at];
+            }
+            reach[v] = sqrtf(s);
+        }
+        __syncthreads();
+        const DgradNear N = {reach, wmax + 16 * (L - 1), near_list, near_count};
+        dgrad16(dbuf, d, act, L == 1 ? w2 : w3, W, N);
+        __syncthreads();
+        const int n = min(*near_count, kNearCap);
+        for (int i = t; i < n; i += kBwdThreads) {
+            const int id = near_list[i];
+            act[((id & 15) >> 3) * NV * 8 + (id >> 4) * 8 + (id & 7)] = __float2bfloat16_rn(dgrad_one(dbuf, W, id));
+        }
+        __syncthreads();
+        channel_sums(act, red);
+        __syncthreads();
+        if (t < NC) {
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; w++) s += red[(4 * (t >> 3) + w) * 20 + (t & 7)];
+            put_grad(gp + off + t, s, first);
+        }
+    };
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const bool first = tile == blockIdx.x;
+        __syncthreads();   // the previous tile is done with the buffers
+        // dz = dL/dz_head = 2 (p a - c) / S * p (1 - p); loss partial sums
+        for (int v = t; v < NV; v += kBwdThreads) {
+            const float pv = pg[tile * NV + v];
+            const float2 ac = acg[tile * NV + v];
+            const float dp = 2.0f * (pv * ac.x - ac.y) * inv;
+            dzs[v] = dp * pv * (1.0f - pv);
+            l += (double)((pv * pv * ac.x - 2.0f * pv * ac.y) * inv);
+        }
+        load_act(sB, a3g + tile * NC * NV);
+        __syncthreads();
+        // head: d wh[c] = sum_v dz[v] A3[c][v], d bh = sum_v dz[v];
+        // dZ3 = bf16(dz wh[c] (A3 > 0)) and its sums (layer 3's bias gradient)
+        if (t < 256) {
+            const int h = t >> 7;
+            float sw[8] = {}, sb[8] = {}, sz = 0.f, wh[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) wh[c] = params[OFF_WH + 8 * h + c];
+            for (int v = t & 127; v < NV; v += 128) {
+                const float dz = dzs[v];
+                const uint4 raw = reinterpret_cast<const uint4 *>(bufB)[h * NV + v];
+                const __nv_bfloat16 *a = reinterpret_cast<const __nv_bfloat16 *>(&raw);
+                __align__(16) __nv_bfloat16 o[8];
+                sz += dz;
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const float av = __bfloat162float(a[c]);
+                    sw[c] = __fmaf_rn(dz, av, sw[c]);
+                    o[c] = __float2bfloat16_rn(av > 0.f ? dz * wh[c] : 0.f);
+                    sb[c] += __bfloat162float(o[c]);
+                }
+                reinterpret_cast<uint4 *>(bufA)[h * NV + v] = *reinterpret_cast<const uint4 *>(o);
+            }
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) {
+                sz += __shfl_xor_sync(0xffffffffu, sz, m);
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    sw[c] += __shfl_xor_sync(0xffffffffu, sw[c], m);
+                    sb[c] += __shfl_xor_sync(0xffffffffu, sb[c], m);
+                }
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    red[warp * 20 + c] = sw[c];
+                    red[warp * 20 + 8 + c] = sb[c];
+                }
+                red[warp * 20 + 16] = sz;
+            }
+        }
+        __syncthreads();
+        if (t < 33) {
+            const int h = (t & 15) >> 3, i = t < 32 ? (t >> 4) * 8 + (t & 7) : 16;
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; w++) s += red[(4 * (t < 32 ? h : 0) + w) * 20 + i];
+            put_grad(gp + (t < 16 ? OFF_WH + t : t < 32 ? OFF_B3 + t - 16 : OFF_BH), s, first);
+        }
+        load_act(sB, a2g + tile * NC * NV);
+        __syncthreads();
+        // layer 3: weight gradient, then dA2 -> dZ2 in place of A2
+        wgrad16(sB, sA, gp + OFF_W3, first);
+        __syncthreads();
+        input_gradient(2, bufA, sA, bufB, OFF_B2, first);
+        __syncthreads();   // dZ3 has been read, dZ2 is complete
+        load_act(sA, a1g + tile * NC * NV);
+        __syncthreads();
+        // layer 2
+        wgrad16(sA, sB, gp + OFF_W2, first);
+        __syncthreads();
+        input_gradient(1, bufB, sB, bufA, OFF_B1, first);
+        // layer 1: the two input channels at q - 1, q, q + 1 as six rows of M,
+        // so only the (dz, dy) taps remain
+        {
+            const __nv_bfloat16 *f = reinterpret_cast<const __nv_bfloat16 *>(feat + tile * NV);
+            __syncthreads();   // dZ2 has been read
+            for (int v = t; v < NV; v += kBwdThreads) {
+                const int q = v >> 8, zy = v & 255, z = zy >> 5, y = zy & 31;
+                const int mzy = (((10 - z) & 7) << 5) | ((40 - y) & 31);
+                __align__(16) __nv_bfloat16 x[8];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const int qi = q + j - 1;
+                    const bool in = qi >= 0 && qi < NQ;
+                    x[2 * j] = in ? f[qi * NZY + zy] : __float2bfloat16_rn(0.f);
+                    x[2 * j + 1] = in ? f[(4 - qi) * NZY + mzy] : __float2bfloat16_rn(0.f);
+                }
+                x[6] = x[7] = __float2bfloat16_rn(0.f);
+                reinterpret_cast<uint4 *>(bufB)[v] = *reinterpret_cast<const uint4 *>(x);
+            }
+            __syncthreads();
+            const int dz = warp / 3 - 1, dy = warp % 3 - 1;
+            const int mi = lane >> 3, ra = (lane & 7) + (mi & 1) * 8;
+            float acc[2][4] = {};
+#pragma unroll 1
+            for (int u = 0; u < 16; u++) {
+                const int kz = u >> 1, blk = u & 1;
+                const uint32_t pa = sB + ((((kz + dz) & 7) << 5) | ((16 * blk + ra + dy) & 31)) * 16;
+                const uint32_t pb = sA + ((mi >> 1) * NV + ((kz << 5) | (16 * blk + ra))) * 16;
+                float c[2][4] = {};
+#pragma unroll
+                for (int q = 0; q < NQ; q++) {
+                    uint32_t a0, a2, B[4];
+                    ldsm2t(pa + q * NZY * 16, a0, a2);
+                    ldsm4t(pb + q * NZY * 16, B);
+                    mma16816(c[0], a0, 0u, a2, 0u, B[0], B[1]);
+                    mma16816(c[1], a0, 0u, a2, 0u, B[2], B[3]);
+                }
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    acc[n][0] += c[n][0];
+                    acc[n][1] += c[n][1];
+                }
+            }
+            const int g = lane >> 2, tq = lane & 3;
+            if (g < 6)
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+                        put_grad(gp + OFF_W1 + ((warp * 3 + (g >> 1)) * NCIN + (g & 1)) * NC + 8 * n + 2 * tq + i, acc[n][i], first);
+        }
     }
 #pragma unroll
     for (int h = 16; h >= 1; h >>= 1) l += __shfl_xor_sync(0xffffffffu, l, h);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
+    if (lane == 0) atomicAdd(loss, l);
 }
 
-// Weight gradient of one layer for the thread's (ci, co):
-// g[t] += sum_v in[ci][v + t] * d[co][v]
-template <typename In, typename D>
-__device__ __forceinline__ void wgrad(const In &in, const D &d, int ci, int co, float (&g)[27])
+// One Adam step: g = sum over the partial slices; the FP32 master weights
+// move, and `used` gets the values the kernels compute with (weights rounded
+// to bf16, biases as they are). A block takes 32 parameters, eight warps an
+// eighth of the slices each: one thread a parameter summed the slices one
+// after another on 58 blocks (101 us at 152 slices).
+__global__ void __launch_bounds__(256)
+    mn_adam_kernel(float *master, float *used, float *m, float *v, const float *gpart, int nslices, float lr, float b1,
+                   float b2, float eps, float c1, float c2, float *grad_out)
 {
-#pragma unroll 1
-    for (int zy = 0; zy < NZY; zy++) {
-        const int z = zy >> 5, y = zy & 31;
-        float dv[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) dv[q] = d(co, q * NZY + zy);
-#pragma unroll
-        for (int dz = -1; dz <= 1; dz++) {
-#pragma unroll
-            for (int dy = -1; dy <= 1; dy++) {
-                const int zy2 = (((z + dz) & 7) << 5) | ((y + dy) & 31);
-                float xin[NQ + 2];
-                xin[0] = 0.f;
-                xin[NQ + 1] = 0.f;
-#pragma unroll
-                for (int q = 0; q < NQ; q++) xin[q + 1] = in(ci, q * NZY + zy2);
-                const int tb = (dz + 1) * 9 + (dy + 1) * 3;
-#pragma unroll
-                for (int j = 0; j < 3; j++)
-#pragma unroll
-                    for (int q = 0; q < NQ; q++) g[tb + j] = __fmaf_rn(xin[q + j], dv[q], g[tb + j]);
-            }
-        }
-    }
-}
-
-constexpr size_t kBwdSmem =
-    sizeof(float) * (NPARAM_PAD + 2 * NV + NV) + 2 * sizeof(__nv_bfloat16) * NC * CS;
-
-__device__ __forceinline__ void load_act(const __nv_bfloat16 *g, __nv_bfloat16 *s, int zy)
-{
-#pragma unroll
-    for (int c = 0; c < NC; c++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) s[c * CS + q * NZY + zy] = g[c * NV + q * NZY + zy];
-}
-
-// The backward pass of the tiles given; each CTA accumulates into
-// gpart[blockIdx.x][NPARAM] (zeroed by the caller).
-__global__ void __launch_bounds__(kThreads, 1)
-    mn_backward_kernel(const float *params, const uint16_t *feat, const __nv_bfloat16 *a1g,
-                       const __nv_bfloat16 *a2g, const __nv_bfloat16 *a3g, const float *dzg, long long ntiles,
-                       float *gpart)
-{
-    extern __shared__ float4 smem4[];
-    float *wsm = reinterpret_cast<float *>(smem4);
-    float *x0 = wsm + NPARAM_PAD;   // [2][NV]
-    float *dzs = x0 + 2 * NV;       // [NV]
-    __nv_bfloat16 *bufA = reinterpret_cast<__nv_bfloat16 *>(dzs + NV);
-    __nv_bfloat16 *bufB = bufA + NC * CS;
-    for (int i = threadIdx.x; i < NPARAM; i += kThreads) wsm[i] = params[i];
-    const int t = threadIdx.x, zy = t, z = zy >> 5, y = zy & 31;
-    const int ci = t >> 4, co = t & 15;   // the thread's weight-gradient pair
-    float *gp = gpart + (size_t)blockIdx.x * NPARAM;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        __syncthreads();
-        // head: dz, A3
-        for (int q = 0; q < NQ; q++) dzs[q * NZY + zy] = dzg[tile * NV + q * NZY + zy];
-        load_act(a3g + tile * NC * NV, bufA, zy);
-        __syncthreads();
-        {
-            // d wh[co] = sum_v dz[v] A3[co][v]; d bh = sum_v dz[v] (threads split the voxels)
-            const int part = t >> 4;   // 16 parts of 80 voxels
-            float s = 0.f, sb = 0.f;
-            for (int v = part * 80; v < part * 80 + 80; v++) {
-                s = __fmaf_rn(dzs[v], __bfloat162float(bufA[co * CS + v]), s);
-                if (co == 0) sb += dzs[v];
-            }
-            atomicAdd(gp + OFF_WH + co, s);
-            if (co == 0) atomicAdd(gp + OFF_BH, sb);
-        }
-        __syncthreads();
-        // dZ3 = bf16(dz * wh[c] * (A3 > 0)), in place
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const int e = c * CS + q * NZY + zy;
-                const float a = __bfloat162float(bufA[e]);
-                bufA[e] = __float2bfloat16_rn(a > 0.f ? dzs[q * NZY + zy] * wsm[OFF_WH + c] : 0.f);
-            }
-        load_act(a2g + tile * NC * NV, bufB, zy);
-        __syncthreads();
-        // layer 3: weight and bias gradients, then dA2 -> dZ2 in place of A2
-        {
-            float g[27];
-#pragma unroll
-            for (int k = 0; k < 27; k++) g[k] = 0.f;
-            wgrad(InBf16{bufB}, InBf16{bufA}, ci, co, g);
-#pragma unroll
-            for (int k = 0; k < 27; k++) gp[OFF_W3 + (k * NC + ci) * NC + co] += g[k];
-            if (ci == 0) {
-                float b = 0.f;
-                for (int v = 0; v < NV; v++) b += __bfloat162float(bufA[co * CS + v]);
-                gp[OFF_B3 + co] += b;
-            }
-        }
-        float acc[NQ][NC];
-        acc_init(acc, nullptr);
-        conv_acc<NC>(InBf16{bufA}, WTrans{wsm + OFF_W3}, z, y, acc);
-        __syncthreads();   // every thread has read A2 for the weight gradient
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const int e = c * CS + q * NZY + zy;
-                bufB[e] = __float2bfloat16_rn(__bfloat162float(bufB[e]) > 0.f ? acc[q][c] : 0.f);
-            }
-        load_act(a1g + tile * NC * NV, bufA, zy);   // dZ3 is no longer needed
-        __syncthreads();
-        // layer 2
-        {
-            float g[27];
-#pragma unroll
-            for (int k = 0; k < 27; k++) g[k] = 0.f;
-            wgrad(InBf16{bufA}, InBf16{bufB}, ci, co, g);
-#pragma unroll
-            for (int k = 0; k < 27; k++) gp[OFF_W2 + (k * NC + ci) * NC + co] += g[k];
-            if (ci == 0) {
-                float b = 0.f;
-                for (int v = 0; v < NV; v++) b += __bfloat162float(bufB[co * CS + v]);
-                gp[OFF_B2 + co] += b;
-            }
-        }
-        acc_init(acc, nullptr);
-        conv_acc<NC>(InBf16{bufB}, WTrans{wsm + OFF_W2}, z, y, acc);
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const int e = c * CS + q * NZY + zy;
-                bufA[e] = __float2bfloat16_rn(__bfloat162float(bufA[e]) > 0.f ? acc[q][c] : 0.f);
-            }
-        load_input(feat + tile * NV, x0, zy);
-        __syncthreads();
-        // layer 1 (two input channels)
-        if (ci < NCIN) {
-            float g[27];
-#pragma unroll
-            for (int k = 0; k < 27; k++) g[k] = 0.f;
-            wgrad(InF32{x0}, InBf16{bufA}, ci, co, g);
-#pragma unroll
-            for (int k = 0; k < 27; k++) gp[OFF_W1 + (k * NCIN + ci) * NC + co] += g[k];
-        } else if (ci == NCIN) {
-            float b = 0.f;
-            for (int v = 0; v < NV; v++) b += __bfloat162float(bufA[co * CS + v]);
-            gp[OFF_B1 + co] += b;
-        }
-    }
-}
-
-// One Adam step: g = sum over the partial slices (then zeroed); the FP32
-// master weights move, and `used` gets the values the kernels compute with
-// (weights rounded to bf16, biases as they are).
-__global__ void mn_adam_kernel(float *master, float *used, float *m, float *v, float *gpart, int nslices, float lr,
-                               float b1, float b2, float eps, float c1, float c2, float *grad_out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (i < NPARAM)
+#pragma unroll 8
+        for (int k = grp; k < nslices; k += 8) s += gpart[(size_t)k * NPARAM + i];
+    part[grp][lane] = s;
+    __syncthreads();
+    if (grp != 0 || i >= NPARAM) return;
     float g = 0.f;
-    for (int s = 0; s < nslices; s++) {
-        g += gpart[(size_t)s * NPARAM + i];
-        gpart[(size_t)s * NPARAM + i] = 0.f;
-    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) g += part[k][lane];
     if (grad_out) grad_out[i] = g;
     if (lr == 0.f) return;
     const float mi = b1 * m[i] + (1.f - b1) * g;
@@ -590,10 +877,20 @@ __device__ __forceinline__ void weight_piece(int p, int &off, int &bytes)
     bytes = 3 * 48 * band_q(ks) * 32;
 }
 
+// The weight images, and behind them the backward pass's B fragments of
+// layers 2 and 3: [tap][lane] of (n 0 k-low, n 0 k-high, n 1 ..., n 1 ...).
 __global__ void mn_build_images_kernel(const float *used, uint8_t *img)
 {
-    const int n1 = 3 * NCOL * 16, n2 = 3 * 48 * 13 * 16;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n1 + 2 * n2; idx += gridDim.x * blockDim.x) {
+    const int n1 = 3 * NCOL * 16, n2 = 3 * 48 * 13 * 16, n3 = 27 * 32 * 8;
+    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n1 + 2 * n2 + 2 * n3; idx += gridDim.x * blockDim.x) {
+        if (idx >= n1 + 2 * n2) {
+            const int e = idx - n1 - 2 * n2, layer = e / n3, r = e % n3;
+            const int part = r & 1, reg = (r >> 1) & 3, lane = (r >> 3) & 31, tap = r >> 8;
+            const int ci = 8 * (reg >> 1) + (lane >> 2), co = 8 * (reg & 1) + 2 * (lane & 3) + part;
+            reinterpret_cast<__nv_bfloat16 *>(img + IMG_BYTES)[e] =
+                __float2bfloat16_rn(used[(layer == 0 ? OFF_W2 : OFF_W3) + (tap * NC + ci) * NC + co]);
+            continue;
+        }
         const int k = idx & 15;
         float v = 0.f;
         uint32_t off;
@@ -1037,10 +1334,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                         *reinterpret_cast<const uint4 *>(stash + (kz * 10 + ch) * 16);
                             }
                             if (TRAIN) {
-                                __nv_bfloat16 *ag = (L == 0 ? a1g : a2g) + tile * NC * NV;
-                                const int vox = (q * 8 + kz) * 32 + ky;
-#pragma unroll
-                                for (int c = 0; c < 8; c++) ag[(h * 8 + c) * NV + vox] = o[c];
+                                __nv_bfloat16 *ag = L == 0 ? a1g : a2g;
+                                *reinterpret_cast<uint4 *>(ag + act_at(tile, 8 * h, (q * 8 + kz) * 32 + ky)) = ov;
                             }
                             if (b == 1) {
                                 // the next layer's input chunk q is complete
@@ -1080,12 +1375,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             combine_block(cur, lane, y);
                             const int vox = (q * 8 + kz) * 32 + ky;
                             float zh = zh0;
+                            __align__(16) __nv_bfloat16 a3[TRAIN ? NC : 1];
 #pragma unroll
                             for (int co = 0; co < NC; co++) {
                                 const float a = bfr(fmaxf(y[co] + s_par[2 * NC + co], 0.f));
-                                if (TRAIN) a3g[tile * NC * NV + co * NV + vox] = __float2bfloat16_rn(a);
+                                if (TRAIN) a3[co] = __float2bfloat16_rn(a);
                                 zh = __fmaf_rn(a, s_par[3 * NC + co], zh);
                             }
+                            if (TRAIN)
+#pragma unroll
+                                for (int hc = 0; hc < 2; hc++)
+                                    *reinterpret_cast<uint4 *>(a3g + act_at(tile, 8 * hc, vox)) =
+                                        reinterpret_cast<const uint4 *>(a3)[hc];
                             const float p = 1.0f / (1.0f + expf(-zh));
                             if (HALF) {
                                 if (2 * tile + b < count) {
@@ -1178,7 +1479,7 @@ static int mn_cuda(const char *what, cudaError_t e)
 MaskNet::~MaskNet()
 {
     for (void *p : {(void *)master_, (void *)used_, (void *)m_, (void *)v_, (void *)gpart_, (void *)a1_, (void *)a2_,
-                    (void *)a3_, (void *)p_, (void *)dz_, (void *)scal_, (void *)grad_, (void *)img_, (void *)err_})
+                    (void *)a3_, (void *)p_, (void *)scal_, (void *)grad_, (void *)img_, (void *)err_})
         if (p) cudaFree(p);
 }
 
@@ -1191,16 +1492,15 @@ int MaskNet::init()
     cudaMemset(m_, 0, pb);
     cudaMemset(v_, 0, pb);
     if ((e = cudaMalloc(&scal_, 2 * sizeof(double))) != cudaSuccess) return mn_cuda("cudaMalloc", e);
-    if ((e = cudaMalloc(&img_, mn::IMG_BYTES)) != cudaSuccess) return mn_cuda("cudaMalloc", e);
+    if ((e = cudaMalloc(&img_, mn::IMG_BYTES + 2 * mn::kWFragBytes)) != cudaSuccess) return mn_cuda("cudaMalloc", e);
     if ((e = cudaMalloc(&err_, sizeof(int))) != cudaSuccess) return mn_cuda("cudaMalloc", e);
     cudaMemset(err_, 0, sizeof(int));
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     grid_ = sms > 0 ? sms : 1;
-    if ((e = cudaMalloc(&gpart_, sizeof(float) * mn::NPARAM * (size_t)grid_)) != cudaSuccess)
+    if ((e = cudaMalloc(&gpart_, sizeof(float) * mn::NPARAM * 2 * (size_t)grid_)) != cudaSuccess)
         return mn_cuda("cudaMalloc", e);
-    cudaMemset(gpart_, 0, sizeof(float) * mn::NPARAM * (size_t)grid_);
     static bool attr[64] = {};
     if (dev >= 0 && dev < 64 && !attr[dev]) {
         const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -1280,17 +1580,16 @@ int MaskNet::forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8
 int MaskNet::ensure_batch(long long ntiles)
 {
     if (ntiles <= cap_) return 0;
-    for (void *p : {(void *)a1_, (void *)a2_, (void *)a3_, (void *)p_, (void *)dz_})
+    for (void *p : {(void *)a1_, (void *)a2_, (void *)a3_, (void *)p_})
         if (p) cudaFree(p);
     a1_ = a2_ = a3_ = nullptr;
-    p_ = dz_ = nullptr;
+    p_ = nullptr;
     cap_ = 0;
     cudaError_t e;
     const size_t act = sizeof(uint16_t) * mn::NC * mn::NV * (size_t)ntiles;
     if ((e = cudaMalloc(&a1_, act)) != cudaSuccess || (e = cudaMalloc(&a2_, act)) != cudaSuccess ||
         (e = cudaMalloc(&a3_, act)) != cudaSuccess ||
-        (e = cudaMalloc(&p_, sizeof(float) * mn::NV * (size_t)ntiles)) != cudaSuccess ||
-        (e = cudaMalloc(&dz_, sizeof(float) * mn::NV * (size_t)ntiles)) != cudaSuccess)
+        (e = cudaMalloc(&p_, sizeof(float) * mn::NV * (size_t)ntiles)) != cudaSuccess)
         return mn_cuda("training buffers", e);
     cap_ = ntiles;
     return 0;
@@ -1316,17 +1615,17 @@ int MaskNet::train_step(const uint16_t *d_feat, const float2 *d_ac, long long nt
             (__nv_bfloat16 *)a3_);
     const long long n = ntiles * mn::NV;
     mn::mn_sum_kernel<<<256, 256, 0, s>>>(d_ac, n, scal_);
-    mn::mn_loss_kernel<<<256, 256, 0, s>>>(p_, d_ac, n, scal_, dz_, scal_ + 1);
-    mn::mn_backward_kernel<<<blocks, mn::kThreads, mn::kBwdSmem, s>>>(
-        used_, d_feat, (const __nv_bfloat16 *)a1_, (const __nv_bfloat16 *)a2_, (const __nv_bfloat16 *)a3_, dz_,
-        ntiles, gpart_);
+    const unsigned slices = (unsigned)std::min<long long>(ntiles, 2 * (long long)grid_);
+    mn::mn_backward_kernel<<<slices, mn::kBwdThreads, mn::kBwdSmem, s>>>(
+        used_, img_ + mn::IMG_BYTES, d_feat, (const __nv_bfloat16 *)a1_, (const __nv_bfloat16 *)a2_,
+        (const __nv_bfloat16 *)a3_, p_, d_ac, scal_, ntiles, gpart_, scal_ + 1);
     float c1 = 1.f, c2 = 1.f;
     if (lr > 0.f) {
         step_++;
         c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)step_)));
         c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)step_)));
     }
-    mn::mn_adam_kernel<<<(mn::NPARAM + 255) / 256, 256, 0, s>>>(master_, used_, m_, v_, gpart_, (int)blocks, lr, 0.9f,
+    mn::mn_adam_kernel<<<(mn::NPARAM + 31) / 32, 256, 0, s>>>(master_, used_, m_, v_, gpart_, (int)slices, lr, 0.9f,
                                                                0.999f, 1e-8f, c1, c2, grad_);
     if (lr > 0.f)
         if (const int rc = build_images(s); rc != 0) return rc;

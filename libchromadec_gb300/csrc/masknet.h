@@ -44,7 +44,7 @@ private:
     float *gpart_ = nullptr;
     double *scal_ = nullptr;
     uint16_t *a1_ = nullptr, *a2_ = nullptr, *a3_ = nullptr;
-    float *p_ = nullptr, *dz_ = nullptr;
+    float *p_ = nullptr;
     long long cap_ = 0;
     int grid_ = 1;
     long long step_ = 0;
