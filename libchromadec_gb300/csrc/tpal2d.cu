@@ -9,16 +9,25 @@
 // within the threshold ratio, for x in [4, 8]; inverse DFT / 512 and
 // overlap-add into the active window. GPU structure:
 //
-//  * one warp per tile: lanes (h, i) hold row i; half-warp h = 0 computes
-//    bins kx 4..8, h = 1 bins 9..12 -- the only bins the filter can keep;
+//  * one warp per tile position of a frame's two fields, packed in the halves
+//    of f32x2 registers through the Y stages: lane (j, i) holds row i of field
+//    j and computes its bins kx 4..12, the only ones the filter can keep;
 //  * black and each row's mean are subtracted first (they only touch bins
 //    kx in {0, +-1} of the windowed row), so invalid rows are exact zeros;
-//  * the 16-point Y DFT is a shuffle FFT across the half-warp;
-//  * decisions are FP32 with a per-kx error bound; decisions inside it are
-//    recomputed in double-float from the raw samples by the whole warp;
+//  * the 16-point Y DFTs run as two radix-4 passes, four lanes a column, with
+//    exchanges through shared memory (as in the 3D walk): eight columns on the
+//    32 lanes, then the ninth;
+//  * for the decisions lane (j, ky) owns the bins (kx 4..8, ky) of field j and
+//    reads their mirrors; decisions are FP32 with a per-kx error bound, those
+//    inside it recomputed in double-float from the raw samples by the whole
+//    warp; both bins of a pair are masked in place;
 //  * overlap-add: tiles of one (tileY parity, tileX parity) class tile the
 //    active area without overlap, so each class writes its own partial plane
 //    (the same layout the 3D kernel writes, read by the demodulator).
+//
+// One field a warp, with the two half-warps splitting kx, DFTs by shuffles and
+// 16-bit row loads, took 1,866 warp instructions a tile at 46 % issue active:
+// 2.17 ms for 300 fields. This form: see tp2_launch.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -29,13 +38,10 @@
 
 namespace tpal {
 
-__constant__ float c2_cwx[9][16];   // w32(x) cos(theta), theta = 2 pi kx (x - 15.5)/32, kx = 4..12, x < 16
-__constant__ float c2_swx[9][16];   // w32(x) sin(theta)
-__constant__ float c2_cix[9][16];   // (2/512) cos(theta)
-__constant__ float c2_six[9][16];   // (2/512) sin(theta)
-// the same as pairs for the f32x2 instructions: (cwx, -swx) and (cix, six)
-__constant__ float2 c2_xf[9][16];
-__constant__ float2 c2_xi[9][16];
+// X-stage tables as pairs for the f32x2 instructions, theta = 2 pi kx (x - 15.5)/32,
+// kx = 4..12, x < 16:
+__constant__ float2 c2_xf[9][16];   // w32(x) (cos theta, -sin theta)
+__constant__ float2 c2_xi[9][16];   // (2/512) (cos theta, sin theta)
 __constant__ float c2_wx[16];       // w32(x), x < 16
 __constant__ float c2_wy[16];       // w16(i)
 __constant__ float2 c2_tw16[16];    // exp(-2 pi i r/16)
@@ -48,18 +54,6 @@ static bool g_tp2_ready[64];
 constexpr int kWarps2 = 4;
 constexpr float kBound2 = 2.0f;
 constexpr float kEps = 5.9604645e-8f;
-
-__device__ __forceinline__ float2 cmul2(float2 a, float2 b)
-{
-    return make_float2(__fmaf_rn(a.x, b.x, -a.y * b.y), __fmaf_rn(a.x, b.y, a.y * b.x));
-}
-
-__device__ __forceinline__ float2 shx(float2 v, int m)
-{
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
-}
-
-__device__ __forceinline__ float l1f(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 
 struct Thr2 {
     float f;
@@ -135,236 +129,333 @@ __device__ __forceinline__ bool df_sim2(df a, df b, df t)
     return !(df_sign(d1) < 0 || df_sign(d2) < 0);
 }
 
-template <bool PER_BIN>
-__global__ void __launch_bounds__(32 * kWarps2) tpal2d_kernel(T2Params P)
+// Shared memory per warp (float4 units): two buffers [9 kx][16 positions],
+// rows of 20, and the bound terms [9][2 fields]. Position p of 16 is stored at
+// p ^ (p >> 2) where four lanes hold four neighbours each (see tpal3d.cu).
+constexpr int kBuf2 = 9 * 20;
+constexpr int kWarpF4_2 = 2 * kBuf2 + 5;
+constexpr int kTw2 = 4 * 5;   // Y twiddles per quarter r: three (x, x, y, y), three (-y, -y)
+constexpr int kBlocks2 = 5;   // resident blocks a SM
+
+__device__ __forceinline__ tw2 twiddle2(const float4 *tw, int r, int v)
 {
+    const float4 a = tw[5 * r + v];
+    return {make_float2(a.x, a.y), make_float2(a.z, a.w), reinterpret_cast<const float2 *>(tw + 5 * r + 3)[v]};
+}
+
+// Forward Y stage of one column (16 rows in `x` to 16 bins in `s`, position p
+// holding bin rev4(p)) and the L1 norms of its rows, by the four lanes r of
+// `mask`'s groups.
+__device__ __forceinline__ void y_forward2(const float4 *x, float4 *ex, float4 *s, float2 *bound, const float4 *tw,
+                                           int r, unsigned mask)
+{
+    cp2 a[4];
+#pragma unroll
+    for (int n = 0; n < 4; n++) a[n] = cp_of(x[r + 4 * n]);
+    float A0 = 0.f, A1 = 0.f;
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+        A0 += fabsf(a[n].re.x) + fabsf(a[n].im.x);
+        A1 += fabsf(a[n].re.y) + fabsf(a[n].im.y);
+    }
+#pragma unroll
+    for (int h = 1; h < 4; h <<= 1) {
+        A0 += __shfl_xor_sync(mask, A0, h);
+        A1 += __shfl_xor_sync(mask, A1, h);
+    }
+    if (r == 0) *bound = make_float2(A0, A1);
+    const cp2 u0 = cadd(a[0], a[2]), u1 = cadd(a[1], a[3]);
+    const cp2 v0 = ctw(csub(a[0], a[2]), twiddle2(tw, r, 0), false), v1 = ctw(csub(a[1], a[3]), twiddle2(tw, r, 1), false);
+    const tw2 t2 = twiddle2(tw, r, 2);
+    ex[0 + r] = f4_of(cadd(u0, u1));
+    ex[4 + (r ^ 1)] = f4_of(ctw(csub(u0, u1), t2, false));
+    ex[8 + (r ^ 2)] = f4_of(cadd(v0, v1));
+    ex[12 + (r ^ 3)] = f4_of(ctw(csub(v0, v1), t2, false));
+    __syncwarp(mask);
+#pragma unroll
+    for (int n = 0; n < 4; n++) a[n] = cp_of(ex[4 * r + (n ^ r)]);
+    const cp2 w0 = cadd(a[0], a[2]), w1 = cadd(a[1], a[3]), w2 = csub(a[0], a[2]), d3 = csub(a[1], a[3]);
+    s[4 * r + (0 ^ r)] = f4_of(cadd(w0, w1));
+    s[4 * r + (1 ^ r)] = f4_of(csub(w0, w1));
+    s[4 * r + (2 ^ r)] = f4_of({add2(w2.re, d3.im), sub2(w2.im, d3.re)});   // odd branch times -i
+    s[4 * r + (3 ^ r)] = f4_of({sub2(w2.re, d3.im), add2(w2.im, d3.re)});
+}
+
+// Inverse Y stage of one column: 16 bins in `s` (bit-reversed) to 16 rows in `x`.
+__device__ __forceinline__ void y_inverse2(const float4 *s, float4 *ex, float4 *x, const float4 *tw, int r, unsigned mask)
+{
+    cp2 G[4];
+#pragma unroll
+    for (int n = 0; n < 4; n++) G[n] = cp_of(s[4 * r + (n ^ r)]);
+    const cp2 w0 = cadd(G[0], G[1]), w1 = csub(G[0], G[1]), w2 = cadd(G[2], G[3]), d3 = csub(G[2], G[3]);
+    ex[4 * r + (0 ^ r)] = f4_of(cadd(w0, w2));
+    ex[4 * r + (2 ^ r)] = f4_of(csub(w0, w2));
+    ex[4 * r + (1 ^ r)] = f4_of({sub2(w1.re, d3.im), add2(w1.im, d3.re)});   // odd branch times +i
+    ex[4 * r + (3 ^ r)] = f4_of({add2(w1.re, d3.im), sub2(w1.im, d3.re)});
+    __syncwarp(mask);
+#pragma unroll
+    for (int n = 0; n < 4; n++) G[n] = cp_of(ex[4 * n + (r ^ n)]);
+    const tw2 t2 = twiddle2(tw, r, 2);
+    const cp2 f1 = ctw(G[1], t2, true), f3 = ctw(G[3], t2, true);
+    const cp2 g0 = cadd(G[0], f1), g1 = csub(G[0], f1);
+    const cp2 g2 = ctw(cadd(G[2], f3), twiddle2(tw, r, 0), true), g3 = ctw(csub(G[2], f3), twiddle2(tw, r, 1), true);
+    x[r] = f4_of(cadd(g0, g2));
+    x[r + 4] = f4_of(cadd(g1, g3));
+    x[r + 8] = f4_of(csub(g0, g2));
+    x[r + 12] = f4_of(csub(g1, g3));
+}
+
+template <bool PER_BIN>
+__global__ void __launch_bounds__(32 * kWarps2, kBlocks2) tpal2d_kernel(T2Params P)
+{
+    __shared__ float4 s_buf[kWarps2 * kWarpF4_2];
+    __shared__ float4 s_tw[kTw2];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int h = lane >> 4, i = lane & 15;
+    const int j = lane >> 4, i = lane & 15;
+    float4 *bx = s_buf + warp * kWarpF4_2, *be = bx + kBuf2;   // rows and spectra; exchanges
+    float *bnd = reinterpret_cast<float *>(be + kBuf2);        // [9][2]: A per kx and field
+    for (int e = threadIdx.x; e < 12; e += blockDim.x) {
+        const int r = e / 3, v = e % 3;
+        const float2 w = c2_tw16[v == 0 ? r : v == 1 ? r + 4 : 2 * r];
+        s_tw[5 * r + v] = make_float4(w.x, w.x, w.y, w.y);
+        reinterpret_cast<float2 *>(s_tw + 5 * r + 3)[v] = make_float2(-w.y, -w.y);
+    }
+    __syncthreads();
     const int tileX0 = P.avs - 16;
     const int ntx = (P.ave - tileX0 + 15) / 16;
     // tile rows: the larger of the two field parities' grids
     const int nty = max((((P.lafl - 0) / 2 + 1) - ((P.fafl + 1 - 0) / 2 - 8) + 7) / 8,
                         (((P.lafl - 1) / 2 + 1) - ((P.fafl + 1 - 1) / 2 - 8) + 7) / 8);
-    const long long item = (long long)blockIdx.x * kWarps2 + warp;
-    const long long per_field = (long long)ntx * nty;
-    if (item >= per_field * P.nout) return;
-    const int o = (int)(item / per_field);
-    const int t = (int)(item % per_field);
+    const int per_frame = ntx * nty;
+    const unsigned nitems = (unsigned)per_frame * (unsigned)(P.nout >> 1);
+    const float wy = c2_wy[i];
+    const int ky = rev4(i), kyr = (8 - ky) & 15;
+    const int at = i ^ (i >> 2), atr = rev4(kyr) ^ (rev4(kyr) >> 2);   // positions of ky and its mirror
+    unsigned n_exact = 0, n_flip = 0;
+    for (unsigned item = blockIdx.x * kWarps2 + warp; item < nitems; item += gridDim.x * kWarps2) {
+    const int o = 2 * (int)(item / per_frame) + j;   // this lane's field (nout is even: whole frames)
+    const int t = (int)(item % per_frame);
     const int tx = t % ntx, ty = t / ntx;
     const int f = P.field_begin + o;
     const int off = (f & 1) ^ P.swap;   // SourceField::getOffset
     const int fl_first = (P.fafl + 1 - off) / 2;   // SourceField::getFirstActiveLine
     const int fl_last = ((P.lafl - off) / 2) + 1;  // SourceField::getLastActiveLine
     const int tileY = fl_first - 8 + 8 * ty;
-    if (tileY >= fl_last) return;
     const int tileX = tileX0 + 16 * tx;
     const int cls = ((ty & 1) << 1) | (tx & 1);
-    const int nk = h ? 4 : 5;     // bins kx 4..8 (h = 0) or 9..12 (h = 1)
-    const int kbase = h ? 5 : 0;  // index into the kx = 4..12 tables
-
-    // --- forward X: row i, DC/black removed, folded about the window centre
     const int fl = tileY + i;
     const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
-    const bool valid = (fp != nullptr) && (fl >= fl_first) && (fl < fl_last);
-    float2 sd[16];   // (s_x, d_x)
+    const bool inside = fl >= fl_first && fl < fl_last;
+    // a black gap frame of a batch: nothing reads its planes
+    if (P.field_ptrs != nullptr && !__any_sync(0xffffffffu, fp != nullptr)) continue;
+
+    // --- forward X: this lane's row, DC/black removed, folded about the window
+    // centre: (s_x, d_x) = (a_x + a_31-x - 2 mean, a_x - a_31-x), exact in FP32
+    float2 sd[16];
     float rowl1 = 0.f;
-    if (valid) {
-        const uint16_t *row = fp + (long long)fl * P.fw;
-        int a[32];
-        int sum = 0;
+    if (fp != nullptr && inside) {
+        uint32_t v[16];   // samples 2k, 2k+1
+        if (tileX >= 0 && fl >= 1 && (fl + 1 < P.fh || tileX + 34 <= P.fw)) {
+            // rows start on any 2-byte boundary: 17 aligned words cover the 32
+            // samples, inside the field, and a funnel shift lines them up
+            const uintptr_t pa = reinterpret_cast<uintptr_t>(fp + fl * P.fw + tileX);
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
+            const unsigned sh = (unsigned)(pa & 2) * 8u;
+            uint32_t w0 = __ldg(w);
 #pragma unroll
-        for (int x = 0; x < 32; x++) {
-            const int xx = max(tileX + x, -fl * P.fw);
-            a[x] = (int)__ldg(row + xx) - P.black;
-            sum += a[x];
-        }
-        const float m32 = (float)sum * 0.03125f;
+            for (int k = 0; k < 16; k++) {
+                const uint32_t w1 = __ldg(w + k + 1);
+                v[k] = __funnelshift_r(w0, w1, sh);
+                w0 = w1;
+            }
+        } else {
 #pragma unroll
-        for (int x = 0; x < 16; x++) {
-            sd[x] = make_float2((float)(16 * (a[x] + a[31 - x]) - sum) * 0.0625f,   // a_x + a_31-x - 2 mean (exact)
-                                (float)(a[x] - a[31 - x]));
-            rowl1 = __fmaf_rn(c2_wx[x], fabsf((float)a[x] - m32) + fabsf((float)a[31 - x] - m32), rowl1);
+            for (int k = 0; k < 16; k++) {   // never before the field start
+                const uint16_t *row = fp + fl * P.fw;
+                v[k] = (uint32_t)__ldg(row + max(tileX + 2 * k, -fl * P.fw)) |
+                       ((uint32_t)__ldg(row + max(tileX + 2 * k + 1, -fl * P.fw)) << 16);
+            }
         }
+        // 2^23 + a from the sample's bits; subtracting 2^24 from one side of
+        // each sum leaves a_x + a_31-x exactly
+        float2 tt[8];
+        float2 u = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float2 p = make_float2(__uint_as_float(__byte_perm(v[k], 0x4B000000u, 0x7610)),
+                                         __uint_as_float(__byte_perm(v[k], 0x4B000000u, 0x7632)));
+            const float2 q = make_float2(__uint_as_float(__byte_perm(v[15 - k], 0x4B000000u, 0x7632)),
+                                         __uint_as_float(__byte_perm(v[15 - k], 0x4B000000u, 0x7610)));
+            sd[2 * k].y = __fsub_rn(p.x, q.x);
+            sd[2 * k + 1].y = __fsub_rn(p.y, q.y);
+            tt[k] = add2(add2(p, make_float2(-16777216.f, -16777216.f)), q);
+            u = add2(u, tt[k]);   // sums of 32 samples: exact
+        }
+        const float mean2 = __fmul_rn(__fadd_rn(u.x, u.y), 0.0625f);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            sd[2 * k].x = __fsub_rn(tt[k].x, mean2);
+            sd[2 * k + 1].x = __fsub_rn(tt[k].y, mean2);
+        }
+        // |a_x - mean| + |a_31-x - mean| = max(|s_x|, |d_x|)
+#pragma unroll
+        for (int x = 0; x < 16; x++) rowl1 = __fmaf_rn(c2_wx[x], fmaxf(fabsf(sd[x].x), fabsf(sd[x].y)), rowl1);
     } else {
 #pragma unroll
         for (int x = 0; x < 16; x++) sd[x] = make_float2(0.f, 0.f);
     }
-    const float wy = c2_wy[i];
     rowl1 *= wy;
 #pragma unroll
     for (int m = 1; m < 16; m <<= 1) rowl1 += __shfl_xor_sync(0xffffffffu, rowl1, m);
-
-    // per-lane FFT twiddles (DIF stages h = 8, 4, 2, 1)
-    float2 tw[4];
     {
-        int s = 0;
+        // rows 8..15 write their imaginary part first: 32 different banks a store
+        const bool upper = i >= 8;
+        float *xr = reinterpret_cast<float *>(bx) + 4 * i + j;
+        float *xs = xr + (upper ? 2 : 0), *xt = xr + (upper ? 0 : 2);
 #pragma unroll
-        for (int hh = 8; hh >= 1; hh >>= 1, s++) tw[s] = c2_tw16[(i & (hh - 1)) * (8 / hh)];
+        for (int k = 0; k < 9; k++) {
+            float2 X = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int x = 0; x < 16; x++) X = __ffma2_rn(c2_xf[k][x], sd[x], X);
+            X = __fmul2_rn(X, make_float2(wy, wy));
+            xs[80 * k] = upper ? X.y : X.x;
+            xt[80 * k] = upper ? X.x : X.y;
+        }
     }
+    __syncwarp();
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++)
+        if (pass == 0 || lane < 4) {
+            const int k = pass == 0 ? lane >> 2 : 8;
+            y_forward2(bx + 20 * k, be + 20 * k, bx + 20 * k, reinterpret_cast<float2 *>(bnd) + k, s_tw, lane & 3,
+                       pass == 0 ? 0xffffffffu : 0xFu);
+        }
+    __syncwarp();
 
-    float2 Y[5];
-    float E[5];
-    // Every lane runs all five bins (the shuffles below need the whole
-    // warp); half-warp 1 has only four, its fifth is a zero dummy.
+    // --- decisions: lane (j, ky), bins A = (kx 4 + k, ky) and their mirrors
+    // B = (kx 12 - k, kyr)
+    const float *sa = reinterpret_cast<const float *>(bx + at) + j, *sr = reinterpret_cast<const float *>(bx + atr) + j;
+    float2 A[5], B[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        const bool real = k < nk;
-        const int row = real ? kbase + k : 8;
-        float2 X = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int x = 0; x < 16; x++) {
-            X = __ffma2_rn(c2_xf[row][x], sd[x], X);   // (cwx sx + .., -swx dx + ..)
-        }
-        const float wk = real ? wy : 0.f;
-        X.x *= wk;
-        X.y *= wk;
-        float A = l1f(X);
-#pragma unroll
-        for (int m = 1; m < 16; m <<= 1) A += __shfl_xor_sync(0xffffffffu, A, m);
-        E[k] = kBound2 * kEps * (A + 0.5f * rowl1);
-        // 16-point DFT over rows (DIF; lane i ends with bin rev4(i))
-        int s = 0;
-#pragma unroll
-        for (int hh = 8; hh >= 1; hh >>= 1, s++) {
-            const bool upper = (i & hh) != 0;
-            const float2 ov = shx(X, hh);
-            X = upper ? cmul2(sub2(ov, X), tw[s]) : add2(X, ov);
-        }
-        Y[k] = X;
+        A[k] = make_float2(sa[80 * k], sa[80 * k + 2]);
+        B[k] = make_float2(sr[80 * (8 - k)], sr[80 * (8 - k) + 2]);
     }
-    const int ky = rev4(i);
-    const int kyr = (8 - ky) & 15;
-    // half-0 lane (ky) pairs with half-1 lane rev4(kyr) for kx 4..7, and with
-    // half-0 lane rev4(kyr) for kx 8.
-    const int mirror_other = 16 + rev4(kyr);
-    const int mirror_same = rev4(kyr);
-    float mag[5], ab[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        mag[k] = __fmaf_rn(Y[k].x, Y[k].x, Y[k].y * Y[k].y);
-        ab[k] = l1f(Y[k]);
-    }
-    // Mirror data: for my bin kx (h = 0, k < 4) the mirror is kx' = 16 - kx,
-    // index k' = 3 - k in half 1; for kx = 8 (k = 4) it is k = 4 in half 0.
-    float rm[5], ra[5], rE[5];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int src = (h == 0) ? mirror_other : 0;
-        rm[k] = __shfl_sync(0xffffffffu, mag[3 - k], src);
-        ra[k] = __shfl_sync(0xffffffffu, ab[3 - k], src);
-        rE[k] = __shfl_sync(0xffffffffu, E[3 - k], src);
-    }
-    rm[4] = __shfl_sync(0xffffffffu, mag[4], mirror_same);
-    ra[4] = __shfl_sync(0xffffffffu, ab[4], mirror_same);
-    rE[4] = __shfl_sync(0xffffffffu, E[4], mirror_same);
-
+    const float tf = (P.frame_t2 != nullptr) ? P.frame_t2[3 * (f >> 1)] : P.t2f;
     unsigned keep = 0, unc = 0;
-    if (h == 0) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-            const int kx = 4 + k;
-            const bool self = (kx == 8) && (ky == kyr);
-            const float a = mag[k], b = rm[k];
-            const float pa = 2.f * E[k] * ab[k] + E[k] * E[k];
-            const float pb = 2.f * rE[k] * ra[k] + rE[k] * rE[k];
-            float tt = (P.frame_t2 != nullptr) ? P.frame_t2[3 * (f >> 1)] : P.t2f;
-            if (PER_BIN) tt = thr2(P, f >> 1, ky, kx).f;
-            bool sm = sim2(a, b, tt);
-            bool u = unc2(a, b, tt, pa, pb);
-            if (PER_BIN && kx == 8) {   // the mirror (also kx 8) visits with its own threshold
-                const float t2 = thr2(P, f >> 1, kyr, 8).f;
-                sm |= sim2(a, b, t2);
-                u |= unc2(a, b, t2, pa, pb);
-            }
-            if (sm || self) keep |= 1u << k;
-            if (u && !self) unc |= 1u << k;
+    for (int k = 0; k < 5; k++) {
+        const float Ea = kBound2 * kEps * (bnd[2 * k + j] + 0.5f * rowl1);
+        const float Eb = kBound2 * kEps * (bnd[2 * (8 - k) + j] + 0.5f * rowl1);
+        const bool self = (k == 4) && (ky == kyr);
+        const float a = __fmaf_rn(A[k].x, A[k].x, __fmul_rn(A[k].y, A[k].y));
+        const float b = __fmaf_rn(B[k].x, B[k].x, __fmul_rn(B[k].y, B[k].y));
+        const float pa = 2.f * Ea * l1(A[k]) + Ea * Ea;
+        const float pb = 2.f * Eb * l1(B[k]) + Eb * Eb;
+        float tt = tf;
+        if (PER_BIN) tt = thr2(P, f >> 1, ky, 4 + k).f;
+        bool sm = sim2(a, b, tt);
+        bool u = unc2(a, b, tt, pa, pb);
+        if (PER_BIN && k == 4) {   // the mirror (also kx 8) visits with its own threshold
+            const float t2 = thr2(P, f >> 1, kyr, 8).f;
+            sm |= sim2(a, b, t2);
+            u |= unc2(a, b, t2, pa, pb);
         }
+        if (sm || self) keep |= 1u << k;
+        if (u && !self) unc |= 1u << k;
     }
-    unsigned n_exact = 0, n_flip = 0;
     unsigned any = __ballot_sync(0xffffffffu, unc != 0);
     while (any) {
         const int src = __ffs(any) - 1;
         const unsigned su = __shfl_sync(0xffffffffu, unc, src);
         const int k = __ffs(su) - 1;
         const int kyb = rev4(src & 15), kxb = 4 + k;
+        const int fs = __shfl_sync(0xffffffffu, f, src), ys = __shfl_sync(0xffffffffu, tileY, src);
+        const int first = __shfl_sync(0xffffffffu, fl_first, src), last = __shfl_sync(0xffffffffu, fl_last, src);
         df mb, mr;
-        exact_pair2(P, f, tileX, tileY, fl_first, fl_last, kyb, kxb, mb, mr);
+        exact_pair2(P, fs, tileX, ys, first, last, kyb, kxb, mb, mr);
         const int kybr = (8 - kyb) & 15;
-        bool sm = df_sim2(mb, mr, thr2(P, f >> 1, kyb, kxb).d);
-        if (kxb == 8) sm |= df_sim2(mb, mr, thr2(P, f >> 1, kybr, 8).d);
+        bool sm = df_sim2(mb, mr, thr2(P, fs >> 1, kyb, kxb).d);
+        if (kxb == 8) sm |= df_sim2(mb, mr, thr2(P, fs >> 1, kybr, 8).d);
         if (lane == src) {
             n_exact++;
             if ((((keep >> k) & 1u) != 0) != sm) n_flip++;
             keep = sm ? (keep | (1u << k)) : (keep & ~(1u << k));
             unc &= ~(1u << k);
         }
-        if (kxb == 8 && lane == rev4(kybr)) {   // the kx-8 mirror is a visitor too
+        if (kxb == 8 && lane == ((src & 16) | rev4(kybr))) {   // the kx-8 mirror is a visitor too
             keep = sm ? (keep | (1u << 4)) : (keep & ~(1u << 4));
             unc &= ~(1u << 4);
         }
         any = __ballot_sync(0xffffffffu, unc != 0);
     }
-    // Half 1 bins (kx 9..12, index k) are kept when their mirror (kx 16-kx,
-    // index 3-k, on half-0 lane rev4(kyr)) was kept.
+    // both bins of each pair, masked in place (kx 8's mirrors are other lanes' A)
+    __syncwarp();
     {
-        const unsigned mk = __shfl_sync(0xffffffffu, keep, rev4(kyr));
-        if (h == 1) {
-            keep = 0;
+        float *wa = reinterpret_cast<float *>(bx + at) + j, *wr = reinterpret_cast<float *>(bx + atr) + j;
 #pragma unroll
-            for (int k = 0; k < 4; k++) keep |= ((mk >> (3 - k)) & 1u) << k;
+        for (int k = 0; k < 5; k++) {
+            const float m = ((keep >> k) & 1u) ? 1.f : 0.f;
+            wa[80 * k] = A[k].x * m;
+            wa[80 * k + 2] = A[k].y * m;
+            if (k < 4) {
+                wr[80 * (8 - k)] = B[k].x * m;
+                wr[80 * (8 - k) + 2] = B[k].y * m;
+            }
         }
     }
+    __syncwarp();
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++)
+        if (pass == 0 || lane < 4) {
+            const int k = pass == 0 ? lane >> 2 : 8;
+            y_inverse2(bx + 20 * k, be + 20 * k, bx + 20 * k, s_tw, lane & 3, pass == 0 ? 0xffffffffu : 0xFu);
+        }
+    __syncwarp();
 
-    // --- inverse Y (DIT, bit-reversed in -> natural rows out) and X partial sums
-    float2 CS[16];   // (cosine sum, sine sum)
+    // --- inverse X of this lane's row: kx 4..8 and kx 9..12 summed apart, then added
+    if (inside) {
+        float2 G[9];
+        const float *gr = reinterpret_cast<const float *>(bx) + 4 * i + j;
 #pragma unroll
-    for (int x = 0; x < 16; x++) CS[x] = make_float2(0.f, 0.f);
+        for (int k = 0; k < 9; k++) G[k] = make_float2(gr[80 * k], gr[80 * k + 2]);
+        float v[32];
 #pragma unroll
-    for (int k = 0; k < 5; k++) {   // all lanes, all five bins (shuffles); half 1's fifth is zero
-        const int row = (k < nk) ? kbase + k : 8;
-        float2 G = (((keep >> k) & 1u) && k < nk) ? Y[k] : make_float2(0.f, 0.f);
-        int s = 3;
+        for (int x = 0; x < 16; x++) {
+            float2 c = make_float2(0.f, 0.f), d = c;
 #pragma unroll
-        for (int hh = 1; hh <= 8; hh <<= 1, s--) {
-            const bool upper = (i & hh) != 0;
-            const float2 w = make_float2(tw[s].x, -tw[s].y);
-            const float2 ov = shx(G, hh);
-            const float2 tt = cmul2(upper ? G : ov, w);
-            G = upper ? sub2(ov, tt) : add2(G, tt);
+            for (int k = 0; k < 5; k++) c = __ffma2_rn(G[k], c2_xi[k][x], c);
+#pragma unroll
+            for (int k = 5; k < 9; k++) d = __ffma2_rn(G[k], c2_xi[k][x], d);
+            c = add2(c, d);   // (cosine sum, sine sum)
+            v[x] = c.x - c.y;
+            v[31 - x] = c.x + c.y;
         }
-#pragma unroll
-        for (int x = 0; x < 16; x++) CS[x] = __ffma2_rn(G, c2_xi[row][x], CS[x]);
-    }
-#pragma unroll
-    for (int x = 0; x < 16; x++) CS[x] = add2(CS[x], shx(CS[x], 16));
-    if (fl >= fl_first && fl < fl_last) {
         float *dst = P.partial + (long long)cls * P.part_class_stride + (long long)o * P.part_field_stride +
                      (long long)(fl - P.fl_lo) * P.part_row_stride - P.avs;
-        // this lane's 16 samples [tileX + 16 h, +16): tileX - avs is a multiple
-        // of 16, so inside the active window they start on a 64-byte boundary
-        // whenever the planes' strides are multiples of 4 floats and their
-        // base is 16-byte aligned: four vector stores
-        const int x0 = tileX + 16 * h;
+        // tileX - avs is a multiple of 16, so inside the active window each half
+        // row starts on a 64-byte boundary whenever the planes' strides are
+        // multiples of 4 floats and their base is 16-byte aligned: four vector
+        // stores a half
         const bool vec = ((P.part_row_stride | P.part_field_stride | P.part_class_stride) & 3) == 0 &&
-                         (reinterpret_cast<uintptr_t>(P.partial) & 15) == 0 && x0 >= P.avs && x0 + 16 <= P.ave;
-        if (vec) {
-            float v[16];
+                         (reinterpret_cast<uintptr_t>(P.partial) & 15) == 0;
 #pragma unroll
-            for (int x = 0; x < 16; x++) {
-                if (h) v[15 - x] = CS[x].x + CS[x].y;
-                else v[x] = CS[x].x - CS[x].y;
-            }
-            float4 *d4 = reinterpret_cast<float4 *>(dst + x0);
+        for (int h = 0; h < 2; h++) {
+            const int x0 = tileX + 16 * h;
+            if (vec && x0 >= P.avs && x0 + 16 <= P.ave) {
+                float4 *d4 = reinterpret_cast<float4 *>(dst + x0);
 #pragma unroll
-            for (int q = 0; q < 4; q++) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        } else {
+                for (int q = 0; q < 4; q++)
+                    d4[q] = make_float4(v[16 * h + 4 * q], v[16 * h + 4 * q + 1], v[16 * h + 4 * q + 2], v[16 * h + 4 * q + 3]);
+            } else {
 #pragma unroll
-            for (int x = 0; x < 16; x++) {
-                const int X = h ? tileX + 31 - x : tileX + x;
-                if (X >= P.avs && X < P.ave) dst[X] = h ? CS[x].x + CS[x].y : CS[x].x - CS[x].y;
+                for (int x = 0; x < 16; x++)
+                    if (x0 + x >= P.avs && x0 + x < P.ave) dst[x0 + x] = v[16 * h + x];
             }
         }
+    }
+    __syncwarp();   // the next item reuses the buffers
     }
     if (P.stats != nullptr) {
         if (n_exact) atomicAdd(P.stats + 0, n_exact);
@@ -413,10 +504,6 @@ int tp2_init_constants(int device)
     }
 #define TP2_CPY(sym, src) \
     if (cudaMemcpyToSymbol(sym, src, sizeof(src)) != cudaSuccess) return -1;
-    TP2_CPY(c2_cwx, cwx);
-    TP2_CPY(c2_swx, swx);
-    TP2_CPY(c2_cix, cix);
-    TP2_CPY(c2_six, six);
     float2 xf[9][16], xi[9][16];
     for (int k = 0; k < 9; k++)
         for (int x = 0; x < 16; x++) {
@@ -442,9 +529,16 @@ int tp2_launch(const T2Params &P, cudaStream_t stream)
     const int ntx = (P.ave - tileX0 + 15) / 16;
     const int nty = std::max((((P.lafl - 0) / 2 + 1) - ((P.fafl + 1 - 0) / 2 - 8) + 7) / 8,
                              (((P.lafl - 1) / 2 + 1) - ((P.fafl + 1 - 1) / 2 - 8) + 7) / 8);
-    const long long items = (long long)ntx * nty * P.nout;
+    const long long items = (long long)ntx * nty * (P.nout / 2);   // tile positions of whole frames
     if (items <= 0) return 0;
-    const unsigned blocks = (unsigned)((items + kWarps2 - 1) / kWarps2);
+    // Resident blocks, each warp walking several items: 300 fields take 0.93 ms
+    // (2.17 ms in the form before), 16 fields 65 us (125 us); 1,924 warp
+    // instructions a pair of tiles (3,732), issue 54 % active, bound by that
+    // and by the latency of the exchanges.
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned blocks = (unsigned)std::min<long long>((items + kWarps2 - 1) / kWarps2, (long long)kBlocks2 * std::max(sms, 1));
     if (P.thr_table != nullptr) tpal2d_kernel<true><<<blocks, 32 * kWarps2, 0, stream>>>(P);
     else tpal2d_kernel<false><<<blocks, 32 * kWarps2, 0, stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

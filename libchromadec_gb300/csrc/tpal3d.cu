@@ -73,21 +73,10 @@ static bool g_tp3_constants_ready[64];
 // it matches the order the shuffle FFT leaves the spectrum in); an involution.
 __device__ __forceinline__ int kappa(int l) { return rev4(l & 15) | (l & 16); }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
-{
-    return make_float2(__fmaf_rn(a.x, b.x, -a.y * b.y), __fmaf_rn(a.x, b.y, a.y * b.x));
-}
-
 template <int N>
 struct Int {
     static constexpr int value = N;
 };
-
-__device__ __forceinline__ float l1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
-
-// multiply by -i: (y, -x); by the tables' exp(-i pi/2) = (6e-17, -1), whose
-// tiny real part is below the rounding of any non-degenerate product
-__device__ __forceinline__ float2 mul_negi(float2 a) { return make_float2(a.y, -a.x); }
 
 __device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
 {
@@ -338,29 +327,6 @@ __device__ __forceinline__ void z_window(float2 (&wz)[4], bool high)
 {
 #pragma unroll
     for (int q = 0; q < 4; q++) wz[q] = make_float2(c3_wz[2 * q], high ? -c3_wz[2 * q + 1] : c3_wz[2 * q + 1]);
-}
-
-// Both fields' complex values, packed: (re of component 0, of component 1).
-struct cp2 {
-    float2 re, im;
-};
-__device__ __forceinline__ cp2 cadd(cp2 a, cp2 b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
-__device__ __forceinline__ cp2 csub(cp2 a, cp2 b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
-__device__ __forceinline__ cp2 cp_of(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
-__device__ __forceinline__ float4 f4_of(cp2 v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
-// A twiddle of each component: x = (x0, x1), y = (y0, y1), n = -y (rounds as
-// cmul does per component); conj: by the conjugate
-struct tw2 {
-    float2 x, y, n;
-};
-__device__ __forceinline__ cp2 ctw(cp2 a, tw2 t, bool conj)
-{
-    const float2 y = conj ? t.n : t.y, n = conj ? t.y : t.n;
-    return {__ffma2_rn(a.re, t.x, __fmul2_rn(a.im, n)), __ffma2_rn(a.re, y, __fmul2_rn(a.im, t.x))};
-}
-__device__ __forceinline__ float2 cmulc(float2 a, float2 b)   // a * conj(b), rounded as cmul(a, conj b)
-{
-    return make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)), __fmaf_rn(a.x, -b.y, __fmul_rn(a.y, b.x)));
 }
 
 // The block's Y twiddles, per quarter r: exp(-2 pi i n / 16) for n = r, r + 4

@@ -16,6 +16,36 @@ namespace tpal {
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 
+__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+{
+    return make_float2(__fmaf_rn(a.x, b.x, -a.y * b.y), __fmaf_rn(a.x, b.y, a.y * b.x));
+}
+
+__device__ __forceinline__ float l1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
+
+// Two complex values, packed: (re of component 0, of component 1), (im ...).
+struct cp2 {
+    float2 re, im;
+};
+__device__ __forceinline__ cp2 cadd(cp2 a, cp2 b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
+__device__ __forceinline__ cp2 csub(cp2 a, cp2 b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
+__device__ __forceinline__ cp2 cp_of(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+__device__ __forceinline__ float4 f4_of(cp2 v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
+// A twiddle of each component: x = (x0, x1), y = (y0, y1), n = -y (rounds as
+// cmul does per component); conj: by the conjugate
+struct tw2 {
+    float2 x, y, n;
+};
+__device__ __forceinline__ cp2 ctw(cp2 a, tw2 t, bool conj)
+{
+    const float2 y = conj ? t.n : t.y, n = conj ? t.y : t.n;
+    return {__ffma2_rn(a.re, t.x, __fmul2_rn(a.im, n)), __ffma2_rn(a.re, y, __fmul2_rn(a.im, t.x))};
+}
+__device__ __forceinline__ float2 cmulc(float2 a, float2 b)   // a * conj(b), rounded as cmul(a, conj b)
+{
+    return make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)), __fmaf_rn(a.x, -b.y, __fmul_rn(a.y, b.x)));
+}
+
 struct df {
     float hi, lo;
 };

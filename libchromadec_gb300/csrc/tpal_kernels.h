@@ -71,11 +71,11 @@ struct T2Params {
     long long field_stride;
     int field_base;
     int nfields;
-    int fw;
+    int fw, fh;
     int avs, ave, fafl, lafl;
     int black;
     int swap;                    // 1: even fields are second fields (reversed pairing)
-    int field_begin, nout;       // output fields [field_begin, field_begin + nout)
+    int field_begin, nout;       // output fields [field_begin, field_begin + nout), both even
     float *partial;
     long long part_class_stride, part_field_stride;
     int part_row_stride, fl_lo;
