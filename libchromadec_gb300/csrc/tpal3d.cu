@@ -584,16 +584,21 @@ struct ZInverse {
         sum(ym, om);
         O1 = make_float2(-O1.x, -O1.y);
     }
+    // slices 4 and 5
+    __device__ __forceinline__ float4 later() const
+    {
+        const float2 d0 = sub2(E0, O0);
+        return make_float4(d0.x, d0.y, __fsub_rn(E1.x, O1.x), __fsub_rn(E1.y, O1.y));
+    }
     // The output spectra at one ky, field 2m: slice 0 + carried slice 4 of
     // tile 2m-4, field 2m+1: slice 1 + carried slice 5; then this tile's
     // slices 4, 5 are carried for frame m+2.
     __device__ __forceinline__ cp2 finish(float4 *carry) const
     {
         const float4 c = *carry;
-        const float2 s0 = add2(E0, O0), d0 = sub2(E0, O0);
+        const float2 s0 = add2(E0, O0);
         const float2 s1 = make_float2(__fadd_rn(E1.x, O1.x), __fadd_rn(E1.y, O1.y));
-        const float2 d1 = make_float2(__fsub_rn(E1.x, O1.x), __fsub_rn(E1.y, O1.y));
-        *carry = make_float4(d0.x, d0.y, d1.x, d1.y);
+        *carry = later();
         return {make_float2(__fadd_rn(s0.x, c.x), __fadd_rn(s1.x, c.z)),
                 make_float2(__fadd_rn(s0.y, c.y), __fadd_rn(s1.y, c.w))};
     }
@@ -819,25 +824,12 @@ __device__ __forceinline__ void x_inverse_store(const T3Params &P, const LaneCon
     }
 }
 
-// The record of (step m, kx group g) in the list of `rec`'s item, or -1.
-__device__ __forceinline__ int find_record(const T3Params &P, int rec, int mg)
-{
-    int at = rec;
-    while (at >= 0 && P.unc_rec[at].mg > mg) at = P.unc_rec[at].prev;
-    while (at >= 0 && P.unc_rec[at].mg < mg) at = P.unc_rec[at].next;
-    return at >= 0 && P.unc_rec[at].mg == mg ? at : -1;
-}
-
 // TMODE: 0 = one uniform threshold, 1 = per-bin table, 2 = per-frame
-// thresholds (batches of captures). EXACT = false: the walk over every work
-// item, guard-band decisions taken in FP32 and recorded for
-// tp3_resolve_kernel (an exact path inside this loop, however rarely taken,
-// slows the whole walk by a third). EXACT = true: the outputs that
-// tp3_resolve_kernel's corrections reach, walked again with the decisions of
-// the corrected records; it writes the same output locations, so its result
-// replaces the FP32 one.
-template <int TMODE, bool EXACT>
-__global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpal3d_kernel(T3Params P)
+// thresholds (batches of captures). Guard-band decisions are taken in FP32 and
+// recorded for tp3_resolve_kernel (an exact path inside this loop, however
+// rarely taken, slows the whole walk by a third).
+template <int TMODE>
+__global__ void __launch_bounds__(32 * kWarps3, TMODE == 1 ? 3 : 4) tpal3d_kernel(T3Params P)
 {
     constexpr bool PER_BIN = (TMODE == 1);
     const int lane = threadIdx.x & 31;
@@ -856,26 +848,17 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
             thr[i] = P.thr_table[3 * ((((i >> 5) & 7) * 32 + kappa(i & 31)) * 3 + (i >> 8))];
     fill_twiddles(P, tw);
     // Work items (tile position, chunk of frames); a grid smaller than the
-    // item count walks them persistently. EXACT: two items per corrected
-    // record, the output of its own step mf and the one its carries feed
-    // (step mf + 2).
-    const unsigned nitems = EXACT ? 2 * min(P.counters[1], P.unc_cap) : (unsigned)(ntiles * P.nchunks);
+    // item count walks them persistently.
+    const unsigned nitems = (unsigned)(ntiles * P.nchunks);
     for (unsigned w = blockIdx.x * kWarps3 + warp; w < nitems; w += gridDim.x * kWarps3) {
-    const int rec = EXACT ? (int)P.rerun[w >> 1] : -1;
-    const int item = EXACT ? P.unc_rec[rec].item : (int)w;
+    const int item = (int)w;
     const int tile = item % ntiles;
     const int chunk = item / ntiles;
     const int tx = tile % P.ntx, ty = tile / P.ntx;
     const int tileX = P.tileX0 + 8 * tx;
     const int tileY = P.tileY0 + 16 * ty;
-    int m0 = P.frame_begin + chunk * P.chunk_frames;
-    int m1 = min(m0 + P.chunk_frames, P.frame_end);
-    if (EXACT) {
-        const int mo = (P.unc_rec[rec].mg >> 2) + 2 * (int)(w & 1);
-        if (mo < m0 || mo >= m1) continue;
-        m0 = mo;
-        m1 = mo + 1;
-    }
+    const int m0 = P.frame_begin + chunk * P.chunk_frames;
+    const int m1 = min(m0 + P.chunk_frames, P.frame_end);
     const int cls = ((ty & 1) << 1) | (tx & 1);
     const LaneConst LC = lane_const(P, lane, tileX, tileY);
     int last = -1;   // the item's latest record
@@ -893,10 +876,10 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
         if (lane < 20) y_stages<true>(m + 3, LC, lane, win, exch, R, bnd, tw);
         __syncwarp();
         if (m > m0) x_inverse_store(P, LC, R, m - 1, tileX, cls);
-        if (m < m0 - 2 || (EXACT && m == m0 - 1) || m == m1) continue;
+        if (m < m0 - 2 || m == m1) continue;
         __syncwarp();   // the output rows have been read: R may be written
 
-        const StepBounds SB = EXACT ? StepBounds{0.f, 0.f} : step_bounds(bnd, m, lane);
+        const StepBounds SB = step_bounds(bnd, m, lane);
         float4 *carry = carry_base + (m & 1) * (5 * 32);
         const float tf_m = (TMODE == 2) ? P.frame_t2[3 * max(m, 0)] : P.t2f;   // uniform threshold of frame m
 
@@ -920,17 +903,12 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
         };
         auto similar = [&](float a, float b, float t) -> bool {
             const float d = __fmaf_rn(-fmaxf(a, b), t, fminf(a, b));
-            if (!EXACT) {
-                const float s = a + b;
-                const float band = __fmaf_rn(e1, sqrt_approx(s), e2);
-                u |= (s >= lim) && (fabsf(d) <= (PER_BIN ? (1.f + t) * band : band));
-            }
+            const float s = a + b;
+            const float band = __fmaf_rn(e1, sqrt_approx(s), e2);
+            u |= (s >= lim) && (fabsf(d) <= (PER_BIN ? (1.f + t) * band : band));
             return d >= 0.f;
         };
         unsigned hits = 0;   // kx groups that reached the screen's bound
-        int fix[3] = {-1, -1, -1};
-        if (EXACT)
-            for (int g = 0; g < 3; g++) fix[g] = find_record(P, rec, m * 4 + g);
 
         // Pass 1: the pairs (kx 2, kx 6) in half-warp 0, (kx 3, kx 5) in half-warp 1
         {
@@ -939,7 +917,7 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
             z_window(wz, false);
             z_dft(win, m, h, LC.posA, wz, YA);
             z_dft(win, m, 4 - h, LC.posB, LC.wzB, YB);
-            bounds(EXACT ? 0.f : __shfl_sync(0xffffffffu, SB.em, h));
+            bounds(__shfl_sync(0xffffffffu, SB.em, h));
             float k[8], kh[8], kr[8], khr[8];   // at ky, at ky + 16; the same for the mirror column
             float ma[8], mb[8];
 #pragma unroll
@@ -947,20 +925,13 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
                 ma[kz] = mag2(YA[kz]);
                 mb[kz] = mag2(YB[kz]);
             }
-            unsigned fl = 0, fh = 0;
-            if (EXACT && fix[h] >= 0) {
-                fl = P.unc_rec[fix[h]].keep[lane & 15];
-                fh = P.unc_rec[fix[h]].keep[16 + (lane & 15)];
-            }
 #pragma unroll
             for (int kz = 0; kz < 8; kz++) {
                 const int kzr = (10 - kz) & 7;
-                bool sim = similar(ma[kz], mb[kzr], PER_BIN ? thr[(8 * h + kz) * 32 + (lane & 15)] : tf_m);
-                if (EXACT && fix[h] >= 0) sim = (fl >> kz) & 1u;
+                const bool sim = similar(ma[kz], mb[kzr], PER_BIN ? thr[(8 * h + kz) * 32 + (lane & 15)] : tf_m);
                 k[kz] = sim ? 1.f : 0.f;
                 if (PER_BIN) {
-                    bool simh = similar(ma[kz ^ 4], mb[kzr ^ 4], thr[(8 * h + kz) * 32 + 16 + (lane & 15)]);
-                    if (EXACT && fix[h] >= 0) simh = (fh >> kz) & 1u;
+                    const bool simh = similar(ma[kz ^ 4], mb[kzr ^ 4], thr[(8 * h + kz) * 32 + 16 + (lane & 15)]);
                     kh[kz] = simh ? 1.f : 0.f;
                 }
             }
@@ -971,10 +942,8 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
             }
             z_inverse<!PER_BIN>(YA, k, kh, carry, R, h, lane & 15);
             z_inverse<!PER_BIN>(YB, kr, khr, carry, R, 4 - h, LC.laneB);
-            if (!EXACT) {
-                const unsigned b = __ballot_sync(0xffffffffu, u);
-                hits = ((b & 0xFFFFu) != 0 ? 1u : 0u) | (b >> 16 != 0 ? 2u : 0u);
-            }
+            const unsigned b = __ballot_sync(0xffffffffu, u);
+            hits = ((b & 0xFFFFu) != 0 ? 1u : 0u) | (b >> 16 != 0 ? 2u : 0u);
         }
         // Pass 2: kx 4, whose mirror bins' magnitudes come from the lanes
         // that own them; all 32 ky.
@@ -983,8 +952,7 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
             float2 Y[8], wz[4];
             z_window(wz, lane >= 16);
             z_dft(win, m, 2, LC.posA, wz, Y);
-            bounds(EXACT ? 0.f : __shfl_sync(0xffffffffu, SB.em, 2));
-            const unsigned f = EXACT && fix[2] >= 0 ? P.unc_rec[fix[2]].keep[lane] : 0u;
+            bounds(__shfl_sync(0xffffffffu, SB.em, 2));
             float2 y[8], o[4];
 #pragma unroll
             for (int kz = 0; kz < 8; kz++) {
@@ -993,7 +961,6 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
                 bool sim = similar(a, b, PER_BIN ? thr[(16 + kz) * 32 + lane] : tf_m);
                 if (PER_BIN) sim |= similar(a, b, thr[(16 + kzr) * 32 + laneB]);   // the mirror bin visits too
                 if (kz == kzr) sim |= laneB == lane;   // a carrier (its own mirror) is always kept
-                if (EXACT && fix[2] >= 0) sim = (f >> kz) & 1u;
                 const float k = sim ? 1.f : 0.f;
                 y[kz] = __fmul2_rn(Y[kz], make_float2(k, k));
             }
@@ -1003,9 +970,9 @@ __global__ void __launch_bounds__(32 * kWarps3, EXACT || TMODE == 1 ? 3 : 4) tpa
             const cp2 own = Z.finish(carry + 32 * 2 + lane);
             const cp2 high = {shfl_xor2(own.re, 16), shfl_xor2(own.im, 16)};
             if (lane < 16) R[20 * 2 + LC.posA] = f4_of(fold_ky(own, high));
-            if (!EXACT && __any_sync(0xffffffffu, u)) hits |= 4u;
+            if (__any_sync(0xffffffffu, u)) hits |= 4u;
         }
-        if (!EXACT && hits != 0) {   // one copy of the rare path
+        if (hits != 0) {   // one copy of the rare path
 #pragma unroll 1
             for (int g = 0; g < 3; g++) {
                 if (!(hits >> g & 1)) continue;
@@ -1321,6 +1288,188 @@ __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
 }
 
 // ---------------------------------------------------------------------------
+// The outputs that corrected decisions reach, once more
+// ---------------------------------------------------------------------------
+// The record of (step m, kx group g) in the list of `rec`'s item, or -1.
+__device__ __forceinline__ int find_record(const T3Params &P, int rec, int mg)
+{
+    int at = rec;
+    while (at >= 0 && P.unc_rec[at].mg > mg) at = P.unc_rec[at].prev;
+    while (at >= 0 && P.unc_rec[at].mg < mg) at = P.unc_rec[at].next;
+    return at >= 0 && P.unc_rec[at].mg == mg ? at : -1;
+}
+
+// Two outputs per corrected record, the one of its own step mf and the one its
+// carries feed (step mf + 2), recomputed with the decisions of the corrected
+// records; they are written where the walk wrote them. The operations and
+// their order are the walk's.
+//
+// There are few of them, so what counts is how long one takes: a block owns an
+// output, its six pairs of fields are transformed by a warp each (a seventh
+// looks the records up), the Z stages of the two tiles that meet in the output
+// by four. 31 -> 8.4 us for a few outputs (the walk's own loop over the steps, a
+// warp an output); for the hundreds of a 500-field capture both take about 30.
+constexpr int kWarpsX = 7;
+constexpr int kPairsX = 6;
+template <int TMODE>
+__global__ void __launch_bounds__(32 * kWarpsX, 2) tpal3d_exact_kernel(T3Params P)
+{
+    constexpr bool PER_BIN = (TMODE == 1);
+    __shared__ float4 win[kPairsX * 80 + 80];   // one more, for the output's unused forward stage
+    __shared__ float4 exch[kPairsX * kExchF4], carry[5 * 32], R[kOutF4], tw[kTwF4];
+    __shared__ float2 bnd[(kPairsX + 1) * 8];
+    __shared__ float thr[PER_BIN ? 3 * 8 * 32 : 1];
+    __shared__ uint8_t s_keep[2][3][32];        // decisions of step mo (0) and mo - 2 (1) per kx group
+    __shared__ int s_fix[2][3];                 // their records, or -1
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned nitems = 2 * min(P.counters[1], P.unc_cap);
+    if (blockIdx.x >= nitems) return;
+    const int ntiles = P.ntx * P.nty;
+    if (PER_BIN)
+        for (int i = threadIdx.x; i < 3 * 8 * 32; i += blockDim.x)
+            thr[i] = P.thr_table[3 * ((((i >> 5) & 7) * 32 + kappa(i & 31)) * 3 + (i >> 8))];
+    fill_twiddles(P, tw);
+    for (unsigned w = blockIdx.x; w < nitems; w += gridDim.x) {
+        const int rec = (int)P.rerun[w >> 1];
+        const int item = P.unc_rec[rec].item, tile = item % ntiles, chunk = item / ntiles;
+        const int tx = tile % P.ntx, ty = tile / P.ntx;
+        const int tileX = P.tileX0 + 8 * tx, tileY = P.tileY0 + 16 * ty;
+        const int mo = (P.unc_rec[rec].mg >> 2) + 2 * (int)(w & 1);
+        const int m0 = P.frame_begin + chunk * P.chunk_frames;
+        if (mo < m0 || mo >= min(m0 + P.chunk_frames, P.frame_end)) continue;   // the whole block
+        const LaneConst LC = lane_const(P, lane, tileX, tileY);
+        if (warp < kPairsX) {   // pair mo - 2 + warp
+            RowWords row;
+            load_row(P, mo - 2 + warp, LC, row);
+            x_forward(row, 0, LC, exch + kExchF4 * warp, bnd + 8 * warp);
+            __syncwarp();
+            if (lane < 20) y_stages<false>(0, LC, lane, win + 80 * warp, exch + kExchF4 * warp, R, bnd + 8 * warp, tw);
+        } else {
+            const int st = lane / 3, g = lane % 3;
+            const int at = lane < 6 ? find_record(P, rec, (mo - 2 * st) * 4 + g) : -1;
+            if (lane < 6) s_fix[st][g] = at;
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                const int r = __shfl_sync(0xffffffffu, at, i);
+                if (r >= 0) s_keep[i / 3][i % 3][lane] = P.unc_rec[r].keep[lane];
+            }
+        }
+        __syncthreads();
+        // warps 0, 1: pass 1 and pass 2 of step mo; 2, 3: of step mo - 2
+        const int st = warp >> 1, pass = warp & 1;
+        const int h = lane >> 4;
+        ZInverse Z[4];   // pass 1: column kx = 2 + h at ky and ky + 16, the mirror column likewise; pass 2: kx = 4
+        if (warp < 4) {
+            const float4 *tile4 = win + (st == 0 ? 2 * 80 : 0);
+            const int m = mo - 2 * st;
+            const float tf_m = (TMODE == 2) ? P.frame_t2[3 * max(m, 0)] : P.t2f;
+            auto similar = [](float a, float b, float t) -> bool { return __fmaf_rn(-fmaxf(a, b), t, fminf(a, b)) >= 0.f; };
+            float2 wz[4], y[8], o[4];
+            if (pass == 0) {
+                float2 YA[8], YB[8];
+                z_window(wz, false);
+                z_dft(tile4, 0, h, LC.posA, wz, YA);
+                z_dft(tile4, 0, 4 - h, LC.posB, LC.wzB, YB);
+                const bool fixed = s_fix[st][h] >= 0;
+                const unsigned fl = s_keep[st][h][lane & 15], fh = s_keep[st][h][16 + (lane & 15)];
+                float k[8], kh[8];
+#pragma unroll
+                for (int kz = 0; kz < 8; kz++) {
+                    const int kzr = (10 - kz) & 7;
+                    bool sim = similar(mag2(YA[kz]), mag2(YB[kzr]), PER_BIN ? thr[(8 * h + kz) * 32 + (lane & 15)] : tf_m);
+                    if (fixed) sim = (fl >> kz) & 1u;
+                    k[kz] = sim ? 1.f : 0.f;
+                    if (PER_BIN) {
+                        bool simh = similar(mag2(YA[kz ^ 4]), mag2(YB[kzr ^ 4]), thr[(8 * h + kz) * 32 + 16 + (lane & 15)]);
+                        if (fixed) simh = (fh >> kz) & 1u;
+                        kh[kz] = simh ? 1.f : 0.f;
+                    }
+                }
+                // masked by k; at ky + 16 by k moved by 4 or, per bin, kh
+                auto sums = [&](const float2 (&Y)[8], bool mirror, ZInverse &lo, ZInverse &hi) {
+#pragma unroll
+                    for (int z = 0; z < 8; z++) {
+                        const float kk = mirror ? k[(10 - z) & 7] : k[z];
+                        y[z] = __fmul2_rn(Y[z], make_float2(kk, kk));
+                    }
+                    z_rotate(y, o);
+                    lo.sum(y, o);
+                    if constexpr (PER_BIN) {
+#pragma unroll
+                        for (int z = 0; z < 8; z++) {
+                            const float kk = mirror ? kh[(10 - z) & 7] : kh[z];
+                            y[z] = __fmul2_rn(Y[z ^ 4], make_float2(kk, kk));
+                        }
+                        z_rotate(y, o);
+                        hi.sum(y, o);
+                    } else {
+                        hi.sum_moved(y, o);
+                    }
+                };
+                sums(YA, false, Z[0], Z[1]);
+                sums(YB, true, Z[2], Z[3]);
+            } else {
+                const int laneB = LC.laneB ^ (lane & 16);
+                float2 Y[8];
+                z_window(wz, lane >= 16);
+                z_dft(tile4, 0, 2, LC.posA, wz, Y);
+                const bool fixed = s_fix[st][2] >= 0;
+                const unsigned f = s_keep[st][2][lane];
+#pragma unroll
+                for (int kz = 0; kz < 8; kz++) {
+                    const int kzr = (10 - kz) & 7;
+                    const float a = mag2(Y[kz]), b = __shfl_sync(0xffffffffu, mag2(Y[kzr]), laneB);
+                    bool sim = similar(a, b, PER_BIN ? thr[(16 + kz) * 32 + lane] : tf_m);
+                    if (PER_BIN) sim |= similar(a, b, thr[(16 + kzr) * 32 + laneB]);   // the mirror bin visits too
+                    if (kz == kzr) sim |= laneB == lane;   // a carrier (its own mirror) is always kept
+                    if (fixed) sim = (f >> kz) & 1u;
+                    const float k = sim ? 1.f : 0.f;
+                    y[kz] = __fmul2_rn(Y[kz], make_float2(k, k));
+                }
+                z_rotate(y, o);
+                Z[0].sum(y, o);
+            }
+        }
+        // where Z[i] meets its carry
+        auto slot = [&](int i) -> float4 * {
+            if (pass == 1) return carry + 32 * 2 + lane;
+            const int at = i < 2 ? lane & 15 : LC.laneB;
+            return carry + 32 * (i < 2 ? h : 4 - h) + ((i & 1) ? at ^ 16 : at);
+        };
+        if (warp == 2 || warp == 3) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (pass == 0 || i == 0) *slot(i) = Z[i].later();
+        }
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int at = c == 0 ? lane & 15 : LC.laneB, col = c == 0 ? h : 4 - h;
+                const cp2 a = Z[2 * c].finish(slot(2 * c)), b = Z[2 * c + 1].finish(slot(2 * c + 1));
+                cp2 g = fold_ky(a, b);
+                if (at >= 16) {   // a is the upper half: component 1 is b - a
+                    g.re.y = -g.re.y;
+                    g.im.y = -g.im.y;
+                }
+                R[20 * col + swz(at & 15)] = f4_of(g);
+            }
+        } else if (warp == 1) {
+            const cp2 own = Z[0].finish(slot(0));
+            const cp2 high = {shfl_xor2(own.re, 16), shfl_xor2(own.im, 16)};
+            if (lane < 16) R[20 * 2 + LC.posA] = f4_of(fold_ky(own, high));
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (lane < 20) y_stages<true>(0, LC, lane, win + 80 * kPairsX, exch, R, bnd + 8 * kPairsX, tw);
+            __syncwarp();
+            x_inverse_store(P, LC, R, mo, tileX, ((ty & 1) << 1) | (tx & 1));
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 static double rc_window(int n, int N) { return 0.5 - (0.5 * cos((2 * M_PI * (n + 0.5)) / N)); }
@@ -1410,20 +1559,17 @@ int tp3_launch(const T3Params &P, cudaStream_t stream, int max_blocks)
     if (!attr_set[dev]) {
         const int b = (int)walk_smem(true);
         const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        if (cudaFuncSetAttribute(tpal3d_kernel<0, false>, a, b) != cudaSuccess ||
-            cudaFuncSetAttribute(tpal3d_kernel<1, false>, a, b) != cudaSuccess ||
-            cudaFuncSetAttribute(tpal3d_kernel<2, false>, a, b) != cudaSuccess ||
-            cudaFuncSetAttribute(tpal3d_kernel<0, true>, a, b) != cudaSuccess ||
-            cudaFuncSetAttribute(tpal3d_kernel<1, true>, a, b) != cudaSuccess ||
-            cudaFuncSetAttribute(tpal3d_kernel<2, true>, a, b) != cudaSuccess)
+        if (cudaFuncSetAttribute(tpal3d_kernel<0>, a, b) != cudaSuccess ||
+            cudaFuncSetAttribute(tpal3d_kernel<1>, a, b) != cudaSuccess ||
+            cudaFuncSetAttribute(tpal3d_kernel<2>, a, b) != cudaSuccess)
             return -1;
         attr_set[dev] = true;
     }
     if (P.unc_rec == nullptr || P.counters == nullptr || P.rerun == nullptr) return -1;
     const unsigned t = 32 * kWarps3;
-    if (P.thr_table != nullptr) tpal3d_kernel<1, false><<<blocks, t, smem, stream>>>(P);
-    else if (P.frame_t2 != nullptr) tpal3d_kernel<2, false><<<blocks, t, smem, stream>>>(P);
-    else tpal3d_kernel<0, false><<<blocks, t, smem, stream>>>(P);
+    if (P.thr_table != nullptr) tpal3d_kernel<1><<<blocks, t, smem, stream>>>(P);
+    else if (P.frame_t2 != nullptr) tpal3d_kernel<2><<<blocks, t, smem, stream>>>(P);
+    else tpal3d_kernel<0><<<blocks, t, smem, stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1436,11 +1582,10 @@ int tp3_resolve_launch(const T3Params &P, cudaStream_t stream)
     // the record and item counts are only known on the device: fixed grids
     // walk them
     tp3_resolve_kernel<<<4 * sms, 32 * kWarps3, sizeof(int4) * kQYZ, stream>>>(P);
-    const size_t smem = walk_smem(P.thr_table != nullptr);
-    const unsigned t = 32 * kWarps3, blocks = 3u * (unsigned)sms;
-    if (P.thr_table != nullptr) tpal3d_kernel<1, true><<<blocks, t, smem, stream>>>(P);
-    else if (P.frame_t2 != nullptr) tpal3d_kernel<2, true><<<blocks, t, smem, stream>>>(P);
-    else tpal3d_kernel<0, true><<<blocks, t, smem, stream>>>(P);
+    const unsigned t = 32 * kWarpsX, blocks = 2u * (unsigned)sms;
+    if (P.thr_table != nullptr) tpal3d_exact_kernel<1><<<blocks, t, 0, stream>>>(P);
+    else if (P.frame_t2 != nullptr) tpal3d_exact_kernel<2><<<blocks, t, 0, stream>>>(P);
+    else tpal3d_exact_kernel<0><<<blocks, t, 0, stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
