@@ -654,6 +654,16 @@ int Engine::set_tc_form(int variant)
     return 0;
 }
 
+int Engine::reserve(int frames)
+{
+    frames = std::min(frames, max_batch_frames_);
+    if (c_.kind != 6)
+        if (const int rc = ensure_partial(2 * frames); rc != 0) return rc;
+    if (c_.kind == 8 && tc_variant_ < 0 && net_ == nullptr)
+        return ensure_deferred(frames, (frames + chunk_frames_ - 1) / chunk_frames_);
+    return 0;
+}
+
 int Engine::decode(const uint16_t *fields, long long stride, int field_base, int nfields, int fb, int fe, void *out,
                    cudaStream_t s)
 {

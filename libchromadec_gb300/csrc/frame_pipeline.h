@@ -26,10 +26,12 @@
 
 namespace chdg {
 
-// Pinned host memory holding `count` decoded frames; frames borrow slices.
+// Pinned host memory holding `count` decoded frames; frames borrow slices. A
+// chunk with an owner is a part of the owner's memory.
 struct HostChunk {
     void *data = nullptr;
     size_t bytes = 0;
+    std::shared_ptr<HostChunk> owner;
     ~HostChunk();
 };
 
@@ -45,6 +47,7 @@ using Deliver = std::function<void(const std::shared_ptr<HostChunk> &chunk, int6
 class FramePipeline {
 public:
     static constexpr int kEdgeFrames = 16;   // size of the first and last batch of a long run
+    static constexpr int kSplitFrames = 9;   // a run of one batch longer than this is decoded in parts
 
     FramePipeline() = default;
     ~FramePipeline();
@@ -79,9 +82,9 @@ public:
 private:
     // Enqueue the window fields of frames [w0, w1) into dwin_[slot] on copy_.
     int upload_window(int slot, int64_t w0, int64_t w1);
-    // upload_window plus the frames' dropout plans and the extra-source
-    // fields they read; nplan = frames with a plan.
-    int upload_batch(int slot, int64_t w0, int64_t w1, int &nplan);
+    // upload_window plus the frames' dropout plans, the extra-source fields
+    // they read and the concealment.
+    int upload_batch(int slot, int64_t w0, int64_t w1);
     const FramePlan &plan_for(int64_t frame);   // cached, window frame (0-based)
     // the concealment's luma filter: PAL's, or the NTSC taps that NTSC and
     // PAL-M use (dropout_corrector.cpp:498-506)
