@@ -800,19 +800,10 @@ __global__ void mn_round_kernel(const float *master, float *used)
 //    tile's features into one of two stages.
 // All waits are bounded; a wait that runs out raises the error flag and the
 // CTA leaves after its copies and MMAs in flight have completed.
-//
-// HALF: features that repeat, f(kz + 4, ky + 16) = f(kz, ky), as every
-// spectrum of a tile does (the walk's Z stage says why). The network commutes
-// with shifts along its periodic axes, so its output repeats the same way, bit
-// for bit, and 128 of the 256 rows suffice: the two M blocks are the ky < 16
-// of two tiles. Each block has its own 18 row groups; its halo groups are its
-// own ky = 15 and ky = 0 with kz moved by 4, so nothing needs the stash. The
-// schedule is the same. 62,160 tiles: 3.80 -> 1.88 ms.
 constexpr int kEpiWarps = 8;
 constexpr int kTcThreads = 32 * (kEpiWarps + 2);
 constexpr int kGroupsA = 34;                       // 32 ky groups + one halo group on each side
-constexpr int kGroupsH = 18;                       // HALF: 16 + 2, a tile
-constexpr int A_BYTES = 2 * kGroupsH * 8 * 160;    // a layer's input, K up to 80
+constexpr int A_BYTES = kGroupsA * 8 * 160;         // a layer's input, K up to 80
 constexpr int NCOL = 3 * 80;                       // accumulator columns of one M block: (q, dz, co)
 constexpr int kSlots = 8;                          // weight-piece ring (a layer's 5 pieces stay for both blocks)
 constexpr int SLOT_BYTES = 3 * 144 * 32;           // the largest piece: three ky taps x 144 rows x K 16
@@ -820,9 +811,9 @@ constexpr int FEAT_BYTES = NV * 2;
 constexpr int kPieces = 10;                        // streamed weight pieces of one tile (layers 2 and 3)
 constexpr int W1_BYTES = 3 * NCOL * 32;            // layer 1's weights, resident
 constexpr int STASH_BYTES = 2 * 8 * 160;           // row groups 16 and 33 of the next layer's input
-constexpr int IN_BYTES = 2 * kGroupsH * 8 * 32;    // layer 1's input, K = 16
-// shared memory: layers 2 and 3's input [36 groups][8 rows][K 80] and layer
-// 1's [36][8][K 16] (34 used unless HALF), both canonical (apart, so a tile's input can be written
+constexpr int IN_BYTES = kGroupsA * 8 * 32;         // layer 1's input, K = 16
+// shared memory: layers 2 and 3's input [34 groups][8 rows][K 80] and layer
+// 1's [34][8][K 16], both canonical (apart, so a tile's input can be written
 // while the previous layers' operands are read), the ring, two feature
 // stages, the stash, the barriers
 constexpr int SM_A = 0;
@@ -830,7 +821,7 @@ constexpr int SM_IN = A_BYTES;
 constexpr int SM_W1 = SM_IN + IN_BYTES;
 constexpr int SM_SLOT = SM_W1 + W1_BYTES;
 constexpr int SM_FEAT = SM_SLOT + kSlots * SLOT_BYTES;
-constexpr int SM_STASH = SM_FEAT + 4 * FEAT_BYTES;   // two stages of up to two tiles
+constexpr int SM_STASH = SM_FEAT + 2 * FEAT_BYTES;
 constexpr int SM_BAR = SM_STASH + STASH_BYTES;
 // barriers: an M block's MMAs of a layer done (2); a release of the MMAs (5:
 // chunk q of the next layer's input written, and for layer 1 the input (0)
@@ -927,25 +918,14 @@ __device__ __forceinline__ void put_row(uint8_t *A, int KB, int ky, int kz, int 
     if (ky == 0) *reinterpret_cast<uint4 *>(base + (kGroupsA - 1) * grp) = v;
 }
 
-// The same for HALF's tile b: group 18 b + ky + 1, and the halo groups at
-// ky = -1 and 16, which repeat ky = 15 and 0 with kz moved by 4.
-__device__ __forceinline__ void put_row_half(uint8_t *A, int KB, int b, int ky, int kz, int c, uint4 v)
-{
-    const int grp = 8 * KB;
-    uint8_t *base = A + b * kGroupsH * grp + c * 128;
-    *reinterpret_cast<uint4 *>(base + (ky + 1) * grp + kz * 16) = v;
-    if (ky == 15) *reinterpret_cast<uint4 *>(base + (kz ^ 4) * 16) = v;
-    if (ky == 0) *reinterpret_cast<uint4 *>(base + (kGroupsH - 1) * grp + (kz ^ 4) * 16) = v;
-}
-
-// OR of a predicate over the epilogue's 256 threads (named barrier 1).
-__device__ __forceinline__ bool epi_or(bool v)
+// OR of a predicate over an epilogue's 256 threads (named barrier id).
+__device__ __forceinline__ bool epi_or(bool v, int id = 1)
 {
     uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\t"
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\tbar.red.or.pred p, %3, %2, q;\n\t"
                  "selp.b32 %0, 1, 0, p;\n\t}\n"
                  : "=r"(r)
-                 : "r"((uint32_t)v), "r"(32 * kEpiWarps)
+                 : "r"((uint32_t)v), "r"(32 * kEpiWarps), "r"(id)
                  : "memory");
     return r != 0;
 }
@@ -996,7 +976,6 @@ __device__ __forceinline__ void mma_band_any(int ks, uint32_t d, uint64_t ab, ui
 // The MMA warp's thread. Per tile and layer: block 0's MMAs (each chunk once
 // released), then block 1's with the same weight pieces, whose slots are then
 // freed.
-template <bool HALF>
 __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, long long step, long long ntiles)
 {
     using namespace tpal::tc;
@@ -1004,11 +983,10 @@ __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, l
              *sfree = S.bars + B_SFREE;
     // operand descriptors at the bases: A with 8-row groups 256 bytes apart
     // (layer 1) or 1280 (layers 2 and 3), the weight slots 256; block 1's A
-    // starts 16 row groups in (HALF: the second tile's 18)
-    constexpr int kBlock1 = HALF ? kGroupsH : 16;
+    // starts 16 row groups in
     const uint64_t a1 = sdesc(smem_addr(S.in), 256), a2 = sdesc(smem_addr(S.A), 1280),
                    b0 = sdesc(smem_addr(S.slots), 256);
-    const uint64_t a1b[2] = {a1, desc_at(a1, kBlock1 * 256)}, a2b[2] = {a2, desc_at(a2, kBlock1 * 1280)};
+    const uint64_t a1b[2] = {a1, desc_at(a1, 16 * 256)}, a2b[2] = {a2, desc_at(a2, 16 * 1280)};
     uint32_t rbits = 0;   // parity of each release barrier's next phase
     long long sc = 0;     // weight pieces taken
     bool ok = true;
@@ -1078,9 +1056,8 @@ __device__ bool tc_mma_role(const TcShared &S, uint32_t tmem, long long first, l
 
 // The copy warp's thread: weight pieces through the ring, features of the
 // next tile into the other stage.
-template <bool HALF>
 __device__ bool tc_copy_role(const TcShared &S, const uint8_t *img, const uint16_t *feat, long long first,
-                             long long step, long long ntiles, long long count)
+                             long long step, long long ntiles)
 {
     using namespace tpal::tc;
     uint64_t *sfull = S.bars + B_SFULL, *sfree = S.bars + B_SFREE, *ffull = S.bars + B_FFULL,
@@ -1092,10 +1069,8 @@ __device__ bool tc_copy_role(const TcShared &S, const uint8_t *img, const uint16
         const int b = (int)(js & 1);
         const long long use = js >> 1;   // earlier fills of this stage
         if (use >= 1 && !bar_wait(ffree + b, (uint32_t)((use - 1) & 1))) return false;
-        // HALF: the pair's tiles 2 tile and, unless it is past the last, 2 tile + 1
-        const uint32_t bytes = HALF && 2 * tile + 1 < count ? 2 * FEAT_BYTES : FEAT_BYTES;
-        bar_arrive_expect_tx(ffull + b, bytes);
-        bulk_g2s(S.stage + b * 2 * FEAT_BYTES, feat + (HALF ? 2 : 1) * tile * NV, bytes, ffull + b);
+        bar_arrive_expect_tx(ffull + b, FEAT_BYTES);
+        bulk_g2s(S.stage + b * FEAT_BYTES, feat + tile * NV, FEAT_BYTES, ffull + b);
         js++;
         return true;
     };
@@ -1173,10 +1148,9 @@ __device__ __forceinline__ void combine_block(const uint32_t (&d)[48], int lane,
                 __shfl_sync(0xffffffffu, __uint_as_float(d[32 + co]), lp);
 }
 
-// HALF: `tile` below counts pairs of tiles, M block b is tile 2 tile + b.
-template <bool TRAIN, bool HALF>
+template <bool TRAIN>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    mn_tc_forward_kernel(const uint8_t *img, const float *params, const uint16_t *feat, long long count,
+    mn_tc_forward_kernel(const uint8_t *img, const float *params, const uint16_t *feat, long long ntiles,
                          float conf_limit, float *p_out, uint8_t *fallback, __nv_bfloat16 *a1g, __nv_bfloat16 *a2g,
                          __nv_bfloat16 *a3g, int *err)
 {
@@ -1193,7 +1167,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint8_t *stash = smem + SM_STASH;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + SM_TSLOT);
     __shared__ float s_par[4 * NC + 1];   // b1, b2, b3, wh, bh
-    __shared__ float red[2][2][kEpiWarps];   // [block, HALF][parity of the tile][warp]
+    __shared__ float red[2][kEpiWarps];   // [parity of the tile][warp]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     for (int i = t; i < 4 * NC + 1; i += kTcThreads) {
         const int off[5] = {OFF_B1, OFF_B2, OFF_B3, OFF_WH, OFF_BH};
@@ -1211,15 +1185,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
-    static_assert(!(TRAIN && HALF), "training takes any features");
-    const long long ntiles = HALF ? (count + 1) / 2 : count;
     const long long first = blockIdx.x, step = gridDim.x;
     bool ok = true;
     if (warp == kEpiWarps) {
-        if (lane == 0) ok = tc_mma_role<HALF>(S, tmem, first, step, ntiles);
+        if (lane == 0) ok = tc_mma_role(S, tmem, first, step, ntiles);
         __syncwarp();
     } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) ok = tc_copy_role<HALF>(S, img, feat, first, step, ntiles, count);
+        if (lane == 0) ok = tc_copy_role(S, img, feat, first, step, ntiles);
         __syncwarp();
     } else {
         uint64_t *full = S.bars + B_FULL, *ready = S.bars + B_READY, *ffull = S.bars + B_FFULL,
@@ -1234,18 +1206,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // thread): row r = (ky, kz), k = 2 q + c (c = 0: the bin, 1: its
         // mirror), zero-padded to 16. Every epilogue warp releases the stage
         // and the first layer's block-0 MMAs.
-        auto write_input = [&](bool both) {
+        auto write_input = [&]() {
             const int b = (int)(js & 1);
             bool done = true;
             if (h == 1) {
                 done = bar_wait(ffull + b, (fbits >> b) & 1);
                 if (done) {
                     fbits ^= 1u << b;
-                    const __nv_bfloat16 *f0 = reinterpret_cast<const __nv_bfloat16 *>(S.stage + b * 2 * FEAT_BYTES);
+                    const __nv_bfloat16 *f = reinterpret_cast<const __nv_bfloat16 *>(S.stage + b * FEAT_BYTES);
                     for (int r = t - 128; r < 256; r += 128) {
-                        // HALF: row r of block r >> 7; a pair without a second tile runs its first twice
-                        const int ky = HALF ? (r >> 3) & 15 : r >> 3, rz = r & 7;
-                        const __nv_bfloat16 *f = HALF && both && r >= 128 ? f0 + NV : f0;
+                        const int ky = r >> 3, rz = r & 7;
                         __align__(16) __nv_bfloat16 v[16];
 #pragma unroll
                         for (int q = 0; q < NQ; q++) {
@@ -1255,11 +1225,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
                         for (int k = 10; k < 16; k++) v[k] = __float2bfloat16_rn(0.f);
 #pragma unroll
-                        for (int c = 0; c < 2; c++) {
-                            const uint4 u = reinterpret_cast<const uint4 *>(v)[c];
-                            if (HALF) put_row_half(S.in, 32, r >> 7, ky, rz, c, u);
-                            else put_row(S.in, 32, ky, rz, c, u);
-                        }
+                        for (int c = 0; c < 2; c++) put_row(S.in, 32, ky, rz, c, reinterpret_cast<const uint4 *>(v)[c]);
                     }
                     fence_async_smem();
                 }
@@ -1273,13 +1239,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             return done;
         };
         if (first < ntiles) {
-            bad = !write_input(2 * first + 1 < count);
+            bad = !write_input();
             // block 1's columns are free for the first tile
             if (lane == 0) bar_arrive(ready + 1);
         }
         long long it = 0;
         for (long long tile = first; tile < ntiles; tile += step, it++) {
-            float conf = 0.f, conf1 = 0.f;   // HALF: block 0's tile, block 1's
+            float conf = 0.f;
             const bool more = tile + step < ntiles;
             for (int L = 0; L < 3; L++) {
                 for (int b = 0; b < 2; b++) {
@@ -1291,7 +1257,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     pfull ^= 1u << b;
                     fence_after();
                     const int erow = b * 128 + qd * 32 + lane;   // the row: ky = erow >> 3, kz
-                    const int ky = HALF ? (erow >> 3) & 15 : erow >> 3;
+                    const int ky = erow >> 3;
                     if (L < 2) {
                         const uint32_t tl = tq + b * 256 + h * 8;
                         float bias[8];
@@ -1312,9 +1278,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 o[c] = __float2bfloat16_rn(fmaxf(y[c] + bias[c], 0.f));
                             const uint4 ov = *reinterpret_cast<const uint4 *>(o);
                             const int ch = 2 * q + h;   // the 16-byte chunk of the input row
-                            if (HALF) {
-                                put_row_half(S.A, 160, b, ky, kz, ch, ov);
-                            } else if (b == 0) {
+                            if (b == 0) {
                                 // groups 16 (ky = 15) and 33 (the halo copy of
                                 // ky = 0) are still read by block 1's MMAs
                                 if (ky == 15)
@@ -1388,17 +1352,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                     *reinterpret_cast<uint4 *>(a3g + act_at(tile, 8 * hc, vox)) =
                                         reinterpret_cast<const uint4 *>(a3)[hc];
                             const float p = 1.0f / (1.0f + expf(-zh));
-                            if (HALF) {
-                                if (2 * tile + b < count) {
-                                    float *po = p_out + (2 * tile + b) * NV;
-                                    po[vox] = p;
-                                    po[(q * 8 + (kz ^ 4)) * 32 + ky + 16] = p;
-                                }
-                                (b ? conf1 : conf) += 2.f * fabsf(p - 0.5f);
-                            } else {
-                                p_out[tile * NV + vox] = p;
-                                conf += fabsf(p - 0.5f);
-                            }
+                            p_out[tile * NV + vox] = p;
+                            conf += fabsf(p - 0.5f);
                         };
                         uint32_t ba[48], bb[48];
                         if (h == 0) {
@@ -1420,7 +1375,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         __syncwarp();
                         if (more) {
                             if (b == 0) {
-                                if (!write_input(2 * (tile + step) + 1 < count)) bad = true;
+                                if (!write_input()) bad = true;
                             } else if (lane == 0) {
                                 bar_arrive(ready + 1);
                             }
@@ -1430,27 +1385,340 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
             // the tile's confidence; a failure anywhere stops every epilogue warp here
 #pragma unroll
-            for (int hh = 16; hh >= 1; hh >>= 1) {
-                conf += __shfl_xor_sync(0xffffffffu, conf, hh);
-                if (HALF) conf1 += __shfl_xor_sync(0xffffffffu, conf1, hh);
-            }
-            if (lane == 0) {
-                red[0][it & 1][warp] = conf;
-                if (HALF) red[1][it & 1][warp] = conf1;
-            }
+            for (int hh = 16; hh >= 1; hh >>= 1) conf += __shfl_xor_sync(0xffffffffu, conf, hh);
+            if (lane == 0) red[it & 1][warp] = conf;
             if (epi_or(bad || *S.abort_flag != 0)) {
                 bad = true;
                 break;
             }
-            if (t < (HALF ? 2 : 1) && fallback != nullptr) {
+            if (t == 0 && fallback != nullptr) {
                 float sum = 0.f;
 #pragma unroll
-                for (int w = 0; w < kEpiWarps; w++) sum += red[t][it & 1][w];
-                const long long at = HALF ? 2 * tile + t : tile;
-                if (at < count) fallback[at] = (sum * (1.0f / NV) < conf_limit) ? 1 : 0;
+                for (int w = 0; w < kEpiWarps; w++) sum += red[it & 1][w];
+                fallback[tile] = (sum * (1.0f / NV) < conf_limit) ? 1 : 0;
             }
         }
         if (bad) *S.abort_flag = 1;
+        ok = !bad;
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    if (!ok) atomicExch(err, 1);
+}
+
+// ---------------------------------------------------------------------------
+// The forward pass over features that repeat
+// ---------------------------------------------------------------------------
+// f(kz + 4, ky + 16) = f(kz, ky), as every spectrum of a tile does (the walk's
+// Z stage says why). The network commutes with shifts along its periodic axes,
+// so its output repeats the same way, bit for bit, and 128 of the 256 rows
+// suffice: an M block is the ky < 16 of a tile of its own, in 18 row groups
+// whose halo groups are its own ky = 15 and ky = 0 with kz moved by 4.
+//
+// What bounds it is the way from a layer's last MMA through the epilogue to
+// the next layer's first: tensor-memory loads, shuffles, conversions and
+// stores of dependent steps. The two M blocks share nothing but the weights,
+// so each has eight epilogue warps and a thread that issues its MMAs, and one
+// block's tensor work fills the other's epilogue. Chunk ks of a layer writes
+// the columns of the outputs ks - 1 .. ks + 1 of the accumulators that the
+// epilogue is still emptying, so it goes as soon as output ks + 1 is read. All
+// weights stay in shared memory, so nothing is streamed but the features.
+//
+// 62,160 tiles: whole tiles 3.80 ms; halves with one epilogue of eight warps
+// that the blocks took turns in (tensor pipe 25 % busy, issue slots 38 %) 1.88.
+constexpr int kHalfThreads = 32 * (2 * kEpiWarps + 3);
+constexpr int kGroupsH = 18;
+constexpr int H_A = 0;                                  // [2 blocks][18 groups][8 rows][K 80]
+constexpr int H_IN = H_A + 2 * kGroupsH * 8 * 160;      // [2][18][8][K 16]
+constexpr int H_W = H_IN + 2 * kGroupsH * 8 * 32;       // the weight images
+constexpr int H_FEAT = H_W + IMG_BYTES;                 // [2 blocks][2 stages]
+constexpr int H_BAR = H_FEAT + 4 * FEAT_BYTES;
+// barriers: a block's MMAs of a layer done (2); a release of a block's MMAs
+// (2 x 5: chunk ks, and the input of layer 1 at 0); the weights landed;
+// feature stages full and free (2 x 2 each); the final drains
+constexpr int HB_FULL = 0, HB_READY = 2, HB_W = HB_READY + 10, HB_FFULL = HB_W + 1, HB_FFREE = HB_FFULL + 4,
+              HB_DRAIN = HB_FFREE + 4, kHalfBars = HB_DRAIN + 2;
+constexpr int H_TSLOT = H_BAR + 8 * kHalfBars;
+constexpr int H_FLAG = H_TSLOT + 4;
+constexpr int kHalfSmem = H_FLAG + 4;
+static_assert(kHalfSmem + 2048 <= 227 * 1024, "shared memory of one CTA");
+static_assert(H_IN % 16 == 0 && H_W % 16 == 0 && H_FEAT % 16 == 0 && H_BAR % 8 == 0 && IMG_BYTES % 16 == 0,
+              "copy alignment");
+
+// One 16-byte chunk c of row (ky, kz) of a block's input (rows of KB bytes):
+// group ky + 1, and the halo groups at ky = -1 and 16.
+__device__ __forceinline__ void put_row_half(uint8_t *A, int KB, int ky, int kz, int c, uint4 v)
+{
+    const int grp = 8 * KB;
+    uint8_t *base = A + c * 128;
+    *reinterpret_cast<uint4 *>(base + (ky + 1) * grp + kz * 16) = v;
+    if (ky == 15) *reinterpret_cast<uint4 *>(base + (kz ^ 4) * 16) = v;
+    if (ky == 0) *reinterpret_cast<uint4 *>(base + (kGroupsH - 1) * grp + (kz ^ 4) * 16) = v;
+}
+
+// The thread that issues block b's MMAs.
+__device__ bool half_mma_role(uint8_t *smem, uint32_t tmem, int b, long long first, long long step, long long count,
+                              volatile int *abort_flag)
+{
+    using namespace tpal::tc;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + H_BAR);
+    uint64_t *full = bars + HB_FULL + b, *ready = bars + HB_READY + 5 * b;
+    const uint64_t a1 = sdesc(smem_addr(smem + H_IN + b * kGroupsH * 256), 256),
+                   a2 = sdesc(smem_addr(smem + H_A + b * kGroupsH * 1280), 1280), w = sdesc(smem_addr(smem + H_W), 256);
+    const uint32_t d = tmem + 256 * b;
+    uint32_t rbits = 0;   // parity of each release barrier's next phase
+    auto take_ready = [&](int q) {
+        if (!bar_wait(ready + q, (rbits >> q) & 1)) return false;
+        rbits ^= 1u << q;
+        fence_after();
+        return true;
+    };
+    bool ok = first >= count || bar_wait(bars + HB_W, 0);
+    fence_after();
+    for (long long tile = first; tile < count && ok && !*abort_flag; tile += step) {
+        ok = take_ready(0);
+        if (ok) {
+            mma_layer1<0>(d, a1, w);
+            mma_layer1<1>(d, a1, desc_at(w, NCOL * 32));
+            mma_layer1<2>(d, a1, desc_at(w, 2 * NCOL * 32));
+        }
+        mma_commit(full);
+        for (int L = 1; L < 3 && ok; L++) {
+            for (int ks = 0; ks < 5 && ok; ks++) {
+                ok = take_ready(ks);
+                if (ok) mma_band_any(ks, d, a2, desc_at(w, (L == 1 ? IMG_L2 : IMG_L3) + band_off(ks)));
+            }
+            mma_commit(full);
+        }
+    }
+    if (!ok) *abort_flag = 1;
+    // every MMA issued has completed before the tensor memory is released
+    mma_commit(bars + HB_DRAIN + b);
+    return bar_wait(bars + HB_DRAIN + b, 0) && ok;
+}
+
+// The thread that copies the weights once and each block's next features.
+__device__ bool half_copy_role(uint8_t *smem, const uint8_t *img, const uint16_t *feat, long long first, long long step,
+                               long long count, volatile int *abort_flag)
+{
+    using namespace tpal::tc;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + H_BAR);
+    bool ok = true;
+    long long n[2] = {0, 0};   // features issued per block
+    auto stage = [&](int b) {
+        const long long tile = first + b + n[b] * step;
+        if (tile >= count) return;
+        const int i = 2 * b + (int)(n[b] & 1);
+        if (n[b] >= 2 && !bar_wait(bars + HB_FFREE + i, (uint32_t)(((n[b] >> 1) - 1) & 1))) {
+            ok = false;
+            return;
+        }
+        bar_arrive_expect_tx(bars + HB_FFULL + i, FEAT_BYTES);
+        bulk_g2s(smem + H_FEAT + i * FEAT_BYTES, feat + tile * NV, FEAT_BYTES, bars + HB_FFULL + i);
+        n[b]++;
+    };
+    if (first < count) {
+        stage(0);
+        stage(1);
+        bar_arrive_expect_tx(bars + HB_W, IMG_BYTES);
+        bulk_g2s(smem + H_W, img, IMG_L2, bars + HB_W);
+        bulk_g2s(smem + H_W + IMG_L2, img + IMG_L2, IMG_L3 - IMG_L2, bars + HB_W);
+        bulk_g2s(smem + H_W + IMG_L3, img + IMG_L3, IMG_BYTES - IMG_L3, bars + HB_W);
+    }
+    for (long long tile = first + step; tile < count && ok && !*abort_flag; tile += step)
+        for (int b = 0; b < 2 && ok; b++) stage(b);
+    if (!ok) *abort_flag = 1;
+    // no copy may still be writing shared memory when the CTA leaves
+    for (int b = 0; b < 2; b++)
+        for (long long k = n[b] > 2 ? n[b] - 2 : 0; k < n[b]; k++)
+            if (!bar_wait(bars + HB_FFULL + 2 * b + (int)(k & 1), (uint32_t)((k >> 1) & 1))) ok = false;
+    if (first < count && !bar_wait(bars + HB_W, 0)) ok = false;
+    return ok;
+}
+
+__global__ void __launch_bounds__(kHalfThreads, 1)
+    mn_tc_half_kernel(const uint8_t *img, const float *params, const uint16_t *feat, long long count, float conf_limit,
+                      float *p_out, uint8_t *fallback, int *err)
+{
+    using namespace tpal::tc;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + H_BAR);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + H_TSLOT);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + H_FLAG);
+    __shared__ float s_par[4 * NC + 1];         // b1, b2, b3, wh, bh
+    __shared__ float red[2][2][kEpiWarps];      // [block][parity of the tile][warp]
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (int i = t; i < 4 * NC + 1; i += kHalfThreads) {
+        const int off[5] = {OFF_B1, OFF_B2, OFF_B3, OFF_WH, OFF_BH};
+        s_par[i] = params[off[i / NC] + i % NC];
+    }
+    if (t == 0) {
+        for (int i = 0; i < kHalfBars; i++) {
+            const bool per_warp = (i >= HB_READY && i < HB_READY + 10) || (i >= HB_FFREE && i < HB_FFREE + 4);
+            bar_init(bars + i, per_warp ? kEpiWarps : 1);
+        }
+        *abort_flag = 0;
+    }
+    if (warp == 0) tmem_alloc(tslot, 512);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tslot;
+    // block b's tiles: first + b, + step, ...
+    const long long first = 2 * (long long)blockIdx.x, step = 2 * (long long)gridDim.x;
+    bool ok = true;
+    if (warp == 2 * kEpiWarps + 2) {
+        if (lane == 0) ok = half_copy_role(smem, img, feat, first, step, count, abort_flag);
+        __syncwarp();
+    } else if (warp >= 2 * kEpiWarps) {
+        const int b = warp - 2 * kEpiWarps;
+        if (lane == 0) ok = half_mma_role(smem, tmem, b, first + b, step, count, abort_flag);
+        __syncwarp();
+    } else {
+        const int b = warp >> 3, qd = warp & 3, h = (warp >> 2) & 1;   // block, lane quadrant, channel half
+        uint64_t *full = bars + HB_FULL + b, *ready = bars + HB_READY + 5 * b;
+        uint8_t *A = smem + H_A + b * kGroupsH * 1280, *in = smem + H_IN + b * kGroupsH * 256;
+        const int kz = lane & 7, ky = qd * 4 + (lane >> 3);           // the thread's row
+        const uint32_t tq = tmem + 256 * b + ((uint32_t)(qd * 32) << 16);
+        uint32_t pfull = 0;
+        long long js = 0;   // tiles whose input was written
+        bool bad = false;
+        // A tile's input from its feature stage: row (ky, kz), k = 2 q + c (c =
+        // 0: the bin, 1: its mirror), zero-padded to 16, a 16-byte chunk a
+        // thread; the stage is released.
+        auto write_input = [&]() {
+            const int i = 2 * b + (int)(js & 1);
+            const bool done = bar_wait(bars + HB_FFULL + i, (uint32_t)((js >> 1) & 1));
+            if (done) {
+                const __nv_bfloat16 *f = reinterpret_cast<const __nv_bfloat16 *>(smem + H_FEAT + i * FEAT_BYTES);
+                __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int q = 4 * h + k;
+                    v[2 * k] = v[2 * k + 1] = __float2bfloat16_rn(0.f);
+                    if (q < NQ) {
+                        v[2 * k] = f[(q * 8 + kz) * 32 + ky];
+                        v[2 * k + 1] = f[((4 - q) * 8 + ((10 - kz) & 7)) * 32 + ((40 - ky) & 31)];
+                    }
+                }
+                put_row_half(in, 32, ky, kz, h, *reinterpret_cast<const uint4 *>(v));
+                fence_async_smem();
+            }
+            __syncwarp();
+            if (lane == 0) bar_arrive(bars + HB_FFREE + i);
+            js++;
+            return done;
+        };
+        if (first + b < count) {
+            bad = !write_input();
+            if (lane == 0) bar_arrive(ready + 0);
+        }
+        long long it = 0;
+        for (long long tile = first + b; tile < count; tile += step, it++) {
+            float conf = 0.f;
+            const bool more = tile + step < count;
+            for (int L = 0; L < 2 && !bad; L++) {
+                if (!bar_wait(full, pfull)) {
+                    bad = true;
+                    break;
+                }
+                pfull ^= 1;
+                fence_after();
+                const uint32_t tl = tq + h * 8;
+                float bias[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) bias[c] = s_par[L * NC + h * 8 + c];
+                auto step_q = [&](int q, uint32_t(&cur)[24], uint32_t(&nxt)[24]) {
+                    tmem_wait_ld(cur);
+                    // cleared for the next layer, whose MMAs all accumulate
+                    tmem_zero8(tl + q * 48);
+                    tmem_zero8(tl + q * 48 + 16);
+                    tmem_zero8(tl + q * 48 + 32);
+                    if (q + 1 < NQ) load_half(tl, q + 1, nxt);
+                    float y[8];
+                    combine_half(cur, lane, y);
+                    __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+                    for (int c = 0; c < 8; c++) o[c] = __float2bfloat16_rn(fmaxf(y[c] + bias[c], 0.f));
+                    put_row_half(A, 160, ky, kz, 2 * q + h, *reinterpret_cast<const uint4 *>(o));
+                    if (q == 0) return;
+                    // chunks 0 .. q - 1 are written, columns 0 .. q read and zeroed
+                    fence_async_smem();
+                    tmem_wait_st();
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        bar_arrive(ready + q - 1);
+                        if (q == NQ - 1) bar_arrive(ready + q);
+                    }
+                };
+                uint32_t ba[24], bb[24];
+                load_half(tl, 0, ba);
+                step_q(0, ba, bb);
+                step_q(1, bb, ba);
+                step_q(2, ba, bb);
+                step_q(3, bb, ba);
+                step_q(4, ba, bb);
+            }
+            // the next tile's input, while layer 3's MMAs run (layer 1's, which
+            // read this region, are done)
+            if (more && !bad && !write_input()) bad = true;
+            if (!bad && !bar_wait(full, pfull)) bad = true;
+            if (!bad) {
+                pfull ^= 1;
+                fence_after();
+                // the sigmoid head over the row's 16 channels, eight at a
+                // time: warps 0-3 take output blocks q = 0..2, warps 4-7 q = 3..4
+                float zh = 0.f;
+                auto head = [&](int q, int half, bool last, uint32_t(&cur)[24], uint32_t(&nxt)[24]) {
+                    tmem_wait_ld(cur);
+                    if (!last) load_half(tq + (half ? 0 : 8), half ? q + 1 : q, nxt);
+                    float y[8];
+                    combine_half(cur, lane, y);
+                    if (half == 0) zh = s_par[4 * NC];
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        const float a = bfr(fmaxf(y[c] + s_par[2 * NC + 8 * half + c], 0.f));
+                        zh = __fmaf_rn(a, s_par[3 * NC + 8 * half + c], zh);
+                    }
+                    if (half == 0) return;
+                    const float p = 1.0f / (1.0f + expf(-zh));
+                    float *po = p_out + tile * NV;
+                    po[(q * 8 + kz) * 32 + ky] = p;
+                    po[(q * 8 + (kz ^ 4)) * 32 + ky + 16] = p;
+                    conf += 2.f * fabsf(p - 0.5f);
+                };
+                uint32_t ba[24], bb[24];
+                const int q0 = h == 0 ? 0 : 3, q1 = h == 0 ? 3 : 5;
+                load_half(tq, q0, ba);
+#pragma unroll 1
+                for (int q = q0; q < q1; q++) {
+                    head(q, 0, false, ba, bb);
+                    head(q, 1, q + 1 == q1, bb, ba);
+                }
+                // the block's columns are read: the next tile's layer 1 may run
+                fence_before();
+                __syncwarp();
+                if (more && lane == 0) bar_arrive(ready + 0);
+            }
+            // the tile's confidence; a failure anywhere stops the block's epilogue here
+#pragma unroll
+            for (int hh = 16; hh >= 1; hh >>= 1) conf += __shfl_xor_sync(0xffffffffu, conf, hh);
+            if (lane == 0) red[b][it & 1][warp & 7] = conf;
+            if (epi_or(bad || *abort_flag != 0, 1 + b)) {
+                bad = true;
+                break;
+            }
+            if ((t & 255) == 0 && fallback != nullptr) {
+                float sum = 0.f;
+#pragma unroll
+                for (int w = 0; w < kEpiWarps; w++) sum += red[b][it & 1][w];
+                fallback[tile] = (sum * (1.0f / NV) < conf_limit) ? 1 : 0;
+            }
+        }
+        if (bad) *abort_flag = 1;
         ok = !bad;
     }
     fence_before();
@@ -1507,9 +1775,9 @@ int MaskNet::init()
         if (cudaFuncSetAttribute(mn::mn_forward_kernel<false>, a, (int)mn::kFwdSmem) != cudaSuccess ||
             cudaFuncSetAttribute(mn::mn_forward_kernel<true>, a, (int)mn::kFwdSmem) != cudaSuccess ||
             cudaFuncSetAttribute(mn::mn_backward_kernel, a, (int)mn::kBwdSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false, false>, a, mn::kTcSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false, true>, a, mn::kTcSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<true, false>, a, mn::kTcSmem) != cudaSuccess)
+            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<false>, a, mn::kTcSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mn::mn_tc_half_kernel, a, mn::kHalfSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(mn::mn_tc_forward_kernel<true>, a, mn::kTcSmem) != cudaSuccess)
             return mn_cuda("cudaFuncSetAttribute", cudaGetLastError());
         attr[dev] = true;
     }
@@ -1563,11 +1831,10 @@ int MaskNet::forward(const uint16_t *d_feat, long long ntiles, float *d_p, uint8
         return mn_fail("forward: the feature buffer must be 16-byte aligned");
     const unsigned blocks = (unsigned)std::min<long long>(ntiles, (long long)grid_ * 1);
     if (tc_ && repeating)
-        mn::mn_tc_forward_kernel<false, true><<<(unsigned)std::min<long long>((ntiles + 1) / 2, grid_), mn::kTcThreads,
-                                                mn::kTcSmem, s>>>(img_, used_, d_feat, ntiles, conf_limit_, d_p,
-                                                                  d_fallback, nullptr, nullptr, nullptr, err_);
+        mn::mn_tc_half_kernel<<<(unsigned)std::min<long long>((ntiles + 1) / 2, grid_), mn::kHalfThreads, mn::kHalfSmem,
+                                s>>>(img_, used_, d_feat, ntiles, conf_limit_, d_p, d_fallback, err_);
     else if (tc_)
-        mn::mn_tc_forward_kernel<false, false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
+        mn::mn_tc_forward_kernel<false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
             img_, used_, d_feat, ntiles, conf_limit_, d_p, d_fallback, nullptr, nullptr, nullptr, err_);
     else
         mn::mn_forward_kernel<false><<<blocks, mn::kThreads, mn::kFwdSmem, s>>>(used_, d_feat, ntiles, conf_limit_,
@@ -1606,7 +1873,7 @@ int MaskNet::train_step(const uint16_t *d_feat, const float2 *d_ac, long long nt
     const unsigned blocks = (unsigned)std::min<long long>(ntiles, grid_);
     cudaMemsetAsync(scal_, 0, 2 * sizeof(double), s);
     if (tc_)
-        mn::mn_tc_forward_kernel<true, false><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
+        mn::mn_tc_forward_kernel<true><<<blocks, mn::kTcThreads, mn::kTcSmem, s>>>(
             img_, used_, d_feat, ntiles, conf_limit_, p_, nullptr, (__nv_bfloat16 *)a1_, (__nv_bfloat16 *)a2_,
             (__nv_bfloat16 *)a3_, err_);
     else
