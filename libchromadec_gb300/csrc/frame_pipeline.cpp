@@ -382,12 +382,11 @@ int FramePipeline::decode(int64_t a, int64_t b, const Deliver &deliver, const st
         // bound the plan cache; plans behind the window are not needed again
         // by this run (references into the map stay valid: only others go)
         if (plans_.size() > 4096) plans_.erase(plans_.begin(), plans_.lower_bound(w0));
-        if (bi >= 2) {
-            // the window of this slot was last read by batch bi-2's kernels,
-            // and its plan buffers were last uploaded for batch bi-2
-            cudaStreamWaitEvent(copy_, ev_comp_[slot], 0);
-            if ((e = cudaEventSynchronize(ev_h2d_[slot])) != cudaSuccess) return cuda_status("sync", e);
-        }
+        // the window of this slot was last read by batch bi-2's kernels, and
+        // its plan buffers were last uploaded for batch bi-2 (or by a run
+        // before this one that was cancelled with an upload in flight)
+        cudaStreamWaitEvent(copy_, ev_comp_[slot], 0);
+        if ((e = cudaEventSynchronize(ev_h2d_[slot])) != cudaSuccess) return cuda_status("sync", e);
         if (const int rc = upload_batch(slot, w0, w1); rc != CHD_OK) return rc;
         cudaEventRecord(ev_h2d_[slot], copy_);
         return CHD_OK;
@@ -397,7 +396,7 @@ int FramePipeline::decode(int64_t a, int64_t b, const Deliver &deliver, const st
         const int slot = (int)(bi & 1);
         const int64_t w0 = std::max<int64_t>(0, c - lb_);
         cudaStreamWaitEvent(comp_, ev_h2d_[slot], 0);
-        if (bi >= 2) cudaStreamWaitEvent(comp_, ev_d2h_[slot], 0);   // output slot drained
+        cudaStreamWaitEvent(comp_, ev_d2h_[slot], 0);   // output slot drained
         if (const int rc = eng_.decode(dwin_[slot], dstride_, (int)(2 * w0), 2 * nframes_, (int)c, (int)ce,
                                        dout_[slot], comp_);
             rc != 0)

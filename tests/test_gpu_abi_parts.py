@@ -72,3 +72,15 @@ def test_frames_outlive_the_run(opened):
     for k, f in held.items():
         assert np.array_equal(f.planes(), frame(k))
         f.close()
+
+
+def test_cancelled_between_parts(opened):
+    d, frame = opened
+    for first in (0, 30):   # the second run's uploads follow those the first left behind
+        res = d.decode_async(list(range(first, first + 20)), cancel_after=1)
+        assert len(res) == 20
+        assert res[0][0] == abi.OK and np.array_equal(res[0][2], frame(res[0][1]))
+        assert all(s == abi.E_CANCELLED for s, _, _ in res[1:])
+    got = {i: p for s, i, p in d.decode_async(list(range(10, 30)))}
+    for k in got:
+        assert np.array_equal(got[k], frame(k)), k
