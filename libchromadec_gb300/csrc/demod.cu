@@ -36,7 +36,7 @@
 // Measured on a 500-field capture against the kernel before it (items on the
 // carrier phase, scalar FIR, run-time format): 1.85 -> 1.33 ms, 2,124 -> 1,395
 // warp instructions per 32 items, 634 -> about 400 wavefronts; 160 fields of
-// packed rgb48 with its border 1,460 -> 540 us. What bounds it now is the
+// packed rgb48 with its border 1,465 -> 478 us. What bounds it now is the
 // latency of the plane loads at the start of a block (two blocks of 8 warps a
 // SM: 128 registers for the window). Four blocks of 8 lines (halo 1.75x),
 // three of 10 or 14, two of 192 threads, L2 prefetches of the block 304 ahead
@@ -705,8 +705,11 @@ static int demod_start(const DemodParams &P, unsigned blocks, size_t smem, cudaS
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// The kernels with a constant format: the two Y'CbCr planar formats at the
-// carrier phases of the PAL (1) and PAL-M (0) presets, without yNR.
+// The kernels with a constant format: the Y'CbCr planar and the two R'G'B'
+// formats at the carrier phases of the PAL (1) and PAL-M (0) presets, without
+// yNR. R'G'B' as a constant: PALcolour to rgb48, 160 fields, 565 -> 478 us, PAL-M
+// 3D to rgbs, 82 fields, 825 -> 788 us; gray, whose luma needs no filter, stays
+// with the general kernel.
 template <int XO, bool COMPOSITE>
 static int demod_launch_xo(const DemodParams &P, unsigned blocks, size_t smem, bool ynr, cudaStream_t stream)
 {
@@ -714,6 +717,8 @@ static int demod_launch_xo(const DemodParams &P, unsigned blocks, size_t smem, b
     if constexpr (XO < 2) {
         if (P.format == 0) return demod_start<XO, 0, COMPOSITE, false>(P, blocks, smem, stream);
         if (P.format == 1) return demod_start<XO, 1, COMPOSITE, false>(P, blocks, smem, stream);
+        if (P.format == 2) return demod_start<XO, 2, COMPOSITE, false>(P, blocks, smem, stream);
+        if (P.format == 3) return demod_start<XO, 3, COMPOSITE, false>(P, blocks, smem, stream);
     }
     return demod_start<XO, -1, COMPOSITE, false>(P, blocks, smem, stream);
 }
