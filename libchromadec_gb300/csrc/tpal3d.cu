@@ -254,8 +254,8 @@ __device__ __forceinline__ bool df_sim(df a, df b, df t)
 //
 // Measured against the walk before it (one ky per lane in the Z stage, shuffle
 // DFTs in the Y stages, every bin's guard band in the loop): 2,671 -> 1,541
-// warp instructions a step, 526 -> 330 us for 60 fields. Both the issue slots
-// and the shared-memory path are about 65 % busy; what is left is latency
+// warp instructions a step, 526 -> 330 us for 60 fields. The path of shared
+// memory and L1 is 80 % busy and the issue slots 66 %; the rest is latency
 // (short scoreboard) and instruction fetch: unrolling the kx pairs, a second
 // copy of the rare path or straight-line code for both passes each measured
 // slower. So did samples by asynchronous 16-byte copies (coalesced, but with
@@ -273,7 +273,7 @@ constexpr int kExchF4 = 5 * 20;
 constexpr int kOutF4 = 5 * 20;         // output spectra, the inverse exchange, then the output rows
 constexpr int kBndF4 = 4 * 4;          // [4 pairs][8] float2: kx 0..4 and the row term at 5
 constexpr int kWarpF4 = kWinF4 + kCarryF4 + kExchF4 + kOutF4 + kBndF4;
-constexpr int kTwF4 = 4 * 11;          // Y twiddles per quarter r, per block
+constexpr int kTwF4 = 4 * 7;           // Y twiddles per quarter r, per block
 constexpr int kThrF4 = 3 * 8 * 32 / 4; // squared per-bin thresholds, per block (per-bin walks only)
 constexpr size_t walk_smem(bool per_bin)
 {
@@ -308,9 +308,9 @@ __device__ __forceinline__ LaneConst lane_const(const T3Params &P, int lane, int
     c.rowL = tileY + y0 + 2 * c.i;
     c.row_ok = c.rowL >= P.fafl && c.rowL <= P.lafl;
     const int fl = c.rowL >> 1;
-    // Nine aligned words around the row stay inside the field: the row is not
-    // its first, and it is not the last unless the words end inside it.
-    c.row_fast = tileX >= 0 && fl >= 1 && (fl + 1 < P.fh || tileX + 18 <= P.fw);
+    // Three aligned vectors around the row stay inside the field: the row is not
+    // its first, and it is not the last unless the vectors end inside it.
+    c.row_fast = tileX >= 0 && fl >= 1 && tileX + 24 <= (fl + 1 < P.fh ? 2 * P.fw : P.fw);
     c.row_off = fl * P.fw + tileX;
     c.ky = rev4(c.i);
     c.laneB = kappa((40 - c.ky) & 31);
@@ -333,7 +333,9 @@ __device__ __forceinline__ void z_window(float2 (&wz)[4], bool high)
 // and 2r in both components, then for the positions 4r + e (bin k =
 // rev4(4r + e)) exp(-2 pi i k / 32) in the component of the field with odd
 // rows and 1 in the other. Entry v of quarter r: (x0, x1, y0, y1) at
-// tw[11 r + v], (-y0, -y1) in half v & 1 of tw[11 r + 7 + v / 2].
+// tw[7 r + v]; (-y0, -y1) is a multiplication, cheaper than two more wavefronts
+// of the shared-memory path that bounds the walk (3,970 -> 3,940 us for 500
+// fields, demodulator included).
 __device__ __forceinline__ void fill_twiddles(const T3Params &P, float4 *tw)
 {
     const int odd = 1 ^ ((P.swap ^ P.tileY0) & 1);   // tile rows start 16 lines apart
@@ -342,15 +344,15 @@ __device__ __forceinline__ void fill_twiddles(const T3Params &P, float4 *tw)
         float2 w = v < 3 ? c3_tw16[v == 0 ? r : v == 1 ? r + 4 : 2 * r] : c3_tw32[rev4(4 * r + v - 3)];
         float2 w0 = w, w1 = w;
         if (v >= 3) (odd ? w0 : w1) = make_float2(1.f, 0.f);
-        tw[11 * r + v] = make_float4(w0.x, w1.x, w0.y, w1.y);
-        reinterpret_cast<float2 *>(tw + 11 * r + 7)[v] = make_float2(-w0.y, -w1.y);
+        tw[7 * r + v] = make_float4(w0.x, w1.x, w0.y, w1.y);
     }
     __syncthreads();
 }
 __device__ __forceinline__ tw2 twiddle(const float4 *tw, int r, int v)
 {
-    const float4 a = tw[11 * r + v];
-    return {make_float2(a.x, a.y), make_float2(a.z, a.w), reinterpret_cast<const float2 *>(tw + 11 * r + 7)[v]};
+    const float4 a = tw[7 * r + v];
+    const float2 y = make_float2(a.z, a.w);
+    return {make_float2(a.x, a.y), y, __fmul2_rn(y, make_float2(-1.f, -1.f))};
 }
 
 constexpr unsigned kYLanes = 0xFFFFFu;   // lanes 0..19 run the Y stages
@@ -358,8 +360,8 @@ constexpr unsigned kYLanes = 0xFFFFFu;   // lanes 0..19 run the Y stages
 // The 16 samples of this lane's row of field 2q + j, as words that a funnel
 // shift lines up.
 struct RowWords {
-    uint32_t w[9];
-    unsigned sh;
+    uint32_t w[12];
+    unsigned at;  // byte of the first sample within w
     bool valid;   // else the row is black: outside the capture or the active lines
 };
 
@@ -368,24 +370,32 @@ __device__ __forceinline__ void load_row(const T3Params &P, int q, const LaneCon
     const int f = 2 * q + LC.j;
     const uint16_t *fp = (f >= 0 && f < P.nfields) ? field_at(P, f) : nullptr;
     r.valid = fp != nullptr && LC.row_ok;
-    r.sh = 0;
+    r.at = 0;
     if (!r.valid) return;
     if (LC.row_fast) {
         // Rows start on any 2-byte boundary (odd line and field lengths):
-        // nine aligned 32-bit words cover the 16 samples and a funnel
-        // shift by 0 or 16 bits lines each pair up.
+        // three aligned 16-byte vectors cover the 16 samples. A warp's load
+        // touches 32 rows however wide it is: as nine words the rows took 98
+        // of a step's 464 wavefronts (3,970 -> 3,930 us for 500 fields).
         const uintptr_t pa = reinterpret_cast<uintptr_t>(fp + LC.row_off);
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
-        r.sh = (unsigned)(pa & 2) * 8u;
+        const uint4 *w = reinterpret_cast<const uint4 *>(pa & ~(uintptr_t)15);
+        r.at = (unsigned)pa & 15u;
 #pragma unroll
-        for (int k = 0; k < 9; k++) r.w[k] = __ldg(w + k);
+        for (int k = 0; k < 3; k++) {
+            const uint4 u = __ldg(w + k);
+            r.w[4 * k] = u.x;
+            r.w[4 * k + 1] = u.y;
+            r.w[4 * k + 2] = u.z;
+            r.w[4 * k + 3] = u.w;
+        }
     } else {
 #pragma unroll
         for (int k = 0; k < 8; k++) {   // never before the field start
             const int e = LC.row_off + 2 * k;
             r.w[k] = (uint32_t)__ldg(fp + max(e, 0)) | ((uint32_t)__ldg(fp + max(e + 1, 0)) << 16);
         }
-        r.w[8] = 0;
+#pragma unroll
+        for (int k = 8; k < 12; k++) r.w[k] = 0;
     }
 }
 
@@ -400,9 +410,14 @@ __device__ __forceinline__ void x_forward(const RowWords &row, int q, const Lane
     float2 sd[8];   // (s_x, d_x)
     float rowl1 = 0.0f;
     if (row.valid) {
-        uint32_t v[8];   // samples 2k, 2k+1
+        // the words lined up by whole words, then by a half
+        uint32_t e[10], g[9], v[8];   // v: samples 2k, 2k+1
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = __funnelshift_r(row.w[k], row.w[k + 1], row.sh);
+        for (int k = 0; k < 10; k++) e[k] = row.at & 8u ? row.w[k + 2] : row.w[k];
+#pragma unroll
+        for (int k = 0; k < 9; k++) g[k] = row.at & 4u ? e[k + 1] : e[k];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = __funnelshift_r(g[k], g[k + 1], (row.at & 2u) * 8u);
         // 2^23 + a from the sample's bits; subtracting 2^24 from one side of
         // each sum leaves a_x + a_15-x exactly
         float2 t[4];
