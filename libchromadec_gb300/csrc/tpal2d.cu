@@ -134,13 +134,14 @@ __device__ __forceinline__ bool df_sim2(df a, df b, df t)
 // p ^ (p >> 2) where four lanes hold four neighbours each (see tpal3d.cu).
 constexpr int kBuf2 = 9 * 20;
 constexpr int kWarpF4_2 = 2 * kBuf2 + 5;
-constexpr int kTw2 = 4 * 5;   // Y twiddles per quarter r: three (x, x, y, y), three (-y, -y)
+constexpr int kTw2 = 4 * 3;   // Y twiddles per quarter r: (x, x, y, y)
 constexpr int kBlocks2 = 5;   // resident blocks a SM
 
 __device__ __forceinline__ tw2 twiddle2(const float4 *tw, int r, int v)
 {
-    const float4 a = tw[5 * r + v];
-    return {make_float2(a.x, a.y), make_float2(a.z, a.w), reinterpret_cast<const float2 *>(tw + 5 * r + 3)[v]};
+    const float4 a = tw[3 * r + v];
+    const float2 y = make_float2(a.z, a.w);
+    return {make_float2(a.x, a.y), y, __fmul2_rn(y, make_float2(-1.f, -1.f))};
 }
 
 // Forward Y stage of one column (16 rows in `x` to 16 bins in `s`, position p
@@ -218,8 +219,7 @@ __global__ void __launch_bounds__(32 * kWarps2, kBlocks2) tpal2d_kernel(T2Params
     for (int e = threadIdx.x; e < 12; e += blockDim.x) {
         const int r = e / 3, v = e % 3;
         const float2 w = c2_tw16[v == 0 ? r : v == 1 ? r + 4 : 2 * r];
-        s_tw[5 * r + v] = make_float4(w.x, w.x, w.y, w.y);
-        reinterpret_cast<float2 *>(s_tw + 5 * r + 3)[v] = make_float2(-w.y, -w.y);
+        s_tw[3 * r + v] = make_float4(w.x, w.x, w.y, w.y);
     }
     __syncthreads();
     const int tileX0 = P.avs - 16;
@@ -256,19 +256,27 @@ __global__ void __launch_bounds__(32 * kWarps2, kBlocks2) tpal2d_kernel(T2Params
     float rowl1 = 0.f;
     if (fp != nullptr && inside) {
         uint32_t v[16];   // samples 2k, 2k+1
-        if (tileX >= 0 && fl >= 1 && (fl + 1 < P.fh || tileX + 34 <= P.fw)) {
-            // rows start on any 2-byte boundary: 17 aligned words cover the 32
-            // samples, inside the field, and a funnel shift lines them up
+        if (tileX >= 0 && fl >= 1 && tileX + 40 <= (fl + 1 < P.fh ? 2 * P.fw : P.fw)) {
+            // rows start on any 2-byte boundary: five aligned 16-byte vectors
+            // cover the 32 samples, inside the field; they are lined up by
+            // whole words, then by a half
             const uintptr_t pa = reinterpret_cast<uintptr_t>(fp + fl * P.fw + tileX);
-            const uint32_t *w = reinterpret_cast<const uint32_t *>(pa & ~(uintptr_t)3);
-            const unsigned sh = (unsigned)(pa & 2) * 8u;
-            uint32_t w0 = __ldg(w);
+            const uint4 *w4 = reinterpret_cast<const uint4 *>(pa & ~(uintptr_t)15);
+            uint32_t w[20];
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const uint32_t w1 = __ldg(w + k + 1);
-                v[k] = __funnelshift_r(w0, w1, sh);
-                w0 = w1;
+            for (int k = 0; k < 5; k++) {
+                const uint4 u = __ldg(w4 + k);
+                w[4 * k] = u.x;
+                w[4 * k + 1] = u.y;
+                w[4 * k + 2] = u.z;
+                w[4 * k + 3] = u.w;
             }
+#pragma unroll
+            for (int k = 0; k < 18; k++) w[k] = pa & 8 ? w[k + 2] : w[k];
+#pragma unroll
+            for (int k = 0; k < 17; k++) w[k] = pa & 4 ? w[k + 1] : w[k];
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = __funnelshift_r(w[k], w[k + 1], (unsigned)(pa & 2) * 8u);
         } else {
 #pragma unroll
             for (int k = 0; k < 16; k++) {   // never before the field start
@@ -531,10 +539,11 @@ int tp2_launch(const T2Params &P, cudaStream_t stream)
                              (((P.lafl - 1) / 2 + 1) - ((P.fafl + 1 - 1) / 2 - 8) + 7) / 8);
     const long long items = (long long)ntx * nty * (P.nout / 2);   // tile positions of whole frames
     if (items <= 0) return 0;
-    // Resident blocks, each warp walking several items: 300 fields take 0.93 ms
-    // (2.17 ms in the form before), 16 fields 65 us (125 us); 1,924 warp
-    // instructions a pair of tiles (3,732), issue 54 % active, bound by that
-    // and by the latency of the exchanges.
+    // Resident blocks, each warp walking several items: 300 fields take 0.87 ms
+    // (2.17 ms in the form before), 16 fields 62 us (125 us); 1,924 warp
+    // instructions a pair of tiles (3,732), issue 57 % and the path of shared
+    // memory and L1 76 % busy. Rows as 17 words instead of five vectors and the
+    // twiddles' negatives from shared memory: 0.93 ms.
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
