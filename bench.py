@@ -40,9 +40,12 @@ OUT_BYTES = {"p16": 948 * 288 * 3 * 2, "ps": 948 * 288 * 3 * 4}   # per output f
 # accounting: 2.5 N log2 N per real FFT each way, window, threshold, OLA,
 # demod+pack), in FLOP; bytes = input field + its output planes.
 FLOP_PER_FIELD_3D = 692_311_680
-# the transform's share of it (2,220 tiles x 259,584 FLOP), for the
-# transform kernel's FP32 roofline
-FLOP_PER_FIELD_3D_TRANSFORM = 576_276_480
+# The separable 3D transform's FP32 operations, for the transform stage's
+# roofline: 4,440 tile positions x (folded X stages both ways 2 x 5 x 16 x 8 x 4,
+# radix-2 Y stages 2 x 5 x 320, Z stages with magnitudes and decisions for half
+# of 160 columns' 204) = 24,640. (As separate tile DFTs, 2,220 x 259,584, the
+# count would be 576 M, more than the kernel's time leaves room for.)
+FLOP_PER_FIELD_3D_TRANSFORM = 109_401_600
 # Transform-PAL 2D by the same convention: 2,257 tiles of 16 x 32 per field,
 # 2 (2.5 x 512 x 9) + 512 + 10 x 80 + 2 x 512 = 25,376 FLOP each
 FLOP_PER_FIELD_2D_TRANSFORM = 57_273_632
@@ -687,7 +690,7 @@ def main():
 
     # roofline of the dominant kernel (the transform): launches per step
     # one engine batch = 4 launches: the transform walk, the resolve pass,
-    # the exact re-walk of the items it lists, the demodulator
+    # the outputs of the records it lists, the demodulator
     launches_transform = (nl.value // 2 if two else nl.value // (5 if a.form == "learned" else 4)) if tc_form < 0 \
         else a.steps * ((nframes + 255) // 256)
     per_launch_ms = mt.value / max(1, launches_transform)
@@ -730,7 +733,7 @@ def main():
                    "format": "yuv444" + a.format, "parallelism": f"replicas x{world}" if world > 1 else "1 GPU",
                    "l2": f"inputs {nfields * FIELD_BYTES_IN / 1e6:.0f} MB > 129 MB L2 (no flush)"},
         "roofline": {
-            "bound": "fp32", "kernel": ("tpal2d_kernel" if two else "tpal3d transform stage (walk, resolve, exact re-walk)")
+            "bound": "fp32", "kernel": ("tpal2d_kernel" if two else "tpal3d transform stage (walk, resolve, corrected outputs)")
             if tc_form < 0 else "tensor-core transform stage (tc3_xy, tc3_zd, tc3_yx)",
             "achieved": tr_tflops, "peak": fp32_peak, "unit": "TFLOP/s", "frac": tr_tflops / fp32_peak,
             "traffic": traffic,
@@ -743,9 +746,9 @@ def main():
             "demod_ms_per_launch": md.value / max(1, launches_transform),
             "note": ("the transform's convention FLOP count (2.5 N log2 N per real FFT each way, window, "
                      "threshold, overlap-add; 2,257 16x32 tiles per field)") if two else
-                    ("the transform's convention FLOP count (2.5 N log2 N per real FFT each way, window, "
-                     "threshold, overlap-add; 2,220 distinct tiles per field); the kernel shares the X/Y "
-                     "stages across Z tiles, so it executes fewer FLOPs than counted"),
+                    ("the separable transform's FP32 operations (X and Y stages shared across Z tiles, half of "
+                     "the Z columns by the spectrum's repeat, magnitudes and decisions; 4,440 tile positions "
+                     "per field)"),
             "hbm": {"achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": achieved_gbs / hbm_peak,
                     "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks
                     else "fallback 6.8 TB/s",

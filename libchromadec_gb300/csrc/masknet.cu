@@ -1428,7 +1428,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 //
 // 62,160 tiles: whole tiles 3.80 ms; halves with one epilogue of eight warps
 // that the blocks took turns in 1.88 (tensor pipe 25 % busy, issue slots 38 %);
-// this 1.53 (30 %, 46 %). Releasing two and three chunks at a time instead of one
+// this 1.53 (31 %, 41 %). Releasing two and three chunks at a time instead of one
 // was 1 % slower, starting each output's sum with an MMA of its own instead of
 // clearing the columns 1.5 %.
 constexpr int kHalfThreads = 32 * (2 * kEpiWarps + 3);

@@ -541,8 +541,8 @@ int tp2_launch(const T2Params &P, cudaStream_t stream)
     if (items <= 0) return 0;
     // Resident blocks, each warp walking several items: 300 fields take 0.87 ms
     // (2.17 ms in the form before), 16 fields 62 us (125 us); 1,924 warp
-    // instructions a pair of tiles (3,732), issue 57 % and the path of shared
-    // memory and L1 76 % busy. Rows as 17 words instead of five vectors and the
+    // instructions a pair of tiles (3,732), issue 62 % and the path of shared
+    // memory and L1 70 % busy. Rows as 17 words instead of five vectors and the
     // twiddles' negatives from shared memory: 0.93 ms.
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

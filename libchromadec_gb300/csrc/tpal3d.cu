@@ -254,8 +254,8 @@ __device__ __forceinline__ bool df_sim(df a, df b, df t)
 //
 // Measured against the walk before it (one ky per lane in the Z stage, shuffle
 // DFTs in the Y stages, every bin's guard band in the loop): 2,671 -> 1,541
-// warp instructions a step, 526 -> 330 us for 60 fields. The path of shared
-// memory and L1 is 80 % busy and the issue slots 66 %; the rest is latency
+// warp instructions a step, 526 -> 325 us for 60 fields. The path of shared
+// memory and L1 is 72 % busy and the issue slots 69 %; the rest is latency
 // (short scoreboard) and instruction fetch: unrolling the kx pairs, a second
 // copy of the rare path or straight-line code for both passes each measured
 // slower. So did samples by asynchronous 16-byte copies (coalesced, but with
@@ -1176,7 +1176,7 @@ int tp3_learned_launch(const T3Params &P, const T3Learn &L, int pass, cudaStream
 // ---------------------------------------------------------------------------
 // One warp per record: decide its guard-band bins exactly and, where an exact
 // decision differs from the FP32 one the walk used, correct the record's
-// decisions and list it for the exact walk. The X stage of the record's two kx
+// decisions and list it for tpal3d_exact_kernel. The X stage of the record's two kx
 // columns is computed once for all its bins; lane (z, part) owns rows
 // 4 part .. 4 part + 3 of field 2m + z. A bin at (kz + 4, ky + 16) has the
 // magnitudes of the bin at (kz, ky) (see the walk), so both are decided from
@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(32 * kWarps3) tp3_resolve_kernel(T3Params P)
             if (g == 2 && lane == (lr ^ 16)) keep = simh ? keep | bitrh : keep & ~bitrh;
             any = __ballot_sync(0xffffffffu, todo != 0);
         }
-        if (__any_sync(0xffffffffu, flipped)) {   // the exact walk takes this group's decisions from the record
+        if (__any_sync(0xffffffffu, flipped)) {   // tpal3d_exact_kernel takes this group's decisions from the record
             R.keep[lane] = (uint8_t)keep;
             if (lane == 0) {
                 const unsigned at = atomicAdd(P.counters + 1, 1u);

@@ -27,10 +27,10 @@ __device__ __forceinline__ const uint16_t *field_at(const Params &P, int f)
 // Deferred exact decisions of the 3D transform. The walk decides every bin
 // in FP32 and, for each kx group with a bin inside the guard band, appends
 // one record; the resolve pass decides those bins exactly, corrects the
-// record where FP32 got one wrong and lists it. The exact walk then walks the
-// outputs those decisions reach again, taking the decisions of every recorded
-// group from its record, and overwrites them. One warp walks one item, so an
-// item's records form a list in (m, g) order.
+// record where FP32 got one wrong and lists it. tpal3d_exact_kernel then
+// computes the outputs those decisions reach again, taking the decisions of
+// every recorded group from its record, and overwrites them. One warp walks one
+// item, so an item's records form a list in (m, g) order.
 struct UncRecord {
     int item;            // work item (tile + ntiles * chunk; tile = tx + ntx * ty)
     int mg;              // 4 m + g: the Z tile T(2m), kx group g (column A is kx = 2 + g)
@@ -139,7 +139,7 @@ struct T3Learn {
 int tp3_init_constants(int device);
 // max_blocks > 0 caps the grid; the blocks then walk the work items persistently.
 int tp3_launch(const T3Params &p, cudaStream_t stream, int max_blocks = 0);
-// The resolve pass and the exact walk of the listed items (after
+// The resolve pass and the outputs of the listed records (after
 // tp3_launch; the counters are zeroed before it).
 int tp3_resolve_launch(const T3Params &p, cudaStream_t stream);
 // Learned form: pass 0 writes the features (and optionally the spectrum and
