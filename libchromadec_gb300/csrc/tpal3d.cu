@@ -1013,8 +1013,10 @@ __device__ __forceinline__ uint16_t bf16_bits(float x)
 // walk computes; PASS 1: the same walk with each bin scaled by its fraction
 // (or, on fallback tiles, masked by the FP32 threshold decisions), then the
 // inverse and overlap-add of the plain walk.
+// Four blocks an SM, as the walk: 12 frames' tiles are two waves instead of three
+// (the learned clip 2,058 -> 2,010 us).
 template <int PASS>
-__global__ void __launch_bounds__(32 * kWarps3, 3) tpal3d_learned_kernel(T3Params P, T3Learn L)
+__global__ void __launch_bounds__(32 * kWarps3, 4) tpal3d_learned_kernel(T3Params P, T3Learn L)
 {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
