@@ -68,7 +68,7 @@ int FramePipeline::init(const Capture *cap, const chdg_geometry &g, const chdg_c
     la_ = eng_.look_ahead();
     flen_ = cap->fieldLen();
     dstride_ = (long long)((flen_ + 63) & ~(size_t)63);
-    const size_t winFields = (size_t)2 * (batch_ + lb_ + la_) + 1;   // +1: tiles read a few samples past a field
+    const size_t winFields = (size_t)2 * (batch_ + lb_ + la_);
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&comp_, cudaStreamNonBlocking)) != cudaSuccess) return cuda_status("stream", e);
     if ((e = cudaStreamCreateWithFlags(&copy_, cudaStreamNonBlocking)) != cudaSuccess) return cuda_status("stream", e);

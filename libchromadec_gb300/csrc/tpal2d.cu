@@ -85,11 +85,11 @@ __device__ __noinline__ void exact_pair2(const T2Params &P, int f, int tileX, in
     dfc acc = {{0.f, 0.f}, {0.f, 0.f}};
     const uint16_t *fp = field_at(P, f);   // f is an output field: inside the buffer or the table
     if (fp != nullptr && fl >= fl_first && fl < fl_last) {
-        const uint16_t *row = fp + (long long)fl * P.fw;
+        const int at0 = fl * P.fw + tileX, end = P.fw * P.fh - 1;
         dfc x1 = acc;
         for (int x = 0; x < 32; x++) {
-            const int xx = max(tileX + x, -fl * P.fw);
-            const float a = (float)((int)row[xx] - P.black);
+            // never outside the field: max(min(at, end), 0)
+            const float a = (float)((int)fp[__vimin_s32_relu(at0 + x, end)] - P.black);
             const float *c = c2_dfx[kx - 4][x];
             x1.re = df_add(x1.re, df_mul_f({c[0], c[1]}, a));
             x1.im = df_add(x1.im, df_mul_f({c[2], c[3]}, a));
@@ -278,12 +278,13 @@ __global__ void __launch_bounds__(32 * kWarps2, kBlocks2) tpal2d_kernel(T2Params
 #pragma unroll
             for (int k = 0; k < 16; k++) v[k] = __funnelshift_r(w[k], w[k + 1], (unsigned)(pa & 2) * 8u);
         } else {
+            // Never outside the field: a tile that hangs over the start of the
+            // first line takes its first sample, one over the end of the last its last.
+            const int at0 = fl * P.fw + tileX, end = P.fw * P.fh - 1;
 #pragma unroll
-            for (int k = 0; k < 16; k++) {   // never before the field start
-                const uint16_t *row = fp + fl * P.fw;
-                v[k] = (uint32_t)__ldg(row + max(tileX + 2 * k, -fl * P.fw)) |
-                       ((uint32_t)__ldg(row + max(tileX + 2 * k + 1, -fl * P.fw)) << 16);
-            }
+            for (int k = 0; k < 16; k++)   // max(min(at, end), 0)
+                v[k] = (uint32_t)__ldg(fp + __vimin_s32_relu(at0 + 2 * k, end)) |
+                       ((uint32_t)__ldg(fp + __vimin_s32_relu(at0 + 2 * k + 1, end)) << 16);
         }
         // 2^23 + a from the sample's bits; subtracting 2^24 from one side of
         // each sum leaves a_x + a_31-x exactly

@@ -150,8 +150,8 @@ __device__ __forceinline__ void x_row_pair(const uint16_t *field, long long base
     } else {
 #pragma unroll
         for (int x = 0; x < 16; x++) {
-            const long long idx = base + x < 0 ? 0 : base + x;   // never before the field start
-            a[x] = (int)__ldg(field + idx) - black;
+            const long long idx = base + x < 0 ? 0 : base + x;   // never outside the field
+            a[x] = (int)__ldg(field + (idx < field_len ? idx : field_len - 1)) - black;
         }
     }
 #pragma unroll
@@ -389,10 +389,14 @@ __device__ __forceinline__ void load_row(const T3Params &P, int q, const LaneCon
             r.w[4 * k + 3] = u.w;
         }
     } else {
+        // Never outside the field: a tile that hangs over the start of the first
+        // line takes its first sample, one over the end of the last its last.
+        const int end = P.fw * P.fh - 1;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {   // never before the field start
+        for (int k = 0; k < 8; k++) {
             const int e = LC.row_off + 2 * k;
-            r.w[k] = (uint32_t)__ldg(fp + max(e, 0)) | ((uint32_t)__ldg(fp + max(e + 1, 0)) << 16);
+            r.w[k] = (uint32_t)__ldg(fp + __vimin_s32_relu(e, end)) |   // max(min(e, end), 0)
+                     ((uint32_t)__ldg(fp + __vimin_s32_relu(e + 1, end)) << 16);
         }
 #pragma unroll
         for (int k = 8; k < 12; k++) r.w[k] = 0;
