@@ -278,6 +278,7 @@ __global__ void mn_sum_kernel(const float2 *ac, long long n, double *out)
 // half; the whole step 764 -> 225 us.
 constexpr int kBwdThreads = 288;
 constexpr int kActBytes = 2 * NV * 16;
+constexpr float kNoMargin = __builtin_nanf("");
 constexpr int kNearCap = 2048;              // values to sum again that are listed; more are summed at once
 constexpr size_t kBwdSmem = 2 * kActBytes + sizeof(float) * (2 * NV + 9 * 20 + 32) + sizeof(uint16_t) * kNearCap + 16;
 constexpr int kWFragBytes = 27 * 32 * 16;   // a layer's weights as B fragments of the input gradient
@@ -397,6 +398,9 @@ __device__ __noinline__ float dgrad_one(const __nv_bfloat16 *d, const float *W, 
 
 // Values near a rounding boundary: reach[v] = the 2-norm of the 27 x 16
 // gradients the value is a sum of, wmax[ci] the layer's largest |W|, near the list and its count.
+// Where either is zero it holds a NaN, so that no value counts as near: the sum
+// is zero in any order. (Tiles without energy consist of such values; all of
+// them summed again, one lane at a time, took 304 tiles 1.79 ms, now 0.22 ms.)
 struct DgradNear {
     const float *reach, *wmax;
     uint16_t *list;
@@ -530,6 +534,8 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
         }
         atomicMax(reinterpret_cast<int *>(wmax + pair), __float_as_int(m));
     }
+    __syncthreads();
+    if (t < 32 && wmax[t] == 0.f) wmax[t] = kNoMargin;
     // Input gradient of layer L (1: layer 2, 2: layer 3) from d into act, and
     // its channel sums, the previous layer's bias gradient, into gp + off.
     auto input_gradient = [&](int L, const __nv_bfloat16 *dbuf, uint32_t d, __nv_bfloat16 *act, int off, bool first) {
@@ -554,7 +560,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
                 const int at = (((z + zy / 3 - 1) & 7) << 5) | ((y + zy % 3 - 1) & 31);
                 for (int qi = max(q - 1, 0); qi <= min(q + 1, NQ - 1); qi++) s += dzs[qi * NZY + at];
             }
-            reach[v] = sqrtf(s);
+            reach[v] = s > 0.f ? sqrtf(s) : kNoMargin;
         }
         __syncthreads();
         const DgradNear N = {reach, wmax + 16 * (L - 1), near_list, near_count};
