@@ -446,8 +446,11 @@ __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_co
         for (int idx = threadIdx.x; idx < lines * YW; idx += blockDim.x) ys[idx] = 0.f;
 
     // 2. burst detection: one warp per line (detectBurst, palcolour.cpp:344-409).
-    //    At most 1,135 samples of at most 2^18: the sums fit 32 bits.
+    //    The window is the caller's (a capture's metadata): only what it has
+    //    of the line is read, at most 1,135 samples of at most 2^18, whose sums
+    //    fit 32 bits.
     const bool gray = format >= 4;
+    const int burst0 = max(P.burst_start, 0), burst1 = min(P.burst_end, P.fw);
     if (!gray)
     for (int ln = warp; ln < lines; ln += kWarps) {
         const int fl = fl0 + ln;
@@ -456,7 +459,7 @@ __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_co
         auto px = [&](int line, int i) -> int {
             return (line < 0 || line >= P.fh) ? 0 : (int)__ldg(field + line * P.fw + i);
         };
-        for (int i = P.burst_start + lane; i < P.burst_end; i += 32) {
+        for (int i = burst0 + lane; i < burst1; i += 32) {
             const int d = 2 * px(fl, i) - px(fl - 2, i) - px(fl + 2, i);   // 4 * ((in0 - (in3+in4)/2) / 2)
             const int e = px(fl + 1, i) - px(fl - 1, i);                   // 2 * ((in2 - in1) / 2)
             switch (i & 3) {
