@@ -350,8 +350,8 @@ __device__ __forceinline__ df df_div_f(float a, df d)
 
 __device__ __forceinline__ float df_round(df v) { return __fadd_rn(v.hi, v.lo); }
 
-// FMT: the output format as a constant (yuv444p16 0, yuv444ps 1), or -1: the
-// launch's, any. With the format known the item loop has no branches and half
+// FMT: the output format as a constant (yuv444p16 0, yuv444ps 1, rgb48 2, rgbs
+// 3), or -1: the launch's, any. With the format known the item loop has no branches and half
 // the code (instruction fetch stalled it).
 template <int XO, int FMT, bool COMPOSITE, bool YNR>
 __global__ void __launch_bounds__(kDemodThreads, 2) demod_kernel(const __grid_constant__ DemodParams P)
@@ -732,7 +732,7 @@ int demod_launch(const DemodParams &launch, cudaStream_t stream)
     DemodParams P = launch;
     const bool composite = P.partial == nullptr;
     const bool ynr = P.nr_y > 0.f;
-    // a few fields: shorter blocks, so that every SM has one
+    // a few fields: shorter blocks, so that every SM (152) has one
     const int field_lines = (P.lafl - P.fafl) / 2 + 1;
     P.lines = demod_lines(ynr);
     while (P.lines > 4 && (long long)P.nout * ((field_lines + P.lines - 1) / P.lines) < 152) P.lines /= 2;

@@ -101,9 +101,9 @@ public:
     const chdg_config &config() const { return c_; }
     int look_behind() const { return c_.kind == 8 ? 2 : 0; }   // TransformPal3D::getLookBehind
     int look_ahead() const { return c_.kind == 8 ? 4 : 0; }    // TransformPal3D::getLookAhead
-    // The scratch of decodes of up to `frames` frames, ahead of a run whose
-    // batches grow (a larger scratch means freeing the smaller: a
-    // synchronisation).
+    // The scratch of decodes of up to `frames` frames in the plain form, ahead
+    // of a run whose batches grow (a larger scratch means freeing the smaller: a
+    // synchronisation). The other forms' tile buffers still grow as they decode.
     int reserve(int frames);
     void set_max_batch_frames(int n) { max_batch_frames_ = n > 0 ? n : 1; }
     void set_chunk_frames(int n) { chunk_frames_ = n > 0 ? n : 1; }

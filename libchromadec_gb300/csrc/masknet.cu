@@ -21,6 +21,8 @@
 //    convolution as implicit GEMMs on the tensor cores (tcgen05, BF16
 //    operands, FP32 accumulators in tensor memory), warp-specialised and
 //    persistent over tiles; described where it is defined.
+//  * mn_tc_half_kernel: the same on features that repeat along (kz + 4, ky +
+//    16), as those the walk computes do: what the engine's decode runs.
 // The CUDA-core kernels (one CTA of 256 threads per tile, persistent over
 // tiles; thread t owns the (kz, ky) column t and computes its 5 q x 16
 // channels):
@@ -265,12 +267,18 @@ __global__ void mn_sum_kernel(const float2 *ac, long long n, double *out)
 //    five q accumulated together. The result is rounded to bf16, and a few
 //    bright bins carry most of a gradient, so a value near a rounding boundary
 //    that falls on the other side moves the gradient by up to 1e-4 of it:
-//    values within a bound of both sums' rounding errors of a boundary are summed
-//    again one product after another, in the order (dz, dy,
-//    co, dq), so what is rounded does not depend on the tensor cores' order.
-// The contractions have N = 16 a tap and operands that shift by single rows, so
-// they are m16n8k16 mma.sync on registers: a tcgen05 tile (M 128, N 16, K 16 a
-// tap) would leave its accumulator almost empty. FP32 accumulation; the weight
+//    values nearer to a boundary than several times what the order of summing
+//    changes are summed again one product after another, in the order (dz, dy,
+//    co, dq), so that gradients do not depend on the tensor cores' order and can be
+//    held against a plain restatement (to 1e-7 of their norm where the
+//    activations are exact). The margin is an estimate (from the products'
+//    2-norm), not a proof.
+// Both contractions are m16n8k16 mma.sync on registers. For the weight gradient
+// (M and N 16 a tap, operands that shift by single rows) a tcgen05 tile would
+// leave its accumulator almost empty. The input gradient could fold its taps
+// into N as the forward pass does; it has not been tried, as its operand would
+// need a second copy of the gradients beside the one that the weight gradient
+// reads. FP32 accumulation; the weight
 // gradient's tensor-core sums are five products long and then added in FP32.
 //
 // 256 tiles: 622 us on the CUDA cores (thread (ci, co) walking the voxels, two
@@ -458,8 +466,10 @@ __device__ __forceinline__ void dgrad16(const __nv_bfloat16 *dbuf, uint32_t d, _
                         // distance to the midpoint of two bf16 values, in
                         // units of 2^(exponent - 23), against 2^-18 of a bound of
                         // the products' 2-norm: each of the 432 sums is rounded
-                        // by 2^-25 of a partial sum of about that norm, so this is
-                        // several times the error of either order
+                        // by at most 2^-25 of a partial sum of about that norm;
+                        // errors of either sign add up to about 2^-20.6 of it, so
+                        // this is several times the error of either order
+                        // (all of one sign they would reach 2^-16)
                         const uint32_t bits = __float_as_uint(x);
                         const int ci = 8 * n + 2 * tq + k;
                         const float dist = (float)abs((int)(bits & 0xFFFFu) - 0x8000);

@@ -31,8 +31,8 @@
 //    error estimate E = K * 2^-24 * (sum_z w_z (A_z[kx] + R_z/2) + sum_z w_z |S_z|_1)
 //    where A is the L1 norm of the field's column-DFT outputs for that kx and R
 //    the L1 norm of its DC-removed windowed rows. A decision whose margin is
-//    inside that band is taken again in double-float from the raw samples by
-//    the resolve pass, so every decision equals the FP64 reference's.
+//    inside that band is taken again from the raw samples, in 64-bit fixed
+//    point, by the resolve pass, so every decision equals the FP64 reference's.
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -69,8 +69,9 @@ __device__ int4 g3_qyz[kQYZ];
 
 static bool g_tp3_constants_ready[64];
 
-// kappa(lane): the ky a lane owns in the Z stage (bit-reversed low nibble, so
-// it matches the order the shuffle FFT leaves the spectrum in); an involution.
+// kappa(lane): the ky a lane owns in the Z stage (bit-reversed low nibble: the
+// positions in which the Y stage leaves the spectrum in shared memory); an
+// involution.
 __device__ __forceinline__ int kappa(int l) { return rev4(l & 15) | (l & 16); }
 
 template <int N>
@@ -1329,7 +1330,8 @@ __device__ __forceinline__ int find_record(const T3Params &P, int rec, int mg)
 // output, its six pairs of fields are transformed by a warp each (a seventh
 // looks the records up), the Z stages of the two tiles that meet in the output
 // by four. 31 -> 8.4 us for a few outputs (the walk's own loop over the steps, a
-// warp an output); for the hundreds of a 500-field capture both take about 30.
+// warp an output), 30 -> 15 us for a 200-field capture, 20 for the 900 corrected
+// decisions of a 500-field one.
 constexpr int kWarpsX = 7;
 constexpr int kPairsX = 6;
 template <int TMODE>
